@@ -516,6 +516,51 @@ def test_sample_on_chip_and_from_memory(ops, vocab):
         assert int(got[7]) == int(torch.argmax(logits[7]))
 
 
+@pytest.mark.parametrize("rows,vocab", [
+    # one, two, four and eight blocks a row at their limits; the steps in values a thread; many rows
+    # (32 values a thread before a further block); the longest row a cluster takes and one more
+    (3, 4096), (3, 4097), (3, 16385), (3, 32769), (3, 49153), (3, 81921), (3, 131072), (3, 131073),
+    (33, 5), (33, 8193), (40, 65536)])
+def test_sample_cluster_edges(ops, rows, vocab):
+    """The kernel that spreads a row over a cluster against the one that re-reads the logits: at
+    most one draw in a call may fall within float32 rounding of a boundary (the sums are taken in
+    another order).  Rows whose outcome rounding cannot move agree exactly: one probability that
+    outweighs the others, the value tied everywhere with top-p 0, greedy rows, NaN and infinities."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(rows, vocab, generator=g) * 4
+    tp = torch.tensor([0.95, 0.9999, 0.5])[torch.arange(rows) % 3].clone()
+    temp = torch.full((rows,), 0.8)
+    cases = []
+    if rows > 3:
+        logits[3, vocab // 2] = 400.0                          # everything on one token
+        logits[4] = 1.0                                        # ties with top-p 0: all of them are kept
+        tp[4] = 0.0
+        logits[5, vocab // 3] = float("nan")
+        logits[6] = float("-inf")
+        logits[7, 1] = float("inf")
+        logits[8, 2:] = float("-inf")
+        temp[9] = 0.0                                          # greedy, with a tie and a NaN
+        logits[9, 0] = float("nan")
+        logits[9, [1, vocab - 1]] = 1000.0
+        cases = [3, 6, 7, 9]
+    seed = torch.arange(rows, dtype=torch.int64) * 13 + 1
+    counter = torch.arange(rows, dtype=torch.int64)
+    outs = []
+    try:
+        for mode in (1, 0):
+            ops.lib.rv_sample_set_onchip(mode)
+            outs.append(ops.sample(logits.cuda(), temp.cuda(), tp.cuda(), seed.cuda(),
+                                   counter.cuda()).cpu())
+    finally:
+        ops.lib.rv_sample_set_onchip(1)
+    assert int((outs[0] != outs[1]).sum()) <= 1, (outs[0].tolist(), outs[1].tolist())
+    for m in cases:
+        assert int(outs[0][m]) == int(outs[1][m])
+    if rows > 3:
+        assert int(outs[0][9]) == 1
+        assert int(outs[0][3]) == vocab // 2
+
+
 def test_sample_frequencies(ops):
     """Draws over many counters follow softmax(logits / T)."""
     logits = torch.tensor([[2.0, 1.0, 0.0, -1.0, 0.5]])
