@@ -27,6 +27,8 @@
 //           column never meets another, so the columns of a head are spread over blocks, and a
 //           row's sums are formed token after token in the same order however a prompt was cut.
 //   finish  warp per (token, head): the division, the head's norm, weight and gate.
+// Portions of bfloat16 models whose sizes allow it take the chunk form on the tensor cores instead
+// (mlstm_chunk.cuh).
 // Plain reference: tests/plain_ops.py mlstm.
 #include "common.cuh"
 
@@ -36,6 +38,8 @@
 __device__ __forceinline__ float ml_logsigmoid(float z) {
     return fminf(z, 0.f) - log1pf(expf(-fabsf(z)));
 }
+
+#include "mlstm_chunk.cuh"
 
 __global__ void __launch_bounds__(512) mlstm_gates_kernel(
     const float* __restrict__ rows, int stride, int i_off, int f_off, const float* __restrict__ bi,
@@ -368,9 +372,18 @@ extern "C" long long rv_mlstm_record(int H, int d, int dv) {
     return (long long)H * (dv + 1) * d + H;
 }
 
-// Floats of scratch for n tokens: gate [n, H, 4], then num [n, H, dv + 1].
-extern "C" long long rv_mlstm_scratch(int n_tokens, int H, int dv) {
-    return (long long)n_tokens * H * (4 + dv + 1);
+// Floats of scratch for n tokens: gate [n, H, 4], then num [n, H, dv + 1]; with `chunks` those of the
+// first `single` tokens, then what the chunk form of the others needs.
+extern "C" long long rv_mlstm_scratch(int n_tokens, int single, int n_reqs, int H, int d, int dv, int chunks) {
+    const long long step = (long long)H * (4 + dv + 1);
+    if (!chunks) return n_tokens * step;
+    return ((single * step + 3) & ~3LL) + mlc_scratch(n_tokens - single, n_reqs - single, H, d, dv);
+}
+
+// Whether portions of these sizes can take the chunk form.
+extern "C" int rv_mlstm_chunks_ok(const float* rows, int stride, int out_dtype, int H, int d, int dv,
+                                  const void* out) {
+    return mlc_ok(rows, stride, out_dtype, H, d, dv, out) ? 1 : 0;
 }
 
 // Rows of a column a lane holds.  (Two rows a lane, which doubles the warps of a single prompt,
@@ -381,10 +394,10 @@ static int ml_rows_per_lane(int d) { return d <= 64 ? 4 : d <= 256 ? 8 : 16; }
 extern "C" int rv_mlstm(const float* rows, int stride, const float* bi, const float* bf,
                         const float* norm_w, float* state, const int* token_req, const int* q_start,
                         const int* state_slot, float* scratch, void* out, int out_dtype,
-                        int n_tokens, int n_reqs, int H, int d, int dv, float cap, float eps,
-                        void* stream) {
+                        int n_tokens, int single, int n_reqs, int H, int d, int dv, float cap, float eps,
+                        int chunks, void* stream) {
     if (n_tokens == 0 || n_reqs == 0) return 0;
-    if (n_tokens < 0 || n_reqs < 0 || H < 1 || d < 1 || dv < 1) RV_FAIL("mlstm: bad sizes");
+    if (n_tokens < 0 || n_reqs < 0 || single < 0 || single > n_reqs || single > n_tokens || H < 1 || d < 1 || dv < 1) RV_FAIL("mlstm: bad sizes");
     if (d > 512) RV_FAIL("mlstm: key heads of %d exceed 512", d);
     if (stride < 2 * H * d + 2 * H * dv + 2 * H) RV_FAIL("mlstm: rows are too short");
     if (!(cap > 0.f)) RV_FAIL("mlstm: the gate cap must be positive");
@@ -394,6 +407,34 @@ extern "C" int rv_mlstm(const float* rows, int stride, const float* bi, const fl
     const long long rec = rv_mlstm_record(H, d, dv);
     const int i_off = 2 * H * d + H * dv, f_off = i_off + H, g_off = f_off + H;
     float* gate = scratch;
+    if (chunks && n_tokens > single) {
+        // requests [single, n_reqs) in chunks; the single tokens before them below
+        const int n = n_tokens - single;
+        MlChunk g = {};
+        g.rows = rows; g.bi = bi; g.bf = bf; g.norm_w = norm_w;
+        g.q_start = q_start; g.state_slot = state_slot; g.token_req = token_req;
+        g.state = state; g.rec = rec; g.out = out;
+        g.stride = stride; g.first_req = single; g.n_reqs = n_reqs;
+        g.H = H; g.d = d; g.dv = dv; g.cap = cap; g.eps = eps;
+        // the arrays by token are named by the token's place in the step, the first ones unused
+        float* at = scratch + (((long long)single * H * (4 + dv + 1) + 3) & ~3LL);
+        g.a = (double*)at - (size_t)single * H;
+        at += (size_t)n * H * 2;
+        g.c = (double*)at - (size_t)single * H;
+        at += (size_t)n * H * 2;
+        g.m = at - (size_t)single * H;
+        at += (size_t)n * H;
+        g.em = at - (size_t)single * H;
+        at += (size_t)n * H;
+        g.m_start = at - (size_t)single * H;
+        at += (size_t)(n_reqs - single) * H;
+        g.keep = at;
+        at += la_items(n, n_reqs - single) * H;
+        g.kv = (float*)(((uintptr_t)at + 15) & ~(uintptr_t)15);
+        if (mlc_run(g, n, s)) return 1;
+        if (single == 0) return 0;
+        n_tokens = n_reqs = single;
+    }
     float* num = scratch + (size_t)n_tokens * H * 4;
     // the gates of a long portion are formed by many threads; the chain between them is one thread's
     const int gate_threads = n_tokens / n_reqs >= 256 ? 512 : ML_THREADS;

@@ -102,6 +102,9 @@ class CudaOps:
         # portions of bfloat16 delta rules with a decay per head: "chunks" = the chunk form on the
         # tensor cores where the sizes allow, "tokens" = token by token
         self.gated_delta_mode = os.environ.get("RVLLM_GATED_DELTA", "chunks")
+        # portions of bfloat16 matrix memories: "chunks" = the chunk form on the tensor cores where the
+        # sizes allow, "tokens" = token by token, "auto" = chunks where the longest portion is long
+        self.mlstm_mode = os.environ.get("RVLLM_MLSTM", "auto")
         # float32 products must be float32: no TF32, no reduced-precision accumulation
         torch.backends.cuda.matmul.allow_tf32 = False
         torch.backends.cudnn.allow_tf32 = False
@@ -1486,14 +1489,26 @@ class CudaOps:
         if state.shape[1] != self.mlstm_record(heads, dim, vdim) or out.shape[1] != heads * vdim:
             raise KernelError("mlstm: the record or the output has another size")
         n = rows.shape[0]
-        need = self.lib.rv_mlstm_scratch(c_int(n), c_int(heads), c_int(vdim))
+        # The chunk form's four launches take some 35 us whatever their portions' lengths, the scan
+        # some 8 us and 0.14 us a token of the longest one (8 heads of 64 by 128; 300 tokens: 44
+        # against 48 us, 64 tokens: 41 against 16, 2,048 tokens: 61 against 283).
+        longest = getattr(ctx, "max_q_len", n)
+        chunks = int((self.mlstm_mode == "chunks" or (self.mlstm_mode == "auto" and longest >= 320))
+                     and self.lib.rv_mlstm_chunks_ok(
+                         _ptr(rows), c_int(rows.shape[1]), c_int(_code(out.dtype)), c_int(heads),
+                         c_int(dim), c_int(vdim), _ptr(out)))
+        # the token-by-token form takes single tokens as any others
+        single = min(getattr(ctx, "n_decode", 0), ctx.n_reqs) if chunks else 0
+        need = self.lib.rv_mlstm_scratch(c_int(n), c_int(single), c_int(ctx.n_reqs), c_int(heads),
+                                         c_int(dim), c_int(vdim), c_int(chunks))
         scratch = torch.empty((need,), dtype=torch.float32, device=rows.device)
         self._check(self.lib.rv_mlstm(
             _ptr(rows), c_int(rows.shape[1]), _ptr(in_bias), _ptr(forget_bias), _ptr(norm_w),
             _ptr(state), _ptr(ctx.token_req), _ptr(ctx.q_start), _ptr(ctx.state_slot),
-            _ptr(scratch), _ptr(out), _code(out.dtype), c_int(n), c_int(ctx.n_reqs), c_int(heads),
-            c_int(dim), c_int(vdim), c_float(cap), c_float(eps), self._stream()), "mlstm")
-        self.launches += 2
+            _ptr(scratch), _ptr(out), _code(out.dtype), c_int(n), c_int(single), c_int(ctx.n_reqs),
+            c_int(heads), c_int(dim), c_int(vdim), c_float(cap), c_float(eps), c_int(chunks),
+            self._stream()), "mlstm")
+        self.launches += (2 if single or not chunks else 0) + (4 if chunks and n > single else 0)
 
     # ---- linear attention with decay -----------------------------------------------------------
 

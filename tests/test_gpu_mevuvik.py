@@ -300,6 +300,71 @@ def test_matrix_memory_kernel(ops, dtype, sizes):
         assert abs(float(recd[H * (dv + 1) * d + h]) - mx) < 1e-5 * max(1.0, abs(mx))
 
 
+@pytest.mark.parametrize("strong", [False, True])
+@pytest.mark.parametrize("sizes", [(1, 16, 16), (2, 64, 128), (3, 48, 80), (1, 128, 64), (1, 112, 144),
+                                   (1, 32, 256)])
+def test_matrix_memory_chunks(ops, sizes, strong):
+    """The chunk form against the definition in float64: portions of one token and around one, two
+    and seventeen chunks of 64 (and of more tokens than a round of the gates' sums), a request whose
+    chunks follow another's, an empty request between, filling tokens at the end that come out as
+    zeros, single tokens before the portions.  Output is bfloat16; the records are float32 sums of
+    operands in three exact parts (bound as in the token-by-token test)."""
+    H, d, dv = sizes
+    W, cap, eps = 32, 12.0 if strong else 5.0, 1e-5
+    t, g = _memory_case(H, d, dv, W, d + dv)
+    if strong:
+        t["i"], t["f"] = t["i"] * 8.0, t["f"] * 8.0
+    m = {"heads": H, "dim": d, "vdim": dv, "gate_cap": cap}
+    w_in = np.concatenate([t[k] for k in ("q", "k", "v", "i", "f", "g")])
+    w_in = np.concatenate([w_in, np.zeros((-w_in.shape[0] % 4, W), w_in.dtype)])
+    cuts = {"a": [65, 1, 64, 2100 if (H, d) == (1, 16) else 190], "b": [1, 63, 128, 2], "c": [129, 130, 1, 1]}
+    hs = {r: rnd(g, torch.float32, sum(c), W).numpy() for r, c in cuts.items()}
+    want = {r: plain.matrix_memory(h, m, t, eps) for r, h in hs.items()}
+    state = torch.zeros(5, ops.mlstm_record(H, d, dv), device="cuda")
+    slot = {"a": 4, "b": 0, "c": 2}
+    done, got = {r: 0 for r in cuts}, {r: [] for r in cuts}
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    was = ops.mlstm_mode
+    try:
+        ops.mlstm_mode = "chunks"
+        for step in range(4):
+            parts = sorted(((r, cuts[r][step]) for r in cuts), key=lambda p: p[1] != 1)
+            single = sum(n == 1 for _, n in parts)
+            layout = parts[:single] + [(None, 0)] * (single == 0) + parts[single:single + 1] + [(None, 0)] + \
+                parts[single + 1:] + [(None, 70)]
+            rows, starts, slots, token_req = [], [0], [], []
+            for ri, (r, n) in enumerate(layout):
+                h = hs[r][done[r]:done[r] + n] if r else np.full((n, W), 1e3)
+                rows.append(h @ w_in.T)
+                starts.append(starts[-1] + n)
+                slots.append(slot[r] if r else -1)
+                token_req += [ri] * n
+            x = dev(torch.from_numpy(np.concatenate(rows)).float())
+            ctx = SimpleNamespace(q_start=i32(starts), state_slot=i32(slots), token_req=i32(token_req),
+                                  n_reqs=len(layout), n_decode=single)
+            out = torch.full((x.shape[0], H * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+            ops.mlstm(x, dev(torch.from_numpy(t["i.b"]).float()), dev(torch.from_numpy(t["f.b"]).float()),
+                      dev(torch.from_numpy(t["norm"]).float()), state, ctx, out, H, d, dv, cap, eps)
+            for ri, (r, n) in enumerate(layout):
+                if r:
+                    got[r].append(out[starts[ri]:starts[ri + 1]].cpu())
+                    done[r] += n
+                else:
+                    assert float(out[starts[ri]:starts[ri + 1]].abs().max() if n else 0.0) == 0.0
+    finally:
+        ops.mlstm_mode = was
+    assert float(state[1].abs().max()) == 0 and float(state[3].abs().max()) == 0
+    for r in cuts:
+        close(torch.cat(got[r]), want[r][0], torch.bfloat16)
+        recd = state[slot[r]].cpu().double()
+        for h in range(H):
+            C, n, mx = want[r][1][h]
+            cols = recd[h * (dv + 1) * d:(h + 1) * (dv + 1) * d].reshape(dv + 1, d)
+            close(cols[:dv], C.T, torch.float32, bound=3e-5, scale=max(1.0, float(np.abs(C).max())))
+            close(cols[dv], n, torch.float32, bound=3e-5, scale=max(1.0, float(np.abs(n).max())))
+            assert abs(float(recd[H * (dv + 1) * d + h]) - mx) < 1e-5 * max(1.0, abs(mx))
+
+
 def test_matrix_memory_long_and_with_strong_gates(ops):
     """600 tokens with input gates far above and forget gates far below the cap's middle: the
     running maximum keeps every exponential in range, and the first tokens still show."""
