@@ -53,6 +53,32 @@ __device__ __forceinline__ void lm_split(float x, float y, unsigned& a, unsigned
     c = *(const unsigned*)&l;
 }
 __device__ __forceinline__ float2 lm_pair(unsigned u) { return __bfloat1622float2(*(const __nv_bfloat162*)&u); }
+// The six of nine products of three parts each that reach a float32's last bits, smallest first.
+__device__ __forceinline__ void lm_mma6(float (&lo)[4], float (&hi)[4], const unsigned (&a)[3][4],
+                                        const unsigned (&b)[3][4]) {
+#pragma unroll
+    for (int x = 2; x >= 0; --x)
+#pragma unroll
+        for (int y = 0; y <= x; ++y) {
+            mma_bf16(lo, a[y], b[x - y][0], b[x - y][1]);
+            mma_bf16(hi, a[y], b[x - y][2], b[x - y][3]);
+        }
+}
+// Two of them in turns: four accumulators, so that a product is done before the next one to its
+// accumulator is issued.
+__device__ __forceinline__ void lm_mma6x2(float (&lo)[4], float (&hi)[4], const unsigned (&a)[3][4],
+                                          const unsigned (&b)[3][4], float (&lo2)[4], float (&hi2)[4],
+                                          const unsigned (&a2)[3][4], const unsigned (&b2)[3][4]) {
+#pragma unroll
+    for (int x = 2; x >= 0; --x)
+#pragma unroll
+        for (int y = 0; y <= x; ++y) {
+            mma_bf16(lo, a[y], b[x - y][0], b[x - y][1]);
+            mma_bf16(hi, a[y], b[x - y][2], b[x - y][3]);
+            mma_bf16(lo2, a2[y], b2[x - y][0], b2[x - y][1]);
+            mma_bf16(hi2, a2[y], b2[x - y][2], b2[x - y][3]);
+        }
+}
 // Where a chunk lies: first token and token count (0: no such chunk).  Whole block.
 __device__ __forceinline__ void lm_locate(const int* q_start, const int* state_slot, int first_req,
                                           int n_reqs, int item, int* at) {

@@ -51,9 +51,11 @@
 //
 // With one decay per head, portions of bfloat16 models take the chunk form on the tensor cores where
 // sizes allow (gated_delta_chunk.cuh).  There an activated q, k or v is rounded to bfloat16, and gdr_prepare
-// does the same (`round`), so that a token is the same in a portion and alone.
+// does the same (`round`), so that a token is the same in a portion and alone.  With a decay per channel
+// they have a chunk form of their own, float32 throughout (gated_delta_channel.cuh).
 #include "common.cuh"
 #include "gated_delta_chunk.cuh"
+#include "gated_delta_channel.cuh"
 
 __device__ __forceinline__ float gd_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float gd_softplus(float a) { return a > 20.f ? a : log1pf(expf(a)); }
@@ -570,22 +572,25 @@ static bool gd_shape(int d, int* R, int* P) {
 
 // Whether the portions of a step take the chunk form: where they are long enough on average that
 // chunks of 64 are not mostly filling.
-static bool gd_chunked(int n_tokens, int n_decode, int n_reqs, int H, int G, int d, int dv, int chunks) {
+static bool gd_chunked(int n_tokens, int n_decode, int n_reqs, int H, int G, int d, int dv, int head_decay, int chunks) {
     const int tokens = n_tokens - n_decode, reqs = n_reqs - n_decode;
-    return chunks && gc_sizes_ok(H, G, d, dv) && reqs > 0 && tokens >= 24LL * reqs && tokens <= 65535 * CS_TOKENS;
+    return chunks && (head_decay ? gc_sizes_ok(H, G, d, dv) : gh_sizes_ok(H, G, d, dv)) && reqs > 0 &&
+           (head_decay ? tokens >= 24LL * reqs : gh_long_enough(tokens, reqs)) && tokens <= 65535 * CS_TOKENS;
 }
 
 // Floats of a row of the scratch `prep`, and of the whole scratch for n tokens: the raw read-outs
 // [n, H dv], then prep, then the chunk form's.
 extern "C" long long rv_gated_delta_scratch(int n_tokens, int n_decode, int n_reqs, int H, int G, int d, int dv,
-                                            int chunks) {
+                                            int head_decay, int chunks) {
     int R = 0, P = 0;
     if (!gd_shape(d, &R, &P)) return -1;
     const long long pw = (long long)(2 * G + H) * R * P + gd_pad4(H * dv) + gd_pad4(H) + gd_pad4(G);
     const long long o = ((long long)n_tokens * H * dv + 3) & ~3LL;
-    if (!gd_chunked(n_tokens, n_decode, n_reqs, H, G, d, dv, chunks)) return o + n_tokens * pw;
-    return o + n_decode * pw +
-           gc_layout(n_tokens, la_items(n_tokens - n_decode, n_reqs - n_decode), H, d, dv, 2 * G * d + H * dv).total;
+    if (!gd_chunked(n_tokens, n_decode, n_reqs, H, G, d, dv, head_decay, chunks)) return o + n_tokens * pw;
+    const long long items = la_items(n_tokens - n_decode, n_reqs - n_decode);
+    const int C = 2 * G * d + H * dv;
+    return o + n_decode * pw + (head_decay ? gc_layout(n_tokens, items, H, d, dv, C).total
+                                           : gh_layout(n_tokens, items, H, d, dv, C).total);
 }
 
 template <int R, int P>
@@ -631,7 +636,7 @@ static void gd_launch_scan(const float* prep, int PW, float* state, long long re
 // pre-activations, then H dv of the output gates'; LW is the stride of its rows, which may lie
 // inside proj's); filt [C, taps]; a_log [H]; dt_bias [H d] or [H]; norm_w
 // [dv]; state [slots, record]; scratch: rv_gated_delta_scratch floats, 16-byte aligned; y [N, H dv].
-// Requests [0, n_decode) bring one token each.  `chunks` (with head_decay and bfloat16 y): the others'
+// Requests [0, n_decode) bring one token each.  `chunks` (with bfloat16 y): the others'
 // portions may take the chunk form.
 extern "C" int rv_gated_delta(const float* proj, int P, const float* lowrank, int LW,
                               const float* filt, const float* a_log, const float* dt_bias,
@@ -659,12 +664,20 @@ extern "C" int rv_gated_delta(const float* proj, int P, const float* lowrank, in
     float* o = scratch;
     float* prep = scratch + (((size_t)n_tokens * H * dv + 3) & ~(size_t)3);
     cudaStream_t s = (cudaStream_t)stream;
-    chunks = chunks && head_decay && out_dtype == RV_DTYPE_BF16;
-    const bool chunked = gd_chunked(n_tokens, n_decode, n_reqs, H, G, d, dv, chunks);
-    if (chunked) {
+    chunks = chunks && out_dtype == RV_DTYPE_BF16;
+    if (!head_decay && (C % 4 || LW % 4 || ((uintptr_t)lowrank & 15))) chunks = 0;
+    const bool chunked = gd_chunked(n_tokens, n_decode, n_reqs, H, G, d, dv, head_decay, chunks);
+    if (chunked && head_decay) {
         const GcArgs g = {proj, lowrank, a_log, dt_bias, nullptr, q_start, state_slot, P, LW, C, n_decode, n_reqs, H,
                           G, d, dv, unit_eps, nullptr, nullptr, nullptr, nullptr, nullptr};
         if (gc_run(g, filt, state, rec, taps, token_req, n_decode, n_tokens, prep + (size_t)n_decode * PW, o, s)) return 1;
+    } else if (chunked) {
+        GhArgs g = {};
+        g.proj = proj; g.lowrank = lowrank; g.a_log = a_log; g.dt_bias = dt_bias;
+        g.q_start = q_start; g.state_slot = state_slot;
+        g.P = P; g.LW = LW; g.C = C; g.first_req = n_decode; g.n_reqs = n_reqs;
+        g.H = H; g.G = G; g.d = d; g.dv = dv; g.unit_eps = unit_eps;
+        if (gh_run(g, filt, state, rec, taps, token_req, n_decode, n_tokens, prep + (size_t)n_decode * PW, o, s)) return 1;
     }
     // what is left to the token-by-token form: everything, or the single tokens
     const int n_tok = chunked ? n_decode : n_tokens, n_req = chunked ? n_decode : n_reqs;
@@ -673,7 +686,7 @@ extern "C" int rv_gated_delta(const float* proj, int P, const float* lowrank, in
         cudaFuncSetAttribute(gdr_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
     rv_launch(gdr_prepare_kernel, dim3(n_tok), dim3(256), smem1, s, proj, P, lowrank, LW, filt, a_log,
               dt_bias, (const float*)state, rec, token_req, q_start, state_slot, prep, PW, H, G, d, dp, dv,
-              taps, unit_eps, head_decay, chunks && gc_sizes_ok(H, G, d, dv));
+              taps, unit_eps, head_decay, chunks && head_decay && gc_sizes_ok(H, G, d, dv));
     RV_CHECK_LAUNCH("gated_delta prepare");
     // the staging buffers are sized for the longest portion the step can have if every request
     // brings a token; the size changes only how often the scan's blocks meet, not what they compute

@@ -62,6 +62,71 @@ __device__ __forceinline__ float gc_norm2(const bf16* p, int d, int sub) {      
     return s;
 }
 
+// X_21 = -X_22 (A_21 X_11) for the 32 / w pairs of blocks of w: 32 columns of w rows of outputs, a
+// thread has every (NT / 32)th row of a column.  The inner product goes where A_21 was, once it has been
+// read.  Every sum takes all of its terms (X is zero above the diagonal), so a warp's loads are known
+// when the loop is unrolled: with sums that begin at a lane's own column a chunk of 64 took 15,000
+// cycles more.
+template <int NT, int w>
+__device__ __forceinline__ void gc_inverse_pairs(float* As, float* Xs) {
+    constexpr int STEP = NT / 32, EACH = w > STEP ? w / STEP : 1;
+    const int col = threadIdx.x & 31, i0 = threadIdx.x >> 5, j = col & (w - 1), o = 2 * w * (col / w);
+    const bool mine = i0 < w;
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const float* left = pass ? Xs + (o + w) * 65 + o + w : As + (o + w) * 65 + o;
+        const float* right = (pass ? As + (o + w) * 65 + o : Xs + o * 65 + o) + j;
+        float s[EACH];
+#pragma unroll
+        for (int u = 0; u < EACH; ++u) s[u] = 0.f;
+        if (mine)
+#pragma unroll 16
+            for (int m = 0; m < w; ++m) {
+                const float r = right[m * 65];
+#pragma unroll
+                for (int u = 0; u < EACH; ++u) s[u] = fmaf(left[(i0 + u * STEP) * 65 + m], r, s[u]);
+            }
+        __syncthreads();
+        float* to = (pass ? Xs : As) + (o + w) * 65 + o + j;
+        if (mine)
+#pragma unroll
+            for (int u = 0; u < EACH; ++u) to[(i0 + u * STEP) * 65] = pass ? -s[u] : s[u];
+        __syncthreads();
+    }
+}
+
+// The inverse X of I + A, both [64][65] (of A what is below the diagonal is read, and overwritten).
+// Every thread of a block of NT calls it.
+template <int NT>
+__device__ __forceinline__ void gc_inverse(float* As, float* Xs) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // First its four diagonal blocks of 16, a warp each, two lanes a column:
+    // x_i = (i = j) - sum_(j <= m < i) A_im x_m.
+    if (warp < 4) {
+        const int o = 16 * warp, j = lane >> 1, half = lane & 1;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float s = 0.f;
+#pragma unroll
+            for (int m = 0; m < i; ++m)
+                if ((m & 1) == half) s = fmaf(As[(o + i) * 65 + o + m], x[m], s);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            x[i] = (i == j ? 1.f : 0.f) - s;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if ((i & 1) == half) Xs[(o + i) * 65 + o + j] = x[i];
+    } else {                                              // beside the blocks: zeros
+        for (int n = tid - 128; n < 64 * 64; n += NT - 128)
+            if (((n >> 4) & 3) != (n >> 10)) Xs[(n >> 6) * 65 + (n & 63)] = 0.f;
+    }
+    __syncthreads();
+    // Then pairs of blocks of 16, and the pair of 32.
+    gc_inverse_pairs<NT, 16>(As, Xs);
+    gc_inverse_pairs<NT, 32>(As, Xs);
+}
+
 __global__ void __launch_bounds__(GC_THREADS) gdc_chunk_kernel(const GcArgs g) {
     rv_pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -143,64 +208,7 @@ __global__ void __launch_bounds__(GC_THREADS) gdc_chunk_kernel(const GcArgs g) {
             }
     }
     __syncthreads();
-    // The inverse X of I + A.  First its four diagonal blocks of 16, a warp each, two lanes a column:
-    // x_i = (i = j) - sum_(j <= m < i) A_im x_m.
-    if (warp < 4) {
-        const int o = 16 * warp, j = lane >> 1, half = lane & 1;
-        float x[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float s = 0.f;
-#pragma unroll
-            for (int m = 0; m < i; ++m)
-                if ((m & 1) == half) s = fmaf(As[(o + i) * 65 + o + m], x[m], s);
-            s += __shfl_xor_sync(0xffffffffu, s, 1);
-            x[i] = (i == j ? 1.f : 0.f) - s;
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if ((i & 1) == half) Xs[(o + i) * 65 + o + j] = x[i];
-    } else {                                              // beside the blocks: zeros
-        for (int n = tid - 128; n < 64 * 64; n += GC_THREADS - 128)
-            if (((n >> 4) & 3) != (n >> 10)) Xs[(n >> 6) * 65 + (n & 63)] = 0.f;
-    }
-    __syncthreads();
-    // Then pairs of blocks of 16, and the pair of 32: X_21 = -X_22 (A_21 X_11); the inner product goes
-    // where A_21 was, once it has been read.
-#pragma unroll
-    for (int w = 16; w <= 32; w <<= 1) {
-        const int per = w * w, pairs = 32 / w;            // outputs of a pair; pairs
-        constexpr int MAXO = 32 * 32 / GC_THREADS;
-        float tmp[MAXO];
-        for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll
-            for (int u = 0; u < MAXO; ++u) {
-                const int n = tid + GC_THREADS * u;
-                if (n >= pairs * per) continue;
-                const int q = n / per, e = n - q * per, i = e / w, j = e - i * w, o = 2 * q * w;
-                float s = 0.f;
-                if (pass == 0)
-#pragma unroll 8
-                    for (int m = j; m < w; ++m)
-                        s = fmaf(As[(o + w + i) * 65 + o + m], Xs[(o + m) * 65 + o + j], s);
-                else
-#pragma unroll 8
-                    for (int m = 0; m <= i; ++m)
-                        s = fmaf(Xs[(o + w + i) * 65 + o + w + m], As[(o + w + m) * 65 + o + j], s);
-                tmp[u] = s;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < MAXO; ++u) {
-                const int n = tid + GC_THREADS * u;
-                if (n >= pairs * per) continue;
-                const int q = n / per, e = n - q * per, i = e / w, j = e - i * w, o = 2 * q * w;
-                if (pass == 0) As[(o + w + i) * 65 + o + j] = tmp[u];
-                else Xs[(o + w + i) * 65 + o + j] = -tmp[u];
-            }
-            __syncthreads();
-        }
-    }
+    gc_inverse<GC_THREADS>(As, Xs);
     const size_t ih = (size_t)item * g.H + h;
     bf16* T = g.T + ih * 3 * 64 * 64;
     for (int n = tid; n < 64 * 32; n += GC_THREADS) {

@@ -148,18 +148,6 @@ __device__ __forceinline__ void mlc_put4(bf16* dst, int step, float4 x, float f)
 #pragma unroll
     for (int s = 0; s < 3; ++s) *(uint2*)(dst + s * step) = p[s];
 }
-// The six of nine products of three parts each that reach a float32's last bits, smallest first.
-__device__ __forceinline__ void mlc_mma(float (&lo)[4], float (&hi)[4], const unsigned (&a)[3][4],
-                                        const unsigned (&b)[3][4]) {
-#pragma unroll
-    for (int x = 2; x >= 0; --x)
-#pragma unroll
-        for (int y = 0; y <= x; ++y) {
-            mma_bf16(lo, a[y], b[x - y][0], b[x - y][1]);
-            mma_bf16(hi, a[y], b[x - y][2], b[x - y][3]);
-        }
-}
-
 // A warp has 16 columns of the values by all d rows.
 template <int D16>
 __global__ void mlc_state_kernel(const MlChunk g) {
@@ -215,7 +203,7 @@ __global__ void mlc_state_kernel(const MlChunk g) {
             for (int s = 0; s < 3; ++s)
                 ldmatrix_x4_trans(b[s], ks + (s * LA_C + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LK + nd * 16 +
                                             (lane >> 4) * 8);
-            mlc_mma(acc[2 * nd], acc[2 * nd + 1], a, b);
+            lm_mma6(acc[2 * nd], acc[2 * nd + 1], a, b);
         }
     }
     float* kv = g.kv + ((size_t)item * g.H + h) * (dv + 1) * d;
@@ -379,7 +367,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
 #pragma unroll
             for (int s = 0; s < 3; ++s)
                 ldmatrix_x4(b[s], ks + (s * LA_C + nb * 16 + (lane & 7) + (lane >> 4) * 8) * LK + kk * 16 + ((lane >> 3) & 1) * 8);
-            mlc_mma(p[2 * nb], p[2 * nb + 1], a, b);
+            lm_mma6(p[2 * nb], p[2 * nb + 1], a, b);
         }
 #pragma unroll
         for (int nd = 0; nd < 4; ++nd) {         // the memory's share
@@ -389,7 +377,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
 #pragma unroll
             for (int s = 0; s < 3; ++s)
                 ldmatrix_x4(b[s], ss + (s * dv + c + (lane & 7) + (lane >> 4) * 8) * LK + kk * 16 + ((lane >> 3) & 1) * 8);
-            mlc_mma(o[2 * nd], o[2 * nd + 1], a, b);
+            lm_mma6(o[2 * nd], o[2 * nd + 1], a, b);
         }
     }
     __syncthreads();                             // the memory has been read
@@ -442,7 +430,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
 #pragma unroll
             for (int s = 0; s < 3; ++s)
                 ldmatrix_x4_trans(b[s], vs + (s * LA_C + kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + c + (lane >> 4) * 8);
-            mlc_mma(o[2 * nd], o[2 * nd + 1], a, b);
+            lm_mma6(o[2 * nd], o[2 * nd + 1], a, b);
         }
     }
     // the division, then the norm over the head's columns (a warp has 64 of them)

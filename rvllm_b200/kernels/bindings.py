@@ -99,8 +99,8 @@ class CudaOps:
         # portions of bfloat16 linear attention: "tensor" = tensor-core kernels where the sizes allow
         # (head sizes in multiples of 16, keys up to 128), "simt" = float32 arithmetic
         self.linear_attention_mode = os.environ.get("RVLLM_LINEAR_ATTENTION", "tensor")
-        # portions of bfloat16 delta rules with a decay per head: "chunks" = the chunk form on the
-        # tensor cores where the sizes allow, "tokens" = token by token
+        # portions of bfloat16 delta rules: "chunks" = the chunk form on the tensor cores where the
+        # sizes allow, "tokens" = token by token
         self.gated_delta_mode = os.environ.get("RVLLM_GATED_DELTA", "chunks")
         # portions of bfloat16 matrix memories: "chunks" = the chunk form on the tensor cores where the
         # sizes allow, "tokens" = token by token, "auto" = chunks where the longest portion is long
@@ -1363,11 +1363,16 @@ class CudaOps:
         if lowrank.shape[0] != n or lowrank.shape[1] < decays + heads * vdim or \
                 dt_bias.numel() != decays:
             raise KernelError("gated_delta: the decay and gate rows have another size")
-        chunks = int(head_decay and out.dtype == torch.bfloat16 and self.gated_delta_mode == "chunks")
-        single = ctx.n_decode if chunks else 0       # the token-by-token form takes them as any others
+        # the chunk forms read aligned rows; anything else goes token by token
+        chunks = int(out.dtype == torch.bfloat16 and self.gated_delta_mode == "chunks"
+                     and (head_decay or ((2 * kv_heads * dim + heads * vdim) % 4 == 0
+                                         and lowrank.stride(0) % 4 == 0
+                                         and lowrank.data_ptr() % 16 == 0)))
+        # the token-by-token form takes single tokens as any others
+        single = getattr(ctx, "n_decode", 0) if chunks else 0
         need = self.lib.rv_gated_delta_scratch(c_int(n), c_int(single), c_int(ctx.n_reqs),
                                                c_int(heads), c_int(kv_heads), c_int(dim), c_int(vdim),
-                                               c_int(chunks))
+                                               c_int(1 if head_decay else 0), c_int(chunks))
         if need < 0:
             raise KernelError(f"gated_delta: key heads of {dim} are not supported")
         scratch = torch.empty((need,), dtype=torch.float32, device=proj.device)

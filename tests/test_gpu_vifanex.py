@@ -346,6 +346,39 @@ def test_gated_delta_remembers_far_tokens(ops, sizes):
         assert float((got[0].double() - torch.from_numpy(want)).abs().max()) < 2e-4 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("decays", ["usual", "strong", "none"])
+@pytest.mark.parametrize("sizes", [(2, 1, 128, 128, 4), (4, 2, 16, 16, 3), (3, 1, 48, 80, 1), (2, 2, 112, 32, 2),
+                                   (1, 1, 80, 144, 4)])
+def test_gated_delta_channel_chunks(ops, sizes, decays):
+    """The chunk form (bfloat16 output, portions of 256 tokens and more together) against the plain
+    rule in float64: requests that end at, one before and one after a chunk's and a block of 16's end,
+    one of a single token; decays that forget a channel within a few tokens (e^-20 a token, e^-1000
+    in a chunk) and decays of almost 1.  The records are float32 sums of operands in three exact
+    parts: the bound of the token-by-token form."""
+    H, G, d, dv, taps = sizes
+    g = torch.Generator().manual_seed(d + dv)
+    eps = 1e-5
+    _, _, filt, a_log, dt_bias, norm_w = delta_case(g, 1, H, G, d, dv, taps, memory=decays == "none")
+    if decays == "strong":
+        a_log = a_log + 3.0
+        dt_bias[::3] += 4.0
+    seqs = []
+    for T in (321, 64, 127, 17, 1):
+        proj, low, *_ = delta_case(g, T, H, G, d, dv, taps)
+        seqs.append((proj, low))
+    want = [plain_delta(p.numpy(), l.numpy(), filt.numpy(), a_log.numpy(), dt_bias.numpy(),
+                        norm_w.numpy(), H, G, d, dv, eps) for p, l in seqs]
+    C = 2 * G * d + H * dv
+    for cuts in ((400,), (257, 48, 127, 16, 1)):
+        slots = [5, 2, 3, 0, 6]
+        got, state = run_delta(ops, seqs, cuts, H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, eps,
+                               torch.bfloat16, slots)
+        for i in range(len(seqs)):
+            close(got[i], want[i][0], torch.bfloat16)
+            S = state[slots[i], (taps - 1) * C:].reshape(H, dv, d).transpose(1, 2)
+            close(S, want[i][1], torch.float32, scale=max(1.0, float(np.abs(want[i][1]).max())))
+
+
 def test_gated_delta_order_within_a_token(ops):
     """Decay, then the correction with the decayed state, then the read-out of the written
     state: one head, two tokens, numbers worked by the plain step."""
