@@ -1,5 +1,5 @@
 // Paged causal attention for prompt portions on the 5th-generation tensor cores (bfloat16,
-// head size 64, pages of 8 to 64 tokens).
+// head size 64 or 128, pages of 8 to 64 tokens).
 //
 // One block per (request, key/value head, block of query tokens).  The block's 128 rows are
 // its query tokens times the G query heads that share the key/value head (row = token * G +
@@ -14,8 +14,17 @@
 //   O += P V      tcgen05.mma (M = 128, N = 64, four K = 16 steps), P from shared memory
 //                 (K-major), V as it lies in the cache ([key][dim], i.e. MN-major), O in TMEM
 //                 columns [64, 128).
-// 65 KB of shared memory and 128 TMEM columns per block: three blocks share an SM, so one
-// block's softmax overlaps the others' copies and MMAs.  The exponent's offset follows the
+// Head size 128: queries, keys and values lie as two halves of 64 dimensions, each laid out as
+// above; S takes eight K = 16 steps, O += P V one product of N = 64 per half.  With RV_SAME the
+// values are the keys (a latent row): a tile is copied once and its stage is free when P V is
+// done, and the ring has three stages.
+//
+// Head size 64: 65 KB of shared memory and 128 TMEM columns per block: three blocks share an SM,
+// so one block's softmax overlaps the others' copies and MMAs; 128: 112 KB (96 KB with RV_SAME) and
+// 256 columns, two blocks.
+// Head size 128 against the mma.sync kernel (us; pages of 16): latent rows, 16 heads: 2,048 tokens 93 ->
+// 40, 1,000 tokens 47 -> 22, 300 tokens 15 -> 10, 256 tokens after 3,840 162 -> 26, window 512 57 -> 19;
+// 32 heads: 2,048 tokens 173 -> 49; 32 / 8 heads with values of their own: 232 -> 86.  The exponent's offset follows the
 // row maximum lazily (it moves only when the maximum has grown by more than 2^8), so O is
 // rescaled on few tiles.
 //
@@ -40,9 +49,13 @@
 #ifndef RV_HD
 #define RV_HD 64
 #endif
+#ifndef RV_SAME
+#define RV_SAME 0           // 1: the values are the keys
+#endif
 #define AT_ROWS 128
 #define AT_KEYS 64
-#define AT_STAGES 2
+#define AT_STAGES (RV_SAME ? 3 : 2)
+#define AT_TILES (RV_SAME ? 1 : 2)       // tiles a stage holds: keys, values
 #define AT_WAIT_CYCLES 400000000ll       // about 0.2 s: far beyond any real wait
 
 typedef __nv_bfloat16 bf16;
@@ -159,14 +172,17 @@ __device__ __forceinline__ unsigned long long at_desc(const void* tile) {
 }
 
 template <int HD>
-__global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel(
+__global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill_tcgen05_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table, int max_blocks,
     const int* __restrict__ q_start, const int* __restrict__ ctx_lens, bf16* __restrict__ out,
     int first_req, int num_heads, int num_kv_heads, int q_block, int page_size, float scale_log2,
     int window, int* __restrict__ status, int nsplit, float* __restrict__ part_o,
     float2* __restrict__ part_ml, const float* __restrict__ sinks) {
-    static_assert(HD == 64, "one 128-byte swizzle row per key");
+    static_assert(HD == 64 || HD == 128, "128-byte swizzle rows: 64 dimensions each");
+    constexpr bool SAME = RV_SAME != 0;
+    constexpr int HALVES = HD / 64;
+    constexpr unsigned TMEM = HD == 64 ? 128u : 256u;           // S, O, a power of two
     rv_pdl_prologue();
     // blocks are handed out in the order x, then y: with the key/value head in x, all heads of a
     // request's longest block of query tokens start first, then all heads of the next longest
@@ -196,12 +212,13 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
     const int ppt = AT_KEYS >> page_shift;                      // pages per tile (1..16)
     const unsigned page_bytes = (unsigned)page_size * HD * 2u;
 
-    constexpr int TILE = AT_KEYS * HD;                          // elements of a K or V tile
+    constexpr int TILE = AT_KEYS * HD;                          // elements of a K or V tile,
+    constexpr int HALF = AT_KEYS * 64;                          // of 64 dimensions of it
     extern __shared__ __align__(16) unsigned char smem_raw[];   // aligned by hand
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    bf16* q_tile = (bf16*)base;                                 // [128 rows][64]
-    bf16* kv_ring = q_tile + AT_ROWS * HD;                      // [stages][K tile, V tile]
-    bf16* p_tile = kv_ring + (size_t)AT_STAGES * 2 * TILE;      // [128 rows][64 keys]
+    bf16* q_tile = (bf16*)base;                                 // [halves][128 rows][64]
+    bf16* kv_ring = q_tile + AT_ROWS * HD;                      // [stages][K tile, V tile][halves][64 keys][64]
+    bf16* p_tile = kv_ring + (size_t)AT_STAGES * AT_TILES * TILE;   // [128 rows][64 keys]
     __shared__ __align__(8) unsigned long long q_bar, s_bar, pv_bar, s_read, p_ready;
     __shared__ __align__(8) unsigned long long k_full[AT_STAGES], k_empty[AT_STAGES];
     __shared__ __align__(8) unsigned long long v_full[AT_STAGES], v_empty[AT_STAGES];
@@ -227,7 +244,7 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(at_smem(&tmem_base_smem)), "r"(128u));
+                     ::"r"(at_smem(&tmem_base_smem)), "r"(TMEM));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -243,15 +260,16 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
         // without blocking on either (a blocked wait for values would hold back the keys).
         if (lane == 0) {
             at_mbar_expect_tx(&q_bar, (unsigned)(q_block * G * HD * 2));
-            at_tma_3d(q_tile, &map_q, 0, g * G, qs + q0, &q_bar);
+            for (int x = 0; x < HALVES; ++x)
+                at_tma_3d(q_tile + (size_t)x * AT_ROWS * 64, &map_q, 64 * x, g * G, qs + q0, &q_bar);
         }
-        int next_k = 0, next_v = 0;
+        int next_k = 0, next_v = SAME ? n_tiles : 0;              // (SAME: there are no value tiles)
         const long long t_start = clock64();
         long long t_progress = t_start;
         auto copy_tile = [&](int n, bool values) {
             const int s = n % AT_STAGES;
             unsigned long long* full = values ? &v_full[s] : &k_full[s];
-            bf16* dst = kv_ring + (size_t)s * 2 * TILE + (values ? TILE : 0);
+            bf16* dst = kv_ring + (size_t)s * AT_TILES * TILE + (values ? TILE : 0);
             const int blk = (t_lo + n) * ppt + lane;
             int page = -1;
             if (lane < ppt && blk < max_blocks && (blk << page_shift) < clen)
@@ -262,8 +280,10 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
                 const uint4 z = make_uint4(0, 0, 0, 0);
                 for (int pi = 0; pi < ppt; ++pi) {
                     if (!((miss >> pi) & 1u)) continue;
-                    uint4* dz = (uint4*)(dst + (size_t)pi * page_size * HD);
-                    for (int i = lane; i < (int)(page_bytes / 16); i += 32) dz[i] = z;
+                    for (int x = 0; x < HALVES; ++x) {
+                        uint4* dz = (uint4*)(dst + x * HALF + (size_t)pi * page_size * 64);
+                        for (int i = lane; i < page_size * 8; i += 32) dz[i] = z;
+                    }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
@@ -271,8 +291,9 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
             if (lane == 0) at_mbar_expect_tx(full, (unsigned)__popc(have) * page_bytes);
             __syncwarp();
             if (lane < ppt && page >= 0)
-                at_tma_3d(dst + (size_t)lane * page_size * HD, values ? &map_v : &map_k, 0, g,
-                          page << page_shift, full);
+                for (int x = 0; x < HALVES; ++x)
+                    at_tma_3d(dst + x * HALF + (size_t)lane * page_size * 64, values ? &map_v : &map_k, 64 * x, g,
+                              page << page_shift, full);
         };
         while ((next_k < n_tiles || next_v < n_tiles) && !failed) {
             bool did = false;
@@ -313,7 +334,7 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
                 while (!ok && clock64() - t0 < AT_WAIT_CYCLES)
                     ok = at_mbar_try_wait(&k_full[n % AT_STAGES], (unsigned)(n / AT_STAGES) & 1u);
             }
-            for (int n = max(0, next_v - AT_STAGES); n < next_v; ++n) {
+            for (int n = max(0, next_v - AT_STAGES); !SAME && n < next_v; ++n) {
                 bool ok = false;
                 while (!ok && clock64() - t0 < AT_WAIT_CYCLES)
                     ok = at_mbar_try_wait(&v_full[n % AT_STAGES], (unsigned)(n / AT_STAGES) & 1u);
@@ -331,7 +352,7 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
             const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) |
                                       ((unsigned)(AT_KEYS >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
             const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                      ((unsigned)(HD >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
+                                      ((unsigned)(64 >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
             auto give_up = [&]() {
                 if (!failed) { failed = 1; atomicCAS(status, 0, 21); }
             };
@@ -341,12 +362,13 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
                 if (!failed) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned long long a0 = at_desc(q_tile);
-                    const unsigned long long b0 = at_desc(kv_ring + (size_t)s * 2 * TILE);
+                    const unsigned long long b0 = at_desc(kv_ring + (size_t)s * AT_TILES * TILE);
 #pragma unroll
-                    for (int k = 0; k < HD / 16; ++k)              // 32 bytes per K = 16 step
-                        at_mma(tmem_s, a0 + 2 * k, b0 + 2 * k, idesc_qk, k != 0);
+                    for (int k = 0; k < HD / 16; ++k)              // 32 bytes per K = 16 step, four a half
+                        at_mma(tmem_s, a0 + (k >> 2) * (AT_ROWS * 128 >> 4) + 2 * (k & 3),
+                               b0 + (k >> 2) * (HALF * 2 >> 4) + 2 * (k & 3), idesc_qk, k != 0);
                 }
-                at_commit(&k_empty[s]);                             // the key stage is free again
+                if (!SAME) at_commit(&k_empty[s]);                  // the key stage is free again
                 at_commit(&s_bar);
             };
             if (!at_mbar_wait(&q_bar, 0, &failed)) give_up();
@@ -358,18 +380,21 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
                     issue_qk(n + 1);
                 }
                 if (!failed && !at_mbar_wait(&p_ready, (unsigned)n & 1u, &failed)) give_up();
-                if (!failed && !at_mbar_wait(&v_full[s], (unsigned)(n / AT_STAGES) & 1u, &failed)) give_up();
+                if (!SAME && !failed && !at_mbar_wait(&v_full[s], (unsigned)(n / AT_STAGES) & 1u, &failed)) give_up();
                 if (!failed) {
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned long long a0 = at_desc(p_tile);
-                    const unsigned long long b0 = at_desc(kv_ring + (size_t)s * 2 * TILE + TILE);
+                    const unsigned long long b0 = at_desc(kv_ring + (size_t)s * AT_TILES * TILE + (SAME ? 0 : TILE));
 #pragma unroll
-                    for (int k = 0; k < AT_KEYS / 16; ++k)
-                        // P: 32 bytes per K = 16 step; V: 16 keys = 16 rows of 128 bytes per step
-                        at_mma(tmem_o, a0 + 2ull * k, b0 + (unsigned long long)(k * (16 * 128 >> 4)),
-                               idesc_pv, (n | k) != 0);
+                    for (int x = 0; x < HALVES; ++x)
+#pragma unroll
+                        for (int k = 0; k < AT_KEYS / 16; ++k)
+                            // P: 32 bytes per K = 16 step; V: 16 keys = 16 rows of 128 bytes per step
+                            at_mma(tmem_o + 64 * x, a0 + 2ull * k,
+                                   b0 + (unsigned long long)(x * (HALF * 2 >> 4) + k * (16 * 128 >> 4)),
+                                   idesc_pv, (n | k) != 0);
                 }
-                at_commit(&v_empty[s]);                             // the value stage is free again
+                at_commit(SAME ? &k_empty[s] : &v_empty[s]);        // the value stage is free again
                 at_commit(&pv_bar);
             }
         }
@@ -518,7 +543,7 @@ __global__ void __launch_bounds__(192, 3) paged_attention_prefill_tcgen05_kernel
     __syncthreads();
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
-                     "r"(128u));
+                     "r"(TMEM));
     }
 }
 
@@ -602,7 +627,7 @@ typedef CUresult (*AtEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, vo
                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// [rows][mid][64] bfloat16 with `mid_stride_bytes` between rows: box [box_rows, box_mid, 64].
+// [rows][mid][RV_HD] bfloat16 with `row_bytes` between rows: box [box_rows, box_mid, 64].
 static int at_map(CUtensorMap* map, const void* ptr, long long rows, int mid, long long row_bytes,
                   int box_rows, int box_mid) {
     static AtEncodeFn fn = nullptr;
@@ -616,7 +641,7 @@ static int at_map(CUtensorMap* map, const void* ptr, long long rows, int mid, lo
     }
     cuuint64_t dims[3] = {RV_HD, (cuuint64_t)mid, (cuuint64_t)rows};
     cuuint64_t strides[2] = {RV_HD * 2, (cuuint64_t)row_bytes};
-    cuuint32_t box[3] = {RV_HD, (cuuint32_t)box_mid, (cuuint32_t)box_rows};
+    cuuint32_t box[3] = {64, (cuuint32_t)box_mid, (cuuint32_t)box_rows};
     cuuint32_t elem[3] = {1, 1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides,
                     box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -636,7 +661,8 @@ extern "C" long long AT_SYM(rv_paged_attention_prefill_tcgen05_scratch_bytes)(in
     return (long long)(6 * (size_t)(n_sms > 0 ? n_sms : 1) * AT_PART_BYTES);
 }
 
-static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int n_sms, long long scratch_bytes) {
+static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window, int n_sms,
+                    long long scratch_bytes) {
     static const int forced = [] {
         const char* e = getenv("RVLLM_PREFILL_SPLIT");
         return e && *e ? atoi(e) : 0;
@@ -646,7 +672,11 @@ static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int n_sms,
     // the tiles every block of query tokens has before its own: a whole prompt (none before it)
     // is a triangle of mostly short blocks, which sharing out only burdens (1,000 tokens alone:
     // 22.7 -> 29.2 us with two parts); four such tiles to a part at least
-    const int before = (max_ctx_len > max_q_len ? max_ctx_len - max_q_len : 0) / AT_KEYS;
+    // (within the window, where there is one: 333 tokens after 1,001 with a window of 300, 32 heads of
+    // 128: 28.6 us shared out over three blocks each, 14.0 us whole)
+    int earlier = max_ctx_len > max_q_len ? max_ctx_len - max_q_len : 0;
+    if (window > 0 && earlier > window) earlier = window;
+    const int before = earlier / AT_KEYS;
     if (forced <= 0 && parts > before / 4) parts = before / 4;
     if (parts > AT_MAX_PARTS) parts = AT_MAX_PARTS;
     while (parts > 1 && (blocks * parts > 3 * places ||
@@ -657,7 +687,7 @@ static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int n_sms,
 
 // Requests [first_req, first_req + n_reqs), the longest bringing max_q_len tokens and holding
 // max_ctx_len; `q` is the q|k|v buffer [n_tokens, q_stride] (the query heads first), `out` is
-// [n_tokens, heads * 64]; `scratch` (may be null: no sharing out) holds the parts.
+// [n_tokens, heads * head size]; `scratch` (may be null: no sharing out) holds the parts.
 extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
     const void* q, int q_stride, int n_tokens, const void* k_cache, const void* v_cache,
     long long total_slots, const int* block_table, int max_blocks, const int* q_start,
@@ -683,7 +713,8 @@ extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
     if (at_map(&map_v, v_cache, total_slots, num_kv_heads, (long long)num_kv_heads * RV_HD * 2,
                page_size, 1))
         return 1;
-    const size_t smem = (size_t)(AT_ROWS * RV_HD + AT_STAGES * 2 * AT_KEYS * RV_HD + AT_ROWS * AT_KEYS) *
+    if (RV_SAME && k_cache != v_cache) return at_fail("paged_attention_prefill_tcgen05: the values are not the keys");
+    const size_t smem = (size_t)(AT_ROWS * RV_HD + AT_STAGES * AT_TILES * AT_KEYS * RV_HD + AT_ROWS * AT_KEYS) *
                             sizeof(bf16) + 1024;
     static bool configured = false;
     if (!configured) {
@@ -694,7 +725,7 @@ extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
     }
     const int nqb = (max_q_len + q_block - 1) / q_block;
     const long long blocks = (long long)num_kv_heads * nqb * n_reqs;
-    const int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, n_sms, scratch_bytes) : 1;
+    const int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;
     if ((long long)n_reqs * (parts > AT_ROWS / 16 ? parts : AT_ROWS / 16) > 65535)
         return at_fail("paged_attention_prefill_tcgen05: too many requests");
     float* part_o = (float*)scratch;

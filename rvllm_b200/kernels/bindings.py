@@ -62,7 +62,7 @@ class CudaOps:
         self._verbose_build = verbose_build
         # bfloat16 attention: "mma" = mma.sync tensor-core kernels (attention_mma.cu, key and value
         # sizes that are multiples of 16 up to 192), "simt" = the float32-arithmetic kernels;
-        # prompt portions also "tcgen05" (attention_tcgen05.cu, head size 64) and "auto" =
+        # prompt portions also "tcgen05" (attention_tcgen05.cu, head sizes 64 and 128) and "auto" =
         # tcgen05 where it applies, else mma
         self.prefill_attention = os.environ.get("RVLLM_PREFILL_ATTENTION", "auto")
         self.decode_attention = os.environ.get("RVLLM_DECODE_ATTENTION", "mma")
@@ -496,13 +496,17 @@ class CudaOps:
         """The tensor-core attention library for keys and values of this size."""
         return self._mma_lib(head_dim, head_dim, False, False)[0]
 
-    def _attn5_lib(self, head_dim: int):
-        """The tcgen05 prefill attention library for this head size, built at first use."""
-        key = ("tcgen05", head_dim)
+    def _attn5_lib(self, head_dim: int, same: bool = False):
+        """The tcgen05 prefill attention library for this head size (`same`: the values are the
+        keys), built at first use."""
+        key = ("tcgen05", head_dim, same)
         lib = self._attn_libs.get(key)
         if lib is None:
-            path = build_variant("attention_tcgen05.cu", {"RV_HD": head_dim},
-                                 f"attn5_hd{head_dim}", verbose=self._verbose_build)
+            defines, tag = {"RV_HD": head_dim}, f"attn5_hd{head_dim}"
+            if same:
+                defines["RV_SAME"] = 1
+                tag += "s"
+            path = build_variant("attention_tcgen05.cu", defines, tag, verbose=self._verbose_build)
             try:
                 lib = ctypes.CDLL(path)
             except OSError as e:
@@ -512,7 +516,7 @@ class CudaOps:
         return lib
 
     def _tcgen05_prefill_ok(self, qkv, out, num_heads, num_kv_heads, head_dim, page_size) -> bool:
-        return (qkv.dtype == torch.bfloat16 and head_dim == 64
+        return (qkv.dtype == torch.bfloat16 and head_dim in (64, 128)
                 and page_size in (8, 16, 32, 64) and num_heads // num_kv_heads <= 128
                 and qkv.shape[1] % head_dim == 0 and qkv.data_ptr() % 16 == 0
                 and out.data_ptr() % 16 == 0)
@@ -520,8 +524,9 @@ class CudaOps:
     def paged_attention_prefill_tcgen05(self, qkv, num_heads, num_kv_heads, head_dim, k_cache,
                                         v_cache, ctx, group, scale, window, out, sinks=None):
         """Requests [n_decode, n_reqs) -- the ones that bring more than one token -- on the
-        tcgen05 kernel (bfloat16, head size 64)."""
-        lib = self._attn5_lib(head_dim)
+        tcgen05 kernel (bfloat16, head size 64 or 128)."""
+        lib = self._attn5_lib(head_dim, head_dim == 128
+                              and self._same_rows(k_cache, v_cache, head_dim, head_dim))
         nd = ctx.n_decode
         fn = getattr(lib, f"rv_paged_attention_prefill_tcgen05_hd{head_dim}")
         # scratch for the parts of a launch too small to fill the GPU (the kernel shares the key
@@ -546,11 +551,11 @@ class CudaOps:
 
     def _prefill_scratch_bytes(self, head_dim: int) -> int:
         """What the tcgen05 prefill attention may use for the parts of shared-out blocks."""
-        if head_dim != 64 or self.prefill_attention not in ("auto", "tcgen05"):
+        if head_dim not in (64, 128) or self.prefill_attention not in ("auto", "tcgen05"):
             return 0
         # rv_paged_attention_prefill_tcgen05_scratch_bytes: six parts an SM, each 128 rows of
-        # 64 float32 values, an offset and a sum (the kernel fits its parts to what it is given)
-        return 6 * self._sm_count * 128 * (64 * 4 + 8)
+        # float32 values, an offset and a sum (the kernel fits its parts to what it is given)
+        return 6 * self._sm_count * 128 * (head_dim * 4 + 8)
 
     def _check_attn(self, lib, tag: str, rc: int, what: str) -> None:
         self.launches += 1
@@ -608,7 +613,10 @@ class CudaOps:
                 self.paged_attention_decode(qkv, num_heads, num_kv_heads, head_dim, k_cache,
                                             v_cache, group.block_table, ctx.ctx_lens, nd,
                                             ctx.max_ctx_len, group.page_size, scale, window, out)
+        # (heads of 128 with one tile of keys at most stay with mma.sync: 4 tokens 4.6 against 5.9 us,
+        # 16 tokens 5.4 - 5.8 against 6.2; 64 tokens take 6.0 either way, 300 17 against 10)
         if (ctx.n_tokens > nd and self.prefill_attention in ("auto", "tcgen05") and vd == head_dim
+                and (head_dim == 64 or ctx.max_ctx_len > 64)
                 and self._tcgen05_prefill_ok(qkv, out, num_heads, num_kv_heads, head_dim,
                                              group.page_size)):
             self.paged_attention_prefill_tcgen05(qkv, num_heads, num_kv_heads, head_dim, k_cache,

@@ -680,6 +680,32 @@ def test_prefill_attention_kernels(ops, case, standout):
         ops.prefill_attention = chosen
 
 
+@pytest.mark.parametrize("same", [False, True])
+@pytest.mark.parametrize("case", [c for c in PREFILL_CASES if max(c[1]) > 64])
+def test_prefill_attention_head_size_128(ops, case, same):
+    """Head size 128 (two halves of 64 dimensions a tile), with values of their own and with values
+    that are the keys (one page tensor under both names), through the default choice; with a sink
+    per head.  The same cases and bound as at head size 64."""
+    q_lens, ctx_lens, nh, nkv, _, ps, window = case
+    hd = 128
+    g = torch.Generator().manual_seed(23)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, q_lens, ctx_lens, nh, nkv, hd, ps,
+                                           window, True)
+    vc = kc if same else vc
+    sinks = torch.randn(nh, generator=g)
+    scale = 1.0 / math.sqrt(hd)
+    ref = torch.zeros(ctx.n_tokens, nh * hd, dtype=torch.bfloat16)
+    PlainOps().paged_attention(q, nh, nkv, hd, kc, vc, ctx, group, scale, window, ref, sinks=sinks)
+    dk = kc.cuda()
+    dv = dk if same else vc.cuda()
+    out = torch.full((ctx.n_tokens, nh * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(q.cuda(), nh, nkv, hd, dk, dv, to_cuda(ctx), to_cuda(group), scale, window,
+                        out, sinks=sinks.cuda())
+    ops.check_status()
+    assert ("tcgen05", 128, same) in ops._attn_libs
+    assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
+
+
 def test_prefill_attention_tcgen05_is_used(ops):
     """The default choice takes the tcgen05 kernel where it applies (its launch is counted by
     its own library) and refuses nothing it cannot do: other head sizes go to the mma kernel."""
