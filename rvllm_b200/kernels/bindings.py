@@ -349,6 +349,13 @@ class CudaOps:
                                 table, positions, slot_mapping, k_cache, v_cache)
         return qkv
 
+    def _float32_product(self, x, w, out_dtype) -> bool:
+        """Whether x . w^T goes to this library's float32 kernel (few rows, or few columns)."""
+        return (x.dtype == torch.float32 and out_dtype == torch.float32 and self.gemm_mode != "cublas"
+                and x.is_contiguous() and w.is_contiguous()
+                and (x.data_ptr() | w.data_ptr()) % 16 == 0
+                and self.lib.rv_gemm_f32_better(x.shape[0], w.shape[0], x.shape[1]) != 0)
+
     def linear(self, x, w, bias=None, out_dtype=None):
         out_dtype = out_dtype or x.dtype
         if x.dtype != w.dtype:
@@ -359,6 +366,11 @@ class CudaOps:
             return torch.empty((0, w.shape[0]), dtype=out_dtype, device=x.device)
         if self._small_product(x, w, out_dtype):
             y = self.linear_tcgen05(x, w, out_dtype)
+        elif self._float32_product(x, w, out_dtype):
+            y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+            self._check(self.lib.rv_gemm_f32(_ptr(x), _ptr(w), _ptr(y), c_int(x.shape[0]),
+                                             c_int(w.shape[0]), c_int(x.shape[1]), self._stream()),
+                        "gemm_f32")
         else:
             # The library chooses an algorithm per shape, and a shape it has not met costs it
             # some 70 us on the host: a prompt portion of 301 tokens, then 302, ... would pay

@@ -631,6 +631,31 @@ def test_gemm_tiled_weights(ops, M, N, K):
     assert float((a.double() - ref).abs().max() / ref.abs().max()) <= 2e-5
 
 
+@pytest.mark.parametrize("M,N,K", [
+    # every number of row groups, one and two row tiles, columns that fill no tile, K that fills no
+    # step (and no split of K), K split over one to eight blocks
+    (1, 256, 256), (8, 300, 1028), (9, 2048, 260), (16, 70000, 512), (24, 4608, 1536), (32, 1001, 2052),
+    (40, 520, 4096), (48, 640, 1024), (56, 257, 3000), (64, 6144, 256), (65, 1536, 6912), (131, 2048, 516),
+    (160, 333, 1540)])
+def test_gemm_f32(ops, M, N, K):
+    """The float32 product against float64.  Each output is up to sixteen sums (even and odd k, eight
+    parts of K) of at most K / 2 fused multiply-adds: its error is below (K / 2 + 16) 2^-24 of the sum of
+    the terms' magnitudes, whatever the order; the sums here are far inside that."""
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g)
+    w = torch.randn(N, K, generator=g) * 0.05
+    x[M // 2, K // 3] = 40.0
+    w[N // 5, K // 3] = 3.0
+    assert ops.lib.rv_gemm_f32_better(M, N, K)
+    before = ops.launches
+    y = ops.linear(x.cuda(), w.cuda())
+    assert ops.launches == before + 1                      # the kernel, not the library
+    ref = x.double() @ w.double().t()
+    bound = (K / 2 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((y.double().cpu() - ref).abs() <= bound).all())
+    assert float((y.double().cpu() - ref).norm() / ref.norm()) < 1e-6
+
+
 PREFILL_CASES = [
     # q_lens, ctx_lens, heads, kv heads, head size, page size, window.  Head size 64: the
     # tcgen05 kernel (128 rows = tokens x heads of a group, tiles of 64 keys): group sizes
