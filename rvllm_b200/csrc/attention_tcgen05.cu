@@ -23,10 +23,14 @@
 // so one block's softmax overlaps the others' copies and MMAs; 128: 112 KB (96 KB with RV_SAME) and
 // 256 columns, two blocks.
 // Head size 128 against the mma.sync kernel (us; pages of 16): latent rows, 16 heads: 2,048 tokens 93 ->
-// 40, 1,000 tokens 47 -> 22, 300 tokens 15 -> 10, 256 tokens after 3,840 162 -> 26, window 512 57 -> 19;
-// 32 heads: 2,048 tokens 173 -> 49; 32 / 8 heads with values of their own: 232 -> 86.  The exponent's offset follows the
-// row maximum lazily (it moves only when the maximum has grown by more than 2^8), so O is
-// rescaled on few tiles.
+// 42, 1,000 tokens 48 -> 23, 300 tokens 15 -> 11, 256 tokens after 3,840 162 -> 27, window 512 57 -> 21;
+// 32 heads: 2,048 tokens 173 -> 54; 32 / 8 heads with values of their own: 234 -> 90.  At head size 64
+// the exponent's offset follows the row maximum lazily (it moves only when the maximum has grown by
+// more than 2^8), so O is rescaled on few tiles.  Heads of 128 move it with the maximum and divide by
+// the sum of the rounded P, as the mma.sync kernel that they ran on before does: a row's largest P is
+// then exactly 1, and the error against 64 bits is that kernel's.  Moving it lazily and adding the
+// unrounded P took 40 us instead of 42 at 2,048 tokens and 49 instead of 54 with 32 heads, with an
+// error of up to 0.8 % more.
 //
 // Roles: warps 0-3 are the 128 rows; warp 4 brings Q (one 3-D TMA copy: [tokens, heads, 64])
 // and the key and value tiles (one 3-D TMA copy per page) into rings of two stages, keys and
@@ -442,26 +446,32 @@ __global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill
                 mx4[3] = fmaxf(mx4[3], sv[j + 3]);
             }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
-            // The exponent's offset follows the row maximum lazily: it moves only when the
-            // maximum has grown by more than 2^8 since it was set (P then stays below 256,
-            // exact in bfloat16 and harmless in the float32 sums), so O is rescaled on few
-            // tiles; the final O / l does not depend on the offsets chosen on the way.
-            const bool moved = mx > m_run + 8.f || (m_run == -INFINITY && mx > -INFINITY);
+            // Head size 64: the exponent's offset follows the row maximum lazily: it moves only when
+            // the maximum has grown by more than 2^8 since it was set (P then stays below 256,
+            // harmless in the float32 sums), so O is rescaled on few tiles.  128: it moves with the
+            // maximum, whose P is then 1.
+            const bool moved = mx > m_run + (HD == 128 ? 0.f : 8.f) || (m_run == -INFINITY && mx > -INFINITY);
             const float m_new = moved ? mx : m_run;
             const float off = m_new == -INFINITY ? 0.f : m_new;
             const float corr = moved ? at_exp2(m_run - off) : 1.f;  // m_run = -inf -> 0
             m_run = m_new;
             // P = 2^(S * scale - offset) as bfloat16, kept in registers while the previous
-            // tile's P V may still be running
+            // tile's P V may still be running.  Heads of 128 add the rounded values to the row sum,
+            // as the mma.sync kernel does, so that both sides of O / l see the same numbers.
             unsigned pk[AT_KEYS / 2];
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int j = 0; j < AT_KEYS; j += 2) {
                 const float e0 = at_exp2(fmaf(sv[j], scale_log2, -off));
                 const float e1 = at_exp2(fmaf(sv[j + 1], scale_log2, -off));
-                sum4[(j >> 1) & 3] += e0 + e1;
                 const __nv_bfloat162 pr = __floats2bfloat162_rn(e0, e1);
                 pk[j >> 1] = *(const unsigned*)&pr;
+                if constexpr (HD == 128) {
+                    const float2 pf = __bfloat1622float2(pr);
+                    sum4[(j >> 1) & 3] += pf.x + pf.y;
+                } else {
+                    sum4[(j >> 1) & 3] += e0 + e1;
+                }
             }
             l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
             // the previous tile's P V must be done before O is touched and P overwritten

@@ -731,6 +731,30 @@ def test_prefill_attention_head_size_128(ops, case, same):
     assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("same", [False, True])
+@pytest.mark.parametrize("lens", [[80], [33, 130]])
+def test_prefill_attention_head_size_128_rounds_alike(ops, lens, same):
+    """The two prompt kernels round the same probabilities (a row's largest is exactly 1) and divide by
+    the sum of the rounded values.  What is left is the order of float32 sums, some 1e-6, which moves
+    some 1e-3 of the bfloat16 roundings by 2^-8: sqrt(1e-3) 2^-8 = 1.2e-4 together, and four times that
+    is the bound.  Other offsets, or a sum of unrounded values, give 3e-3."""
+    g = torch.Generator().manual_seed(24)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, lens, lens, 8, 2, 128, 16)
+    k = kc.cuda()
+    v = k if same else vc.cuda()
+    outs, chosen = [], ops.prefill_attention
+    try:
+        for kernel in ("tcgen05", "mma"):
+            ops.prefill_attention = kernel
+            out = torch.empty(sum(lens), 8 * 128, dtype=torch.bfloat16, device="cuda")
+            ops.paged_attention(q.cuda(), 8, 2, 128, k, v, to_cuda(ctx), to_cuda(group), 128 ** -0.5, None, out)
+            outs.append(out.double())
+        ops.check_status()
+    finally:
+        ops.prefill_attention = chosen
+    assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 4.9e-4
+
+
 def test_prefill_attention_tcgen05_is_used(ops):
     """The default choice takes the tcgen05 kernel where it applies (its launch is counted by
     its own library) and refuses nothing it cannot do: other head sizes go to the mma kernel."""
