@@ -350,8 +350,13 @@ class CudaOps:
         return qkv
 
     def _float32_product(self, x, w, out_dtype) -> bool:
-        """Whether x . w^T goes to this library's float32 kernel (few rows, or few columns)."""
+        """Whether x . w^T goes to this library's float32 kernel (few rows, or few columns).  What
+        the kernel cannot see from its pointers is looked at here: operands that do not fit one
+        another, that lie on another device or that want gradients are the library's."""
         return (x.dtype == torch.float32 and out_dtype == torch.float32 and self.gemm_mode != "cublas"
+                and x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1]
+                and x.get_device() == w.get_device() == torch.cuda.current_device()
+                and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
                 and x.is_contiguous() and w.is_contiguous()
                 and (x.data_ptr() | w.data_ptr()) % 16 == 0
                 and self.lib.rv_gemm_f32_better(x.shape[0], w.shape[0], x.shape[1]) != 0)
