@@ -63,7 +63,9 @@ __device__ __forceinline__ void gf_reduce(const float* sm, float* y, int m0, int
 template <int TMG, int TNG>
 __global__ void __launch_bounds__(TMG* TNG) gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                             float* __restrict__ y, int M, int N, int K, int per_split) {
-    rv_pdl_launch_dependents();
+    // Neither operand is read before the kernel before has ended: the matrix need not be a weight, it
+    // may be what that kernel writes (rows of 32 bits by a matrix of 16 are cast just before).
+    rv_pdl_prologue();
     constexpr int TN = 4, BM = 8 * TMG, BN = TN * TNG, THREADS = TMG * TNG, STAGE = (BM + BN) * GF_LD;
     extern __shared__ __align__(16) float sm[];           // [stages][BM rows of x, BN rows of w][GF_LD]
     const int tid = threadIdx.x, ng = tid % TNG, mg = tid / TNG;
@@ -82,12 +84,12 @@ __global__ void __launch_bounds__(TMG* TNG) gemm_f32_kernel(const float* __restr
             cp_async_16(to + r * GF_LD + (p & 3) * 4, from + (size_t)min(first + r, all - 1) * K + (there ? k : 0), there);
         }
     };
-    // the weights are constant: their first tiles are requested before the kernel before has ended
-    for (int s = 0; s < GF_STAGES - 1 && s < steps; ++s) get(s, true);
-    rv_pdl_wait();
 #pragma unroll
     for (int s = 0; s < GF_STAGES - 1; ++s) {
-        if (s < steps) get(s, false);
+        if (s < steps) {
+            get(s, true);
+            get(s, false);
+        }
         cp_async_commit();
     }
     unsigned long long acc[8][TN];

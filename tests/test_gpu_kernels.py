@@ -656,6 +656,32 @@ def test_gemm_f32(ops, M, N, K):
     assert float((y.double().cpu() - ref).norm() / ref.norm()) < 1e-6
 
 
+@pytest.mark.parametrize("M,N,K", [(5, 4608, 1536), (64, 1536, 6912)])
+def test_gemm_f32_of_a_matrix_made_just_before(ops, M, N, K):
+    """The matrix may be what the launch before writes: a bfloat16 one is cast for float32 rows, and
+    a caller may update its matrix between two products.  Every product is of the new values; the
+    bound is the one above, of the terms' magnitudes."""
+    g = torch.Generator().manual_seed(M)
+    x = torch.randn(M, K, generator=g).cuda()
+    w16 = [(torch.randn(N, K, generator=g) * 0.05).bfloat16().cuda() for _ in range(2)]
+    bound = [(K / 2 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) for w in w16]
+    w32 = torch.empty(N, K, device="cuda")
+    ys = []
+    for i in range(12):
+        ys.append((i & 1, ops.linear(x, w16[i & 1])))          # cast, then multiplied
+        w32.copy_(w16[i & 1])
+        ys.append((i & 1, ops.linear(x, w32)))
+        ops.add_bias(w32, torch.ones(K, device="cuda"))        # a launch that lets the next one in early
+        ops.add_bias(w32, torch.full((K,), -1.0, device="cuda"))
+    for i, y in ys:
+        assert bool(((y.double() - x.double() @ w16[i].double().t()).abs() <= bound[i]).all())
+    w32.zero_()
+    ops.add_bias(w32, torch.ones(K, device="cuda"))
+    y = ops.linear(x, w32)
+    assert bool(((y.double() - x.double().sum(1, keepdim=True)).abs() <=
+                 (K / 2 + 16) * 2.0 ** -24 * x.double().abs().sum(1, keepdim=True)).all())
+
+
 PREFILL_CASES = [
     # q_lens, ctx_lens, heads, kv heads, head size, page size, window.  Head size 64: the
     # tcgen05 kernel (128 rows = tokens x heads of a group, tiles of 64 keys): group sizes
