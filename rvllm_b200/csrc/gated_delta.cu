@@ -570,12 +570,12 @@ static bool gd_shape(int d, int* R, int* P) {
     return false;
 }
 
-// Whether the portions of a step take the chunk form: where they are long enough on average that
-// chunks of 64 are not mostly filling.
+// Whether the portions of a step take the chunk form: with a decay per channel where the caller wants it,
+// per head where they are long enough on average that chunks of 64 are not mostly filling.
 static bool gd_chunked(int n_tokens, int n_decode, int n_reqs, int H, int G, int d, int dv, int head_decay, int chunks) {
     const int tokens = n_tokens - n_decode, reqs = n_reqs - n_decode;
-    return chunks && (head_decay ? gc_sizes_ok(H, G, d, dv) : gh_sizes_ok(H, G, d, dv)) && reqs > 0 &&
-           (head_decay ? tokens >= 24LL * reqs : gh_long_enough(tokens, reqs)) && tokens <= 65535 * CS_TOKENS;
+    return chunks && (head_decay ? gc_sizes_ok(H, G, d, dv) && tokens >= 24LL * reqs : gh_sizes_ok(H, G, d, dv)) &&
+           reqs > 0 && tokens > 0 && tokens <= 65535 * CS_TOKENS;
 }
 
 // Floats of a row of the scratch `prep`, and of the whole scratch for n tokens: the raw read-outs

@@ -632,10 +632,6 @@ static size_t gh_chunk_smem(int d, int dv) {
 static bool gh_sizes_ok(int H, int G, int d, int dv) {
     return d % 16 == 0 && d <= 128 && dv % 16 == 0 && (2 * G * d + H * dv) % 4 == 0 && gh_chunk_smem(d, dv) <= 220 * 1024;
 }
-// Which portions: the five launches take some 45 us whatever the lengths, the scan by token 20 us and 0.2 a
-// token of the longest (8 heads of 128 by 128: one request of 300 tokens 66 against 83 us, of 128 51
-// against 37; 8 requests of 64 tokens 69 against 74, of 32 64 against 49).
-static bool gh_long_enough(int tokens, int reqs) { return tokens >= 256 && tokens >= 48LL * reqs; }
 struct GhScratch {
     long long rows, logs, W, K, Q, S, U, Pm, V, dec, total;   // in floats, every part a multiple of four
 };

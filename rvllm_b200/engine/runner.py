@@ -46,7 +46,22 @@ class ModelRunner:
         self.captures = 0                # launch sequences captured so far
         self._graph_pool = None
         self.capture_failures = 0
+        # the lengths of a step's longest portion at which launches change (None: they do not follow
+        # it), and the context length up to which they are other ones (0: none)
+        self._portion_limits, self._shallow = self._launch_rules()
         self._reserve_workspace()
+
+    def _launch_rules(self) -> Tuple[Optional[tuple], int]:
+        from ..parts.base import mixer_class
+        limits, shallow = None, 0
+        spec = self.model.spec
+        for call in spec.order if self.use_graphs else ():
+            m = spec.layers[call.layer].mixer
+            rules = mixer_class(m.kind).launch_rules(m, self.ops)
+            if rules[0] is not None:
+                limits = tuple(sorted({*(limits or ()), *rules[0]}))
+            shallow = max(shallow, rules[1])
+        return limits, shallow
 
     def _reserve_workspace(self) -> None:
         """Size the kernels' shared scratch for the largest step this cache allows (padded
@@ -143,34 +158,54 @@ class ModelRunner:
             ctx.token_ids[:len(ordered)].copy_(device_tokens)
         return self.model.forward(ctx, self.cache.views())
 
+    def _mixture_sizes(self, ordered: List[StepEntry]) -> Optional[tuple]:
+        """What a step with prompt portions is padded to: (D, P, T, block-table width, longest
+        portion, deepest context).  The last two are what the kernels are told (`max_q_len`,
+        `max_ctx_len`).  Where launches follow the longest portion it is the next of 64, 96, 128,
+        192, 256, ... and of the lengths at which they change that holds the longest one (and
+        the tokens that fill the batch), else all tokens of the portions; where they are others
+        up to some context length, that length is the deepest context of the steps within it,
+        else what the block table holds.  None: more rows are wanted than come out."""
+        n_decode = 0
+        while n_decode < len(ordered) and len(ordered[n_decode].tokens) == 1:
+            n_decode += 1
+        portions = [len(e.tokens) for e in ordered[n_decode:]]
+        D = 0 if n_decode == 0 else 1 << (n_decode - 1).bit_length()
+        P = 1 << len(portions).bit_length()              # a power of two above their number
+        tokens = D + sum(portions)
+        gran = 64 if tokens <= 1024 else (128 if tokens <= 4096 else 256)
+        T = -(-tokens // gran) * gran
+        if sum(len(e.want) for e in ordered) > D + P:
+            return None
+        ps = self.cache.page_size
+        ctx_max = max(self.cache.requests[e.req].computed + len(e.tokens) for e in ordered)
+        blocks = -(-ctx_max // ps)
+        block_bucket = max(16, 1 << (blocks - 1).bit_length())
+        longest = max(1, T - D)
+        if self._portion_limits is not None:
+            most, size = max(portions + [T - tokens]), 64
+            while size < most:
+                size = size // 2 * 3 if size & (size - 1) == 0 else size // 3 * 4
+            longest = min([longest, size] + [n for n in self._portion_limits if n >= most])
+        deepest = block_bucket * ps
+        if ctx_max <= self._shallow:
+            deepest = min(deepest, self._shallow)
+        return D, P, T, block_bucket, longest, deepest
+
     def _run_padded_mixture(self, ordered: List[StepEntry], row_order=None) -> Optional[torch.Tensor]:
         """Steps with prompt portions, padded to sizes that come again: D single-token
         requests (a power of two), P prompt portions (a power of two, one more than there
-        are), T tokens in all (a multiple of 64, of 128 above 1,024, of 256 above 4,096) and a
-        block-table width as in single-token steps.  The second step that pads to the same
+        are), T tokens in all (a multiple of 64, of 128 above 1,024, of 256 above 4,096), a
+        block-table width as in single-token steps and what `_mixture_sizes` adds for some models.  The second step that pads to the same
         sizes is captured, and every later one replayed, whatever the portions' lengths and
         the requests are: in live traffic exact shapes hardly ever come twice, and a step of
         a small model launched kernel by kernel waits for the host (about 1.8 ms for some 140
         launches).  Returns None when this step has to go another way."""
         if self.max_mixed_graphs < 0:             # off; 0: the padded layout without captures
             return None
-        n_decode = 0
-        while n_decode < len(ordered) and len(ordered[n_decode].tokens) == 1:
-            n_decode += 1
-        n_prefill = len(ordered) - n_decode
-        D = 0 if n_decode == 0 else 1 << (n_decode - 1).bit_length()
-        P = 1 << n_prefill.bit_length()                  # a power of two above n_prefill
-        tokens = D + sum(len(e.tokens) for e in ordered[n_decode:])
-        gran = 64 if tokens <= 1024 else (128 if tokens <= 4096 else 256)
-        T = -(-tokens // gran) * gran
-        W = D + P
-        if sum(len(e.want) for e in ordered) > W:
+        key = self._mixture_sizes(ordered)
+        if key is None:
             return None
-        ps = self.cache.page_size
-        ctx_max = max(self.cache.requests[e.req].computed + len(e.tokens) for e in ordered)
-        blocks = -(-ctx_max // ps)
-        block_bucket = max(16, 1 << (blocks - 1).bit_length())
-        key = (D, P, T, block_bucket)
         g = self._mixed_graphs.get(key)
         if g is None:
             seen = ("mixed",) + key
@@ -216,11 +251,11 @@ class ModelRunner:
         """The step in the padded layout, launched kernel by kernel: the same kernels on the
         same sizes as the replayed launch sequence of these sizes, so a position's logits do
         not depend on whether its step had been captured yet."""
-        D, P, T, block_bucket = key
+        D, P, T, block_bucket, longest, deepest = key
         ctx = self.builder.build(ordered, pad_blocks=block_bucket, row_order=row_order,
                                  pad_mixed=(D, P, T, D + P))
-        ctx.max_ctx_len = block_bucket * self.cache.page_size
-        ctx.max_q_len = max(1, T - D)
+        ctx.max_ctx_len = deepest
+        ctx.max_q_len = longest
         return self.model.forward(ctx, self.cache.views())[:ctx.n_wanted]
 
     def _run_repeated_shape(self, ordered: List[StepEntry], row_order=None) -> Optional[torch.Tensor]:
@@ -232,8 +267,11 @@ class ModelRunner:
         ctx_max = max(self.cache.requests[e.req].computed + len(e.tokens) for e in ordered)
         blocks = -(-ctx_max // ps)
         block_bucket = max(16, 1 << (blocks - 1).bit_length())
+        deepest = block_bucket * ps
+        if ctx_max <= self._shallow:
+            deepest = min(deepest, self._shallow)
         key = (tuple(len(e.tokens) for e in ordered), tuple(tuple(e.want) for e in ordered),
-               block_bucket, tuple(row_order) if row_order is not None else None)
+               block_bucket, tuple(row_order) if row_order is not None else None, deepest)
         g = self._shape_graphs.get(key)
         if g is None:
             if key not in self._seen_shapes:
@@ -439,12 +477,12 @@ class _MixedGraph:
     """A captured launch sequence for steps of any mixture padded to (D single-token requests,
     P prompt portions, T tokens, block tables `block_bucket` wide): `BatchBuilder.build` with
     `pad_mixed`.  Its index arrays live at fixed addresses; a step refills them and replays.
-    Launch sizes that depend on a portion's length or a context's are taken from the padded
-    sizes, so that they cover every later replay."""
+    Launch sizes that depend on a portion's length or a context's are taken from the key, so
+    that they cover every later replay."""
 
     def __init__(self, runner: ModelRunner, key):
         self.runner = weakref.proxy(runner)     # no cycle: graphs die with their runner
-        self.D, self.P, self.T, self.block_bucket = key
+        self.D, self.P, self.T, self.block_bucket, self.longest, self.deepest = key
         self.last_used = 0
         R, W = self.D + self.P, self.D + self.P
         n_groups = len(runner.cache.groups)
@@ -462,8 +500,8 @@ class _MixedGraph:
         ctx = runner.builder.build(entries, pad_blocks=self.block_bucket,
                                    buffers=(self.host, self.dev), row_order=row_order,
                                    pad_mixed=(self.D, self.P, self.T, self.D + self.P))
-        ctx.max_ctx_len = self.block_bucket * runner.cache.page_size
-        ctx.max_q_len = max(1, self.T - self.D)
+        ctx.max_ctx_len = self.deepest
+        ctx.max_q_len = self.longest
         return ctx
 
     def run(self, entries, row_order=None) -> torch.Tensor:
@@ -497,7 +535,7 @@ class _ShapeGraph:
 
     def __init__(self, runner: ModelRunner, key, block_bucket: int):
         self.runner = weakref.proxy(runner)     # no cycle: graphs die with their runner
-        self.block_bucket = block_bucket
+        self.block_bucket, self.deepest = block_bucket, key[-1]
         n_tokens, n_reqs = sum(key[0]), len(key[0])
         n_want = sum(len(w) for w in key[1])
         n_groups = len(runner.cache.groups)
@@ -515,7 +553,7 @@ class _ShapeGraph:
         runner = self.runner
         ctx = runner.builder.build(entries, pad_blocks=self.block_bucket,
                                    buffers=(self.host, self.dev), row_order=row_order)
-        ctx.max_ctx_len = self.block_bucket * runner.cache.page_size
+        ctx.max_ctx_len = self.deepest
         if self.graph is None:
             launches = runner.model.ops.launches
             graph = torch.cuda.CUDAGraph()

@@ -105,6 +105,10 @@ class CudaOps:
         # portions of bfloat16 matrix memories: "chunks" = the chunk form on the tensor cores where the
         # sizes allow, "tokens" = token by token, "auto" = chunks where the longest portion is long
         self.mlstm_mode = os.environ.get("RVLLM_MLSTM", "auto")
+        # only steps whose longest portion has more tokens than this take the chunk forms of the matrix
+        # memory and of the delta rule with a decay per channel (the reasons are where they are asked)
+        self.mlstm_above = 384
+        self.gated_delta_above = 288
         # float32 products must be float32: no TF32, no reduced-precision accumulation
         torch.backends.cuda.matmul.allow_tf32 = False
         torch.backends.cudnn.allow_tf32 = False
@@ -590,6 +594,14 @@ class CudaOps:
         """Whether the values are the keys: one page tensor under both names."""
         return v_head_dim == head_dim and k_cache.data_ptr() == v_cache.data_ptr()
 
+    def attention_launch_rules(self, head_dim: int, v_head_dim: int):
+        """`Mixer.launch_rules` of `paged_attention` at these head sizes."""
+        tcgen05 = self.prefill_attention in ("auto", "tcgen05") and head_dim == v_head_dim == 128
+        return ((), self._shallow_128) if tcgen05 else (None, 0)
+
+    # contexts of one tile of keys: heads of 128 stay with the mma.sync kernel
+    _shallow_128 = 64
+
     def paged_attention(self, qkv, num_heads, num_kv_heads, head_dim, k_cache, v_cache,
                         ctx, group, scale, window, out, sinks=None, v_head_dim=None):
         """`sinks` float32 [heads]: one more term exp(sinks[h]) in head h's softmax denominator;
@@ -633,7 +645,7 @@ class CudaOps:
         # (heads of 128 with one tile of keys at most stay with mma.sync: 4 tokens 4.6 against 5.9 us,
         # 16 tokens 5.4 - 5.8 against 6.2; 64 tokens take 6.0 either way, 300 17 against 10)
         if (ctx.n_tokens > nd and self.prefill_attention in ("auto", "tcgen05") and vd == head_dim
-                and (head_dim == 64 or ctx.max_ctx_len > 64)
+                and (head_dim == 64 or ctx.max_ctx_len > self._shallow_128)
                 and self._tcgen05_prefill_ok(qkv, out, num_heads, num_kv_heads, head_dim,
                                              group.page_size)):
             self.paged_attention_prefill_tcgen05(qkv, num_heads, num_kv_heads, head_dim, k_cache,
@@ -1367,6 +1379,22 @@ class CudaOps:
         """Floats of one request's record: convolution inputs, then the state."""
         return (taps - 1) * (2 * kv_heads * dim + heads * vdim) + heads * dim * vdim
 
+    def _channel_chunks(self, ctx, n, heads, dim) -> bool:
+        """Whether the portions of a step are worth the chunk form with a decay per channel.  Its
+        launches take some 45 us and 4.3 us a chunk of 64 (8 heads of 128 by 128; heads of 64 2.1); the
+        scan by token 20 us and 0.2 us a token of the longest portion (heads of 64 0.14), but not
+        less than 0.12 us (0.045) a token of all.  So: a long portion (8 heads of 128: 257 tokens
+        57 us by token against 65 in chunks, 288 64 against 66, 320 92 against 66); not mostly short
+        ones beside it, whose chunks are filling (257 and 31 of 16: 113 against 162); and with heads
+        of 64 and fewer only while the longest is what the scan waits for (one of 400: 72 against
+        51, but 8 of 257: 98 against 114 and 16 of 300: 196 against 208).  The longest portion
+        and the count of requests may be padded ones: the first by half, hence 16 where exact
+        sizes would allow 24, the second towards the scan."""
+        single = getattr(ctx, "n_decode", 0)
+        longest, tokens, reqs = getattr(ctx, "max_q_len", n), n - single, ctx.n_reqs - single
+        return (longest > self.gated_delta_above and tokens >= 48 * reqs
+                and (dim > 64 or tokens * heads <= 16 * longest))
+
     def gated_delta(self, proj, lowrank, filt, a_log, dt_bias, norm_w, state, ctx, out, heads,
                     kv_heads, dim, vdim, taps, unit_eps, eps, head_decay=False, gate="sigmoid"):
         """The gated delta rule over the step's tokens, with a decay per key channel or, with
@@ -1390,7 +1418,8 @@ class CudaOps:
             raise KernelError("gated_delta: the decay and gate rows have another size")
         # the chunk forms read aligned rows; anything else goes token by token
         chunks = int(out.dtype == torch.bfloat16 and self.gated_delta_mode == "chunks"
-                     and (head_decay or ((2 * kv_heads * dim + heads * vdim) % 4 == 0
+                     and (head_decay or (self._channel_chunks(ctx, n, heads, dim)
+                                         and (2 * kv_heads * dim + heads * vdim) % 4 == 0
                                          and lowrank.stride(0) % 4 == 0
                                          and lowrank.data_ptr() % 16 == 0)))
         # the token-by-token form takes single tokens as any others
@@ -1519,11 +1548,14 @@ class CudaOps:
         if state.shape[1] != self.mlstm_record(heads, dim, vdim) or out.shape[1] != heads * vdim:
             raise KernelError("mlstm: the record or the output has another size")
         n = rows.shape[0]
-        # The chunk form's four launches take some 35 us whatever their portions' lengths, the scan
-        # some 8 us and 0.14 us a token of the longest one (8 heads of 64 by 128; 300 tokens: 44
-        # against 48 us, 64 tokens: 41 against 16, 2,048 tokens: 61 against 283).
+        # The longest portion decides.  The chunk form's launches take 32 - 50 us and little more for
+        # many portions, the scan some 8 us and 0.12 us a token of the longest one: 8 heads of 64 by
+        # 128 with 257 tokens 39 us by token against 43 in chunks, 320 40 against 41, 400 56 against
+        # 43, 512 73 against 44; 257 and 7 of 16 41 against 48; 8 of 60 39 against 48.  (Other sizes
+        # meet earlier, 16 heads at some 220 tokens, and many portions do: 8 of 128 58 against 50.)
         longest = getattr(ctx, "max_q_len", n)
-        chunks = int((self.mlstm_mode == "chunks" or (self.mlstm_mode == "auto" and longest >= 320))
+        chunks = int((self.mlstm_mode == "chunks"
+                      or (self.mlstm_mode == "auto" and longest > self.mlstm_above))
                      and self.lib.rv_mlstm_chunks_ok(
                          _ptr(rows), c_int(rows.shape[1]), c_int(_code(out.dtype)), c_int(heads),
                          c_int(dim), c_int(vdim), _ptr(out)))

@@ -140,6 +140,13 @@ class Attention(Mixer):
             return 0
         return sizer(max_requests, spec.num_heads, max(spec.head_dim, spec.v_head_dim), max_context)
 
+    @staticmethod
+    def launch_rules(spec: AttentionSpec, ops):
+        rules = getattr(ops, "attention_launch_rules", None)
+        if rules is None or spec.keep_first:
+            return None, 0
+        return rules(spec.head_dim, spec.v_head_dim or spec.head_dim)
+
     def __init__(self, spec: AttentionSpec, tensors, ops, dtype):
         if spec.num_heads % spec.num_kv_heads:
             raise ValueError(f"invalid attention head counts: {spec.num_heads} query, "

@@ -91,6 +91,11 @@ class LatentAttention(Mixer):
             return 0
         return sizer(max_requests, spec.num_heads, spec.kv_rank + spec.rot_dim, max_context)
 
+    @staticmethod
+    def launch_rules(spec: LatentAttentionSpec, ops):
+        rules = getattr(ops, "attention_launch_rules", None)
+        return (None, 0) if rules is None else rules(spec.kv_rank + spec.rot_dim, spec.kv_rank + spec.rot_dim)
+
     def __init__(self, spec: LatentAttentionSpec, tensors, ops, dtype):
         self.spec = spec
         self.ops = ops

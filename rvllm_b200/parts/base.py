@@ -100,6 +100,14 @@ class Mixer:
         runner reserves the largest answer once, before it captures any launch sequence."""
         return 0
 
+    @staticmethod
+    def launch_rules(spec, ops):
+        """(limits, shallow): None, or the lengths of a step's longest prompt portion above which
+        the mixer launches another form (none of them: only its launches' sizes follow that
+        length); and the context length up to which it launches another kernel (0: none).  A
+        replayed step has to have been captured with what these sizes choose."""
+        return None, 0
+
     def __init__(self, spec, tensors, ops, dtype):
         raise NotImplementedError
 

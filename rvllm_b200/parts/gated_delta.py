@@ -92,6 +92,11 @@ class GatedDelta(Mixer):
     def cache_need(spec: GatedDeltaSpec):
         return StateNeed((GatedDelta.record_size(spec),))
 
+    @staticmethod
+    def launch_rules(spec: GatedDeltaSpec, ops):
+        limit = getattr(ops, "gated_delta_above", None)
+        return (None, 0) if limit is None or spec.decay == "head" else ((limit,), 0)
+
     def __init__(self, spec: GatedDeltaSpec, tensors, ops, dtype):
         self._check(spec)
         self.spec = spec

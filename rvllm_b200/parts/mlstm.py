@@ -61,6 +61,11 @@ class MLSTM(Mixer):
     def cache_need(spec: MLSTMSpec):
         return StateNeed((MLSTM.record_size(spec),))
 
+    @staticmethod
+    def launch_rules(spec: MLSTMSpec, ops):
+        limit = getattr(ops, "mlstm_above", None)
+        return (None, 0) if limit is None else ((limit,), 0)
+
     def __init__(self, spec: MLSTMSpec, tensors, ops, dtype):
         self._check(spec)
         self.spec = spec

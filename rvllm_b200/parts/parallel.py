@@ -53,6 +53,12 @@ class Parallel(Mixer):
         return max(mixer_class(b.kind).workspace_bytes(b, ops, max_requests, max_context)
                    for b in spec.branches)
 
+    @staticmethod
+    def launch_rules(spec: ParallelSpec, ops):
+        rules = [mixer_class(b.kind).launch_rules(b, ops) for b in spec.branches]
+        limits = [r[0] for r in rules if r[0] is not None]
+        return sum(limits, ()) if limits else None, max(r[1] for r in rules)
+
     def __init__(self, spec: ParallelSpec, tensors, ops, dtype):
         self._check(spec)
         self.spec = spec

@@ -61,3 +61,82 @@ def test_float32_product_leaves_other_devices_and_gradients(ops):
     with torch.no_grad():
         ops.linear(on_device(8, 512), on_device(300, 512, grad=True))
     assert len(ops.calls) == 1
+
+
+class Cuda(OnDevice):
+    is_cuda = True
+
+
+def cuda(*shape, dtype=torch.float32):
+    return torch.zeros(*shape, dtype=dtype).as_subclass(Cuda)
+
+
+def forms(ops, lens, longest=None, heads=8, dim=64, singles=0, reqs=None):
+    """Whether a step of these portions takes the chunk forms of the matrix memory and of the delta
+    rule with a decay per channel; `longest`, `reqs`: what the step says, when it is padded."""
+    n, taken = sum(lens) + singles, {}
+    ctx = SimpleNamespace(n_decode=singles, n_reqs=singles + (reqs or len(lens)), max_q_len=longest or max(lens),
+                          token_req=None, q_start=None, state_slot=None)
+    value = lambda a: a.value if hasattr(a, "value") else a
+    ops.mlstm_mode, ops.mlstm_above, ops.gated_delta_mode, ops.gated_delta_above = "auto", 384, "chunks", 288
+    ops.lib.rv_mlstm_chunks_ok = lambda *a: 1
+    ops.lib.rv_mlstm_scratch = ops.lib.rv_gated_delta_scratch = lambda *a: 0
+    ops.lib.rv_mlstm = lambda *a: taken.update(memory=bool(value(a[-2]))) or 0
+    ops.lib.rv_gated_delta = lambda *a: taken.update(delta=bool(value(a[-2]))) or 0
+    ops.mlstm(cuda(n, 4 * heads * dim + 2 * heads), cuda(heads), cuda(heads), cuda(heads * dim),
+              cuda(1, heads * (dim + 1) * dim + heads), ctx, cuda(n, heads * dim, dtype=torch.bfloat16),
+              heads, dim, dim, 5.0, 1e-5)
+    C = 3 * heads * dim
+    ops.gated_delta(cuda(n, C + heads), cuda(n, 2 * heads * dim), cuda(C, 4), cuda(heads), cuda(heads * dim),
+                    cuda(dim), cuda(1, 3 * C + heads * dim * dim), ctx, cuda(n, heads * dim, dtype=torch.bfloat16),
+                    heads, heads, dim, dim, 4, 1e-6, 1e-5)
+    return taken["memory"], taken["delta"]
+
+
+def test_chunk_forms_are_for_long_portions(ops):
+    """By the longest portion, not by the tokens of all; the delta rule's also by how full its chunks
+    are and, for small heads, by whether the scan waits for the longest portion alone."""
+    assert forms(ops, [60] * 8) == (False, False)
+    assert forms(ops, [288]) == (False, False) and forms(ops, [384]) == (False, True)
+    assert forms(ops, [400]) == (True, True) and forms(ops, [1489, 559]) == (True, True)
+    assert forms(ops, [400] + [16] * 31) == (True, False)
+    assert forms(ops, [400], singles=31) == (True, True)
+    assert forms(ops, [400] * 8) == (True, False)
+    assert forms(ops, [400] * 8, dim=128) == (True, True)
+    assert forms(ops, [400] * 8, dim=128, heads=16) == (True, True)
+
+
+def sizes_of(lens, limits, shallow=0, context=0, page=16):
+    from rvllm_b200.engine.batch import StepEntry
+    from rvllm_b200.engine.runner import ModelRunner
+    r = object.__new__(ModelRunner)
+    r._portion_limits, r._shallow = limits, shallow
+    r.cache = SimpleNamespace(page_size=page, requests={i: SimpleNamespace(computed=context) for i in range(len(lens))})
+    return r._mixture_sizes([StepEntry(i, (0,) * n, (0,)) for i, n in enumerate(lens)])
+
+
+@pytest.mark.parametrize("lens", [[60] * 8, [40] * 8, [1] * 8 + [48] * 10, [288], [289], [300, 20, 20], [384], [385],
+                                  [400], [700], [2000], [1, 1, 1, 260], [257, 257, 257], [30] * 31])
+def test_padded_steps_choose_as_exact_ones(ops, lens):
+    """What a padded step tells the kernels about its longest portion chooses the same form of the
+    matrix memory as the portions themselves, and covers every request's tokens, the filling ones
+    included; the delta rule's may stay with the scan, but takes chunks only where the portions do."""
+    single = sum(n == 1 for n in lens)
+    portions = lens[single:]
+    D, P, T, _, longest, deepest = sizes_of(lens, (288, 384))
+    assert longest >= max(portions) and longest >= T - D - sum(portions) and longest <= T - D
+    assert deepest == sizes_of(lens, None)[5] and sizes_of(lens, None)[4] == T - D
+    tail = [T - D - sum(portions)]
+    for dim in (64, 128):
+        exact = forms(ops, portions, singles=single, dim=dim)
+        padded = forms(ops, portions + tail, longest=longest, singles=D, reqs=P, dim=dim)
+        assert padded[0] == exact[0] and padded[1] <= exact[1], (dim, exact, padded)
+
+
+def test_padded_steps_of_shallow_contexts():
+    """Where attention has another kernel for short contexts, steps within them are told so."""
+    assert sizes_of([20, 30], (), shallow=64)[5] == 64
+    assert sizes_of([20, 30], (), shallow=64, context=34)[5] == 64
+    assert sizes_of([20, 30], (), shallow=64, context=35)[5] == 256
+    assert sizes_of([20, 30], None, shallow=0)[5] == 256
+    assert sizes_of([20, 30], (), shallow=64, page=2)[5] == 32

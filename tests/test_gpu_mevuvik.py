@@ -365,6 +365,32 @@ def test_matrix_memory_chunks(ops, sizes, strong):
             assert abs(float(recd[H * (dv + 1) * d + h]) - mx) < 1e-5 * max(1.0, abs(mx))
 
 
+def test_matrix_memory_alone_and_beside_a_long_portion(ops):
+    """A request of 100 tokens goes token by token alone and in chunks beside one of 500: the same
+    record within the float32 bound of the chunk form, the same output within bfloat16's."""
+    H, d, dv, W = 2, 64, 128, 32
+    t, g = _memory_case(H, d, dv, W, 5)
+    w_in = np.concatenate([t[k] for k in ("q", "k", "v", "i", "f", "g")])
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    rows = [dev(torch.from_numpy(rnd(g, torch.float32, n, W).numpy() @ w_in.T).float()) for n in (100, 500)]
+    got = []
+    for parts, launches in ((rows[:1], 3), (rows, 5)):
+        lens = [len(x) for x in parts]
+        state = torch.zeros(2, ops.mlstm_record(H, d, dv), device="cuda")
+        x = torch.cat(parts)
+        ctx = SimpleNamespace(q_start=i32(np.cumsum([0] + lens).tolist()), state_slot=i32([0, 1][:len(lens)]),
+                              token_req=i32(sum(([i] * n for i, n in enumerate(lens)), [])), n_reqs=len(lens),
+                              n_decode=0, max_q_len=max(lens))
+        out = torch.empty(len(x), H * dv, device="cuda", dtype=torch.bfloat16)
+        before = ops.launches
+        ops.mlstm(x, dev(torch.from_numpy(t["i.b"]).float()), dev(torch.from_numpy(t["f.b"]).float()),
+                  dev(torch.from_numpy(t["norm"]).float()), state, ctx, out, H, d, dv, 5.0, 1e-5)
+        assert ops.launches - before == launches
+        got.append((out[:100].cpu(), state[0].cpu()))
+    close(got[1][0], got[0][0].double(), torch.bfloat16)
+    close(got[1][1], got[0][1].double(), torch.float32, bound=3e-5)
+
+
 def test_matrix_memory_long_and_with_strong_gates(ops):
     """600 tokens with input gates far above and forget gates far below the cap's middle: the
     running maximum keeps every exponential in range, and the first tokens still show."""
