@@ -10,12 +10,14 @@
 // tiles of 64 would work 192).  Small products have few tiles: their K is split over a cluster of up to
 // eight blocks, which leave their tiles in shared memory and add them in rank order.
 //
-// Bound by the weights' bytes up to some 16 rows, above by the multiply-adds' loads (30 - 40 of 74
-// TFLOP/s).  The library's float32 products take tiles of 32 x 32 to 64 x 128 on the same cores, without
-// a split of K; at equal sizes (us, N x K): 1 row 4608 x 1536 39 -> 16, 13824 x 1536 52 -> 27,
-// 1536 x 6912 80 -> 36, 65536 x 1024 117 -> 77; 16 rows 39 -> 18, 52 -> 37, 81 -> 41, 117 -> 88; 64 rows
-// 1536 x 1536 28 -> 19, 1536 x 6912 109 -> 70; 131 rows 36 -> 30, 166 -> 121.  With many rows and columns it
-// is the slower one (131 rows 13824 x 1536 188 -> 209, 2,048 rows 1,377 -> 2,111), see rv_gemm_f32_better.
+// Bound by the multiply-adds' loads from some 32 rows on (30 - 40 of 74 TFLOP/s).  With fewer rows by
+// latency, not by the matrix's bytes: up to 8 rows a block is one warp and K is split eight ways at most, so
+// N = 1,536 gives 96 warps to 148 multiprocessors (1 row: 12 % of the bytes' time at 1536 x 6912, 24 %
+// at 4608 x 1536, 45 % at 65536 x 1024).  The library's float32 products take tiles of 32 x 32 to 64 x 128
+// on the same cores; at equal sizes (us, N x K): 1 row 4608 x 1536 39 -> 18, 13824 x 1536 52 -> 29, 1536 x
+// 6912 79 -> 52, 65536 x 1024 113 -> 92; 16 rows 39 -> 19, 52 -> 37, 79 -> 50, 113 -> 84; 64 rows 1536 x 1536
+// 38 -> 19, 1536 x 6912 110 -> 68; 144 rows 36 -> 32, 156 -> 127.  With many rows and columns it is the slower
+// one (131 rows 13824 x 1536 188 -> 209, 2,048 rows 1,377 -> 2,111), see rv_gemm_f32_better.
 // Operands in three bfloat16 parts on mma.sync were measured too: 131 rows 13824 x 1536 147 us, but
 // slower than the library below 96 rows and above 144, and than this at N = 1536.
 // Its sums are nearer to float64 (relative error 2 - 4e-7 at these sizes, the library's 3e-7 - 1.5e-6).
@@ -178,11 +180,26 @@ static cudaError_t gf_launch(const float* x, const float* w, float* y, int M, in
     return cudaLaunchKernelEx(&cfg, gemm_f32_kernel<TMG, TNG>, x, w, y, M, N, K, per_split);
 }
 
-// Whether this kernel is the faster one (us here / the library's): 16 rows or fewer (above); 64 rows and
-// some 6,000 columns (4608 x 1536: 32 rows 24 / 39, 64 rows 37 / 40, but 13824 x 1536 32 rows 54 / 52);
-// 160 rows and some 2,000 columns (1536 x 1536: 131 rows 30 / 36, 200 rows 43 / 43).
+// Whether this kernel is the faster one.  Both sides were measured at 256 to 6,912 of K, 256 to 65,536
+// columns and 1 to 160 rows, and at sizes drawn between them, matrices beyond L2 (us here / the library's):
+//   K below 512 (1,024 with fewer than 1,536 or more than 6,144 columns or more than 16 rows): a launch of few steps, whose
+//     cluster is not repaid: 256 x 256 8 rows 12 / 7, 64 rows 10 / 7; 1209 x 828 11 rows 14 / 13; 18291 x 780 14 rows 35 / 28.
+//   up to 16 rows: 4608 x 512 11 / 15, 1536 x 1536 14 / 27, 4608 x 4096 45 / 102.  K above 2,048 with
+//     fewer columns than 1,536 is even with the library, which splits K too (256 x 4096 32 / 30).
+//   up to 32 rows: 512 x 1024 9 / 14, 6144 x 1024 17 / 27, but 9216 x 1024 29 / 28.
+//   up to 64 rows: 1024 x 1024 12 / 26, 4608 x 1536 37 / 40, 6144 x 1024 32 / 32; 897 x 2164 26 / 23, 9216 x
+//     1024 46 / 35.
+//   up to 144 rows (three tiles of 48): 1536 x 1024 22 / 25, 1536 x 1536 32 / 36, but 160 rows 27 / 25 and
+//     37 / 36; 428 x 3624 119 rows 46 / 34.
+//   2,048 columns: to 96 rows 18 / 26 (K 1,024), to 128 rows from K 1,536 on 35 / 37; 2,560: 30 / 30.
 extern "C" int rv_gemm_f32_better(int M, int N, int K) {
-    return K % 4 == 0 && K >= 256 && N >= 256 && (M <= 16 || (M <= 64 && N <= 6144) || (M <= 160 && N <= 2048));
+    if (K % 4 || K < 512 || N < 256) return 0;
+    if (K < 1024) return M <= 16 && N >= 1536 && N <= 6144;
+    if (M <= 16) return K <= 2048 || N >= 1536;
+    if (M <= 32) return N <= 6144;
+    if (N < 1024) return 0;
+    if (M <= 64) return N <= 6144;
+    return (M <= 144 && N <= 1536) || (M <= (K >= 1536 ? 128 : 96) && N <= 2048);
 }
 
 // K a multiple of 4, x and w on 16-byte boundaries.

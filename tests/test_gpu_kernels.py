@@ -3,12 +3,14 @@ other than the engine's: widths that are no power of two, head sizes 48 and 80, 
 of 3, pages of 8, filters of 2 to 5 taps."""
 import math
 import random
+from ctypes import c_int
 from types import SimpleNamespace
 
 import pytest
 import torch
 
 from plain_ops import PlainOps, sample_row, uniform
+from rvllm_b200.kernels.bindings import _ptr
 
 pytestmark = pytest.mark.gpu
 
@@ -646,10 +648,16 @@ def test_gemm_f32(ops, M, N, K):
     w = torch.randn(N, K, generator=g) * 0.05
     x[M // 2, K // 3] = 40.0
     w[N // 5, K // 3] = 3.0
-    assert ops.lib.rv_gemm_f32_better(M, N, K)
     before = ops.launches
     y = ops.linear(x.cuda(), w.cuda())
-    assert ops.launches == before + 1                      # the kernel, not the library
+    chosen = ops.lib.rv_gemm_f32_better(M, N, K)
+    assert ops.launches == before + (1 if chosen else 0)   # the kernel, or the library
+    assert chosen == ((M, N, K) in ((8, 300, 1028), (24, 4608, 1536), (32, 1001, 2052),
+                                    (65, 1536, 6912)))
+    if not chosen:                                         # sizes at which the library is faster
+        xd, wd = x.cuda(), w.cuda()
+        y = torch.empty(M, N, device="cuda")
+        assert ops.lib.rv_gemm_f32(_ptr(xd), _ptr(wd), _ptr(y), c_int(M), c_int(N), c_int(K), ops._stream()) == 0
     ref = x.double() @ w.double().t()
     bound = (K / 2 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
     assert bool(((y.double().cpu() - ref).abs() <= bound).all())
