@@ -20,11 +20,11 @@
 // done, and the ring has three stages.
 //
 // Head size 64: 65 KB of shared memory and 128 TMEM columns per block: three blocks share an SM,
-// so one block's softmax overlaps the others' copies and MMAs; 128: 112 KB (96 KB with RV_SAME) and
+// so one block's softmax overlaps the others' copies and MMAs; 128: 113 KB (97 KB with RV_SAME) and
 // 256 columns, two blocks.
 // Head size 128 against the mma.sync kernel (us; pages of 16): latent rows, 16 heads: 2,048 tokens 93 ->
 // 42, 1,000 tokens 48 -> 23, 300 tokens 15 -> 11, 256 tokens after 3,840 162 -> 27, window 512 57 -> 21;
-// 32 heads: 2,048 tokens 173 -> 54; 32 / 8 heads with values of their own: 234 -> 90.  At head size 64
+// 32 heads: 2,048 tokens 173 -> 54; 32 / 8 heads with values of their own: 233 -> 66.  At head size 64
 // the exponent's offset follows the row maximum lazily (it moves only when the maximum has grown by
 // more than 2^8), so O is rescaled on few tiles.  Heads of 128 move it with the maximum and divide by
 // the sum of the rounded P, as the mma.sync kernel that they ran on before does: a row's largest P is
@@ -175,6 +175,23 @@ __device__ __forceinline__ unsigned long long at_desc(const void* tile) {
     return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// What the warps meet at: static memory, but for heads of 128 with values of their own.  Two of their
+// blocks would be 256 bytes more than a multiprocessor has, so there it lies in what the tiles'
+// alignment leaves of the dynamic memory (32 / 8 heads, 2,048 tokens: 89 us with one block a
+// multiprocessor, 66 with two; latent rows, which have two either way: 53 static, 62 so).
+#define AT_BARRIERS_DYNAMIC (RV_HD == 128 && !RV_SAME)
+struct AtShared {
+    unsigned long long q_bar, s_bar, pv_bar, s_read, p_ready;
+    unsigned long long k_full[AT_STAGES], k_empty[AT_STAGES], v_full[AT_STAGES], v_empty[AT_STAGES];
+    unsigned tmem_base;
+    volatile int failed;
+};
+static_assert(sizeof(AtShared) <= 512, "fits the larger part of the alignment's bytes");
+template <int HD>
+constexpr size_t at_tile_bytes() {
+    return (size_t)(AT_ROWS * HD + AT_STAGES * AT_TILES * AT_KEYS * HD + AT_ROWS * AT_KEYS) * sizeof(bf16);
+}
+
 template <int HD>
 __global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill_tcgen05_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -223,11 +240,19 @@ __global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill
     bf16* q_tile = (bf16*)base;                                 // [halves][128 rows][64]
     bf16* kv_ring = q_tile + AT_ROWS * HD;                      // [stages][K tile, V tile][halves][64 keys][64]
     bf16* p_tile = kv_ring + (size_t)AT_STAGES * AT_TILES * TILE;   // [128 rows][64 keys]
-    __shared__ __align__(8) unsigned long long q_bar, s_bar, pv_bar, s_read, p_ready;
-    __shared__ __align__(8) unsigned long long k_full[AT_STAGES], k_empty[AT_STAGES];
-    __shared__ __align__(8) unsigned long long v_full[AT_STAGES], v_empty[AT_STAGES];
-    __shared__ unsigned tmem_base_smem;
-    __shared__ volatile int failed;
+#if AT_BARRIERS_DYNAMIC
+    // the 1,024 bytes that the alignment may take lie before the tiles or behind them: the larger
+    // part has at least 512
+    AtShared& sh = *(AtShared*)(base - smem_raw >= 512 ? smem_raw : base + at_tile_bytes<HD>());
+#else
+    __shared__ AtShared sh;
+#endif
+    unsigned long long &q_bar = sh.q_bar, &s_bar = sh.s_bar, &pv_bar = sh.pv_bar, &s_read = sh.s_read,
+                       &p_ready = sh.p_ready;
+    unsigned long long(&k_full)[AT_STAGES] = sh.k_full, (&k_empty)[AT_STAGES] = sh.k_empty;
+    unsigned long long(&v_full)[AT_STAGES] = sh.v_full, (&v_empty)[AT_STAGES] = sh.v_empty;
+    unsigned& tmem_base_smem = sh.tmem_base;
+    volatile int& failed = sh.failed;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
@@ -695,6 +720,26 @@ static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window
     return parts < 1 ? 1 : parts;
 }
 
+static int at_configure(size_t smem) {
+    static bool configured = false;
+    if (configured) return 0;
+    cudaError_t e = cudaFuncSetAttribute(paged_attention_prefill_tcgen05_kernel<RV_HD>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return at_fail(cudaGetErrorString(e));
+    configured = true;
+    return 0;
+}
+// Shared memory of a block, all that counts against a multiprocessor's (-1: an error).
+extern "C" long long AT_SYM(rv_paged_attention_prefill_tcgen05_shared_bytes)() {
+    cudaFuncAttributes a;
+    int dev = 0, reserved = 0;
+    if (cudaFuncGetAttributes(&a, paged_attention_prefill_tcgen05_kernel<RV_HD>) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
+        return -1;
+    return (long long)(at_tile_bytes<RV_HD>() + 1024 + a.sharedSizeBytes + reserved);
+}
+
 // Requests [first_req, first_req + n_reqs), the longest bringing max_q_len tokens and holding
 // max_ctx_len; `q` is the q|k|v buffer [n_tokens, q_stride] (the query heads first), `out` is
 // [n_tokens, heads * head size]; `scratch` (may be null: no sharing out) holds the parts.
@@ -724,15 +769,8 @@ extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
                page_size, 1))
         return 1;
     if (RV_SAME && k_cache != v_cache) return at_fail("paged_attention_prefill_tcgen05: the values are not the keys");
-    const size_t smem = (size_t)(AT_ROWS * RV_HD + AT_STAGES * AT_TILES * AT_KEYS * RV_HD + AT_ROWS * AT_KEYS) *
-                            sizeof(bf16) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(paged_attention_prefill_tcgen05_kernel<RV_HD>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return at_fail(cudaGetErrorString(e));
-        configured = true;
-    }
+    const size_t smem = at_tile_bytes<RV_HD>() + 1024;
+    if (at_configure(smem)) return 1;
     const int nqb = (max_q_len + q_block - 1) / q_block;
     const long long blocks = (long long)num_kv_heads * nqb * n_reqs;
     const int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;

@@ -789,6 +789,17 @@ def test_prefill_attention_head_size_128_rounds_alike(ops, lens, same):
     assert float((outs[0] - outs[1]).norm() / outs[1].norm()) < 4.9e-4
 
 
+@pytest.mark.parametrize("head_dim,same,blocks", [(64, False, 3), (128, False, 2), (128, True, 2)])
+def test_prefill_attention_blocks_a_multiprocessor(ops, head_dim, same, blocks):
+    """As many blocks' shared memory fits a multiprocessor as the kernel's bounds are set for, so
+    that one block's softmax runs beside another's copies and products."""
+    need = getattr(ops._attn5_lib(head_dim, same),
+                   f"rv_paged_attention_prefill_tcgen05_shared_bytes_hd{head_dim}")()
+    # a block's memory is given out in pieces of 128 bytes
+    assert 0 < blocks * (-(-need // 128) * 128) <= \
+        torch.cuda.get_device_properties(0).shared_memory_per_multiprocessor
+
+
 def test_prefill_attention_tcgen05_is_used(ops):
     """The default choice takes the tcgen05 kernel where it applies (its launch is counted by
     its own library) and refuses nothing it cannot do: other head sizes go to the mma kernel."""
