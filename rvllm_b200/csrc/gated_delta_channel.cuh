@@ -13,7 +13,10 @@
 // are made in blocks of 16 by 16 tokens: below the diagonal blocks the decay from j to i passes the
 // first token of i's block, e^(from there to i) and e^(from j to there), neither above 1, go to the two
 // operands of a product; within a diagonal block every pair's own power is taken.  The sums start anew in
-// every block of 16, forwards and backwards, so that no exponent is a difference of large ones.
+// every block of 16, forwards and backwards.  Only within a diagonal block an exponent is a difference of
+// two sums, which are large behind a token that forgets strongly; there a sum is a float32 and what its
+// additions lost (a bfloat16: some 2^-33 of it), so that the difference has its own float32 precision.  A
+// log decay below -192 counts as -192: either way the power, and every power across the token, is 0.
 //
 //   gch_logs    log decays -> [n, H d]
 //   conv_silu   q | k | v pass the convolutions and silu -> rows [n, C] float32 (conv_silu.cuh)
@@ -38,6 +41,7 @@
 
 #define GH_THREADS 512      // threads of a block of gch_chunk
 #define GH_LOG2E 1.4426950408889634f
+#define GH_NOTHING -192.f   // a power of two that is no float32, whatever it is multiplied by
 
 struct GhArgs {
     const float *proj, *lowrank, *a_log, *dt_bias;
@@ -56,6 +60,12 @@ __device__ __forceinline__ float gh_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Four of them, on a 4-byte boundary.
+__device__ __forceinline__ void gh_lost(const bf16* p, float (&x)[4]) {
+    const float2 a = lm_pair(*(const unsigned*)p), b = lm_pair(*(const unsigned*)(p + 2));
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
 // The log decays (powers of two) of the portions' tokens, four channels a thread.
@@ -83,7 +93,8 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int d = 16 * UNITS, LD = d + 8, UP = (UNITS + 1) / 2;
     float* As = (float*)smraw;                            // [64][65]
-    float* Xs = As + 64 * 65;                             // [64][65]: the inverse
+    float* Xs = As + 64 * 65;                             // [64][65]: the inverse; before it
+    bf16* ls = (bf16*)Xs;                                 // [64][d + 2]: what the sums bs have lost
     float* tot = Xs + 64 * 65;                            // [4][d]: a block of 16's sum; before it; behind it
     float *pre = tot + 4 * d, *post = pre + 4 * d;
     float* ks = post + 4 * d;                             // [64][LD] each: keys, queries, the sums of the
@@ -155,9 +166,15 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) l[i] = bs[(16 * J + i) * LD + c];
 #pragma unroll
+        for (int i = 0; i < 16; ++i) l[i] = l[i] < GH_NOTHING ? GH_NOTHING : l[i];       // (NaN stays)
+        float lost = 0.f;
+#pragma unroll
         for (int i = 0; i < 16; ++i) {
-            s += l[i];
+            const float t = s + l[i], z = t - s;
+            lost += (s - (t - z)) + (l[i] - z);
+            s = t;
             bs[(16 * J + i) * LD + c] = s;
+            ls[(16 * J + i) * (d + 2) + c] = __float2bfloat16_rn(lost);
         }
         tot[J * d + c] = s;
         s = 0.f;
@@ -178,7 +195,7 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, p[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 2
         for (int c = (tid & 1) * 4; c < d; c += 8) {
-            float ki[2][4], qi[2][4], bi[2][4], kj[2][4], bj[2][4];
+            float ki[2][4], qi[2][4], bi[2][4], kj[2][4], bj[2][4], li[2][4], lj[2][4];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 la_load<float, 4>(ks + (i0 + e) * LD + c, ki[e]);
@@ -186,6 +203,8 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
                 la_load<float, 4>(bs + (i0 + e) * LD + c, bi[e]);
                 la_load<float, 4>(ks + (j0 + e) * LD + c, kj[e]);
                 la_load<float, 4>(bs + (j0 + e) * LD + c, bj[e]);
+                gh_lost(ls + (i0 + e) * (d + 2) + c, li[e]);
+                gh_lost(ls + (j0 + e) * (d + 2) + c, lj[e]);
             }
 #pragma unroll
             for (int x = 0; x < 4; ++x)
@@ -193,7 +212,7 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const float w = kj[j][x] * gh_exp2(bi[i][x] - bj[j][x]);
+                        const float w = kj[j][x] * gh_exp2((bi[i][x] - bj[j][x]) + (li[i][x] - lj[j][x]));
                         s[i][j] = fmaf(ki[i][x], w, s[i][j]);
                         p[i][j] = fmaf(qi[i][x], w, p[i][j]);
                     }

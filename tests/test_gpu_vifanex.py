@@ -379,6 +379,35 @@ def test_gated_delta_channel_chunks(ops, sizes, decays):
             close(S, want[i][1], torch.float32, scale=max(1.0, float(np.abs(want[i][1]).max())))
 
 
+@pytest.mark.parametrize("log_decay", [50.0, 300.0, 3e38])
+@pytest.mark.parametrize("d", [64, 128])
+def test_gated_delta_channel_chunks_behind_a_token_that_forgets(ops, d, log_decay):
+    """One token in sixteen forgets by e^-50, by e^-300 or altogether (its log decay is no float32),
+    the others next to nothing.  In the chunk form the powers between the tokens behind it must
+    not suffer from the size of the sums: the state's error against float64 is no more than
+    four roundings of a weight (2.4e-7) above what the form token by token shows."""
+    H, G, dv, taps, T = 2, 1, 64, 1, 330
+    g = torch.Generator().manual_seed(d)
+    proj, low, filt, _, _, norm_w = delta_case(g, T, H, G, d, dv, taps)
+    a_log, dt_bias = torch.ones(H, dtype=torch.float64), torch.zeros(H * d, dtype=torch.float64)
+    low[:, :H * d] -= 5.0
+    low[5::16, :H * d] = log_decay
+    want = plain_delta(proj.numpy(), low.numpy(), filt.numpy(), a_log.numpy(), dt_bias.numpy(), norm_w.numpy(),
+                       H, G, d, dv, 1e-5)[1]
+    errors, was = [], ops.gated_delta_mode
+    try:
+        for mode in ("chunks", "tokens"):
+            ops.gated_delta_mode = mode
+            _, state = run_delta(ops, [(proj, low)], (T,), H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, 1e-5,
+                                 torch.bfloat16, [0])
+            S = state[0].reshape(H, dv, d).transpose(1, 2).double().cpu().numpy()
+            errors.append(float(np.linalg.norm(S - want) / np.linalg.norm(want)))
+    finally:
+        ops.gated_delta_mode = was
+    print(errors)
+    assert errors[0] < errors[1] + 4 * 2.0 ** -24, errors
+
+
 def test_gated_delta_order_within_a_token(ops):
     """Decay, then the correction with the decayed state, then the read-out of the written
     state: one head, two tokens, numbers worked by the plain step."""
