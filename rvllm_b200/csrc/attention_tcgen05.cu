@@ -707,10 +707,14 @@ static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window
     // the tiles every block of query tokens has before its own: a whole prompt (none before it)
     // is a triangle of mostly short blocks, which sharing out only burdens (1,000 tokens alone:
     // 22.7 -> 29.2 us with two parts); four such tiles to a part at least
-    // (within the window, where there is one: 333 tokens after 1,001 with a window of 300, 32 heads of
-    // 128: 28.6 us shared out over three blocks each, 14.0 us whole)
+    // (within the window, where there is one and blocks are not so few that shares of two tiles pay
+    // too: us by the window / by the whole context, 32 / 8 heads: of 128, 333 tokens after 1,001 window
+    // 300 (88 blocks) 15 / 26, 100 + 60 tokens window 256 (64) 13 / 20, 64 after 4,032 window 512 (16) 15 /
+    // 12; 16 / 1 heads of 128, 26 blocks 11 / 13, 8 blocks 14 / 11; heads of 64, 88 blocks 12.5 / 16.3,
+    // 64 blocks 14.6 / 16.5, 16 / 8 heads 48 blocks 12.3 / 12.0, 32 blocks 13.4 / 12.3, 8 blocks 12 / 9)
+    const bool few = blocks < (RV_HD == 64 ? 64 : 24) && window >= 4 * AT_KEYS;
     int earlier = max_ctx_len > max_q_len ? max_ctx_len - max_q_len : 0;
-    if (window > 0 && earlier > window) earlier = window;
+    if (window > 0 && !few && earlier > window) earlier = window;
     const int before = earlier / AT_KEYS;
     if (forced <= 0 && parts > before / 4) parts = before / 4;
     if (parts > AT_MAX_PARTS) parts = AT_MAX_PARTS;

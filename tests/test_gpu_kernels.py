@@ -711,6 +711,9 @@ PREFILL_CASES = [
     ([100, 7], [3000, 900], 4, 4, 64, 32, None),
     ([64], [1800], 8, 2, 64, 16, 700),
     ([30], [8100], 8, 2, 64, 16, None),           # 16 parts
+    # with a window, shared out by the tiles within it: many blocks; a window of fewer than four tiles
+    ([100, 60], [900, 1000], 32, 8, 64, 16, 300),
+    ([40], [2000], 8, 2, 64, 16, 200),
 ]
 
 
