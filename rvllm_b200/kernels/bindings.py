@@ -599,8 +599,21 @@ class CudaOps:
         tcgen05 = self.prefill_attention in ("auto", "tcgen05") and head_dim == v_head_dim == 128
         return ((), self._shallow_128) if tcgen05 else (None, 0)
 
-    # contexts of one tile of keys: heads of 128 stay with the mma.sync kernel
+    # contexts of one tile of keys: heads of 128 stay with the mma.sync kernel (4 tokens 4.6 against
+    # 5.9 us, 16 tokens 5.4 - 5.8 against 6.2; 64 tokens take 6.0 either way, 300 17 against 10)
     _shallow_128 = 64
+
+    def _tcgen05_better_128(self, ctx, n_decode, window) -> bool:
+        """Whether portions with heads of 128 are worth the tcgen05 kernel rather than mma.sync.  Both
+        launch blocks for every portion as if it were the longest, and a block without tokens costs
+        tcgen05 some 3 ns more.  So: contexts of more than a tile, and either portions that are
+        much of what is launched, or few of them for the context's depth, in which it gains
+        (32 / 8 heads, us here / mma.sync: 500 and 15 of 20 tokens 27 / 30, 31 of 20 41 / 39; 1,000
+        and 31 of 20 76 / 83, 63 of 20 128 / 112; 70 and 31 of 10 14 / 11; 31 of 66 36 / 71)."""
+        reqs, tokens = ctx.n_reqs - n_decode, ctx.n_tokens - n_decode
+        depth = min(ctx.max_ctx_len, ctx.max_q_len + window) if window else ctx.max_ctx_len
+        return ctx.max_ctx_len > self._shallow_128 and reqs <= 8191 and ctx.max_q_len <= 65535 and (
+            reqs * ctx.max_q_len <= 4 * tokens or 16 * reqs <= depth)
 
     def paged_attention(self, qkv, num_heads, num_kv_heads, head_dim, k_cache, v_cache,
                         ctx, group, scale, window, out, sinks=None, v_head_dim=None):
@@ -642,10 +655,8 @@ class CudaOps:
                 self.paged_attention_decode(qkv, num_heads, num_kv_heads, head_dim, k_cache,
                                             v_cache, group.block_table, ctx.ctx_lens, nd,
                                             ctx.max_ctx_len, group.page_size, scale, window, out)
-        # (heads of 128 with one tile of keys at most stay with mma.sync: 4 tokens 4.6 against 5.9 us,
-        # 16 tokens 5.4 - 5.8 against 6.2; 64 tokens take 6.0 either way, 300 17 against 10)
         if (ctx.n_tokens > nd and self.prefill_attention in ("auto", "tcgen05") and vd == head_dim
-                and (head_dim == 64 or ctx.max_ctx_len > self._shallow_128)
+                and (head_dim == 64 or self._tcgen05_better_128(ctx, nd, window))
                 and self._tcgen05_prefill_ok(qkv, out, num_heads, num_kv_heads, head_dim,
                                              group.page_size)):
             self.paged_attention_prefill_tcgen05(qkv, num_heads, num_kv_heads, head_dim, k_cache,

@@ -140,3 +140,16 @@ def test_padded_steps_of_shallow_contexts():
     assert sizes_of([20, 30], (), shallow=64, context=35)[5] == 256
     assert sizes_of([20, 30], None, shallow=0)[5] == 256
     assert sizes_of([20, 30], (), shallow=64, page=2)[5] == 32
+
+
+@pytest.mark.parametrize("lens,context,window,better", [
+    ([300], 300, None, True), ([20, 30], 30, None, False), ([500] + [20] * 15, 500, None, True),
+    ([500] + [20] * 31, 500, None, False), ([1000] + [20] * 63, 1000, None, False), ([70] + [10] * 31, 70, None, False),
+    ([66] * 31, 66, None, True), ([4] * 31, 504, None, True), ([500] + [20] * 31, 800, None, True),
+    ([500] + [20] * 31, 800, 10, False), ([2] * 8192, 5000, None, False),
+    ([70000], 70000, None, False)])
+def test_prefill_kernel_for_heads_of_128(ops, lens, context, window, better):
+    """By how much of what is launched has tokens, and by the depth of the context; more portions,
+    or longer ones, than the tcgen05 kernel's grid has are left to the other kernel, which takes them."""
+    ctx = SimpleNamespace(n_reqs=len(lens) + 3, n_tokens=sum(lens) + 3, max_q_len=max(lens), max_ctx_len=context)
+    assert ops._tcgen05_better_128(ctx, 3, window) is better
