@@ -24,7 +24,7 @@
 // 256 columns, two blocks.
 // Head size 128 against the mma.sync kernel (us; pages of 16): latent rows, 16 heads: 2,048 tokens 93 ->
 // 42, 1,000 tokens 48 -> 23, 300 tokens 15 -> 11, 256 tokens after 3,840 162 -> 27, window 512 57 -> 21;
-// 32 heads: 2,048 tokens 173 -> 54; 32 / 8 heads with values of their own: 233 -> 66.  At head size 64
+// 32 heads: 2,048 tokens 173 -> 55; 32 / 8 heads with values of their own: 233 -> 58.  At head size 64
 // the exponent's offset follows the row maximum lazily (it moves only when the maximum has grown by
 // more than 2^8), so O is rescaled on few tiles.  Heads of 128 move it with the maximum and divide by
 // the sum of the rounded P, as the mma.sync kernel that they ran on before does: a row's largest P is
@@ -178,7 +178,7 @@ __device__ __forceinline__ unsigned long long at_desc(const void* tile) {
 // What the warps meet at: static memory, but for heads of 128 with values of their own.  Two of their
 // blocks would be 256 bytes more than a multiprocessor has, so there it lies in what the tiles'
 // alignment leaves of the dynamic memory (32 / 8 heads, 2,048 tokens: 89 us with one block a
-// multiprocessor, 66 with two; latent rows, which have two either way: 53 static, 62 so).
+// multiprocessor, 58 with two).
 #define AT_BARRIERS_DYNAMIC (RV_HD == 128 && !RV_SAME)
 struct AtShared {
     unsigned long long q_bar, s_bar, pv_bar, s_read, p_ready;
@@ -192,8 +192,11 @@ constexpr size_t at_tile_bytes() {
     return (size_t)(AT_ROWS * HD + AT_STAGES * AT_TILES * AT_KEYS * HD + AT_ROWS * AT_KEYS) * sizeof(bf16);
 }
 
+// (Heads of 128: bounds of 256 threads, for 128 registers.  A quarter of a multiprocessor may get two warps of
+// either block, 4 x 32 x 128 registers, which is all it has: with a few more 2,048 tokens of 32 latent
+// heads took 63 us instead of 55, and 32 / 8 heads with values of their own 68 instead of 58.)
 template <int HD>
-__global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill_tcgen05_kernel(
+__global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_attention_prefill_tcgen05_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table, int max_blocks,
     const int* __restrict__ q_start, const int* __restrict__ ctx_lens, bf16* __restrict__ out,
@@ -515,6 +518,20 @@ __global__ void __launch_bounds__(192, HD == 64 ? 3 : 2) paged_attention_prefill
                     at_tmem_st16(tmem_o + lane_base + (unsigned)c, v);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+            if (key0 + AT_KEYS > clen && (clen & (page_size - 1))) {
+                // The context ends within a page, which was copied whole: its later slots may hold
+                // another request's values, and P = 0 does not take away one that is not
+                // finite.  They are zeros from here on (all 128 rows' threads share the work).
+                bf16* vt = kv_ring + (size_t)(n % AT_STAGES) * AT_TILES * TILE + (SAME ? 0 : TILE);
+                if (!SAME && !at_mbar_wait(&v_full[n % AT_STAGES], (unsigned)(n / AT_STAGES) & 1u, &failed) && !failed) {
+                    failed = 1;
+                    atomicCAS(status, 0, 21);
+                }
+                const int first = clen - key0, count = (AT_KEYS - first) * 8;
+                for (int x = 0; x < HALVES; ++x)
+                    for (int i = tid; i < count; i += AT_ROWS)
+                        *(uint4*)(vt + x * HALF + first * 64 + i * 8) = make_uint4(0u, 0u, 0u, 0u);
             }
             {
                 // row m of the P tile: 128 bytes whose 16-byte chunks are XOR-swizzled with m & 7

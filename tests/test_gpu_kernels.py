@@ -768,6 +768,32 @@ def test_prefill_attention_head_size_128(ops, case, same):
     assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("hd,same", [(64, False), (128, False), (128, True)])
+@pytest.mark.parametrize("q_lens,ctx_lens,ps", [([70], [70], 16), ([33, 130], [433, 130], 64), ([20], [1994], 8),
+                                                ([300, 5, 66], [300, 90, 2000], 32)])
+def test_prefill_attention_slots_beyond_the_context(ops, hd, same, q_lens, ctx_lens, ps):
+    """The last page's slots beyond a request's context may hold what another request left there, a
+    NaN or an infinity: the outputs are the same as with zeros there, to the bit."""
+    g = torch.Generator().manual_seed(hd)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, q_lens, ctx_lens, 8, 2, hd, ps)
+    outs = []
+    for junk in (0.0, float("nan"), float("inf")):
+        k, v = kc.clone(), (None if same else vc.clone())
+        for r, c in enumerate(ctx_lens):
+            last = int(group.block_table[r, (c - 1) // ps])
+            for t in (k, v):
+                if t is not None:
+                    t.view(-1, ps, 2, hd)[last, (c - 1) % ps + 1:] = junk
+        dk = k.cuda()
+        dv = dk if same else v.cuda()
+        out = torch.empty(sum(q_lens), 8 * hd, dtype=torch.bfloat16, device="cuda")
+        ops.paged_attention(q.cuda(), 8, 2, hd, dk, dv, to_cuda(ctx), to_cuda(group), hd ** -0.5, None, out)
+        outs.append(out)
+    ops.check_status()
+    assert ("tcgen05", hd, same) in ops._attn_libs and bool(torch.isfinite(outs[0]).all())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 @pytest.mark.parametrize("same", [False, True])
 @pytest.mark.parametrize("lens", [[80], [33, 130]])
 def test_prefill_attention_head_size_128_rounds_alike(ops, lens, same):
