@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         }
     }
     __syncthreads();
-    gc_inverse<GH_THREADS>(As, Xs);
+    gc_inverse<GH_THREADS, true>(As, Xs);
     // q e^(B) and k e^(B): a thread has a lane's place in a fragment, rows j, j + 8 and channels c, c + 1,
     // c + 8, c + 9; k e^(B_L - B): channels c, c + 8 and tokens j, j + 1, j + 8, j + 9
     constexpr int SLOTS = 4 * UNITS * 32, OWN = (SLOTS + GH_THREADS - 1) / GH_THREADS;

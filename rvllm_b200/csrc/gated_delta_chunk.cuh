@@ -96,10 +96,27 @@ __device__ __forceinline__ void gc_inverse_pairs(float* As, float* Xs) {
 }
 
 // The inverse X of I + A, both [64][65] (of A what is below the diagonal is read, and overwritten).
-// Every thread of a block of NT calls it.
-template <int NT>
+// Every thread of a block of NT calls it.  A row of X depends on the rows of A up to its own; sums that take
+// zeros along must not bring it a later one that is not finite.  So with CHECK such rows of A, and all
+// behind the first of them, are left out and those of X are NaN.
+template <int NT, bool CHECK>
 __device__ __forceinline__ void gc_inverse(float* As, float* Xs) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ int first_bad;
+    if (CHECK) {
+        if (tid == 0) first_bad = 64;
+        __syncthreads();
+        for (int n = tid; n < 64 * 64; n += NT) {
+            const int i = n >> 6, j = n & 63;
+            if (j < i && !(fabsf(As[i * 65 + j]) <= 3.4028234e38f)) atomicMin(&first_bad, i);
+        }
+        __syncthreads();
+        if (first_bad < 64) {
+            for (int n = tid; n < 64 * 64; n += NT)
+                if ((n >> 6) >= first_bad) As[(n >> 6) * 65 + (n & 63)] = 0.f;
+            __syncthreads();
+        }
+    }
     // First its four diagonal blocks of 16, a warp each, two lanes a column:
     // x_i = (i = j) - sum_(j <= m < i) A_im x_m.
     if (warp < 4) {
@@ -125,6 +142,11 @@ __device__ __forceinline__ void gc_inverse(float* As, float* Xs) {
     // Then pairs of blocks of 16, and the pair of 32.
     gc_inverse_pairs<NT, 16>(As, Xs);
     gc_inverse_pairs<NT, 32>(As, Xs);
+    if (CHECK && first_bad < 64) {
+        for (int n = tid; n < 64 * 64; n += NT)
+            if ((n >> 6) >= first_bad && (n & 63) <= (n >> 6)) Xs[(n >> 6) * 65 + (n & 63)] = __int_as_float(0x7fc00000);
+        __syncthreads();
+    }
 }
 
 __global__ void __launch_bounds__(GC_THREADS) gdc_chunk_kernel(const GcArgs g) {
@@ -208,7 +230,7 @@ __global__ void __launch_bounds__(GC_THREADS) gdc_chunk_kernel(const GcArgs g) {
             }
     }
     __syncthreads();
-    gc_inverse<GC_THREADS>(As, Xs);
+    gc_inverse<GC_THREADS, true>(As, Xs);
     const size_t ih = (size_t)item * g.H + h;
     bf16* T = g.T + ih * 3 * 64 * 64;
     for (int n = tid; n < 64 * 32; n += GC_THREADS) {

@@ -429,6 +429,33 @@ def test_delta_rule_with_a_decay_per_head(ops, monkeypatch, dtype, sizes, strong
         assert float((state[4] - 3.0).abs().max()) == 0 and float(state[1].abs().max()) == 0
 
 
+@pytest.mark.parametrize("bad", [55, 64 + 20])
+def test_delta_rule_per_head_bad_key_and_earlier_tokens(ops, bad):
+    """A key that is not finite, in a portion in chunks: the tokens of the blocks of 16 before its own
+    come out as without it, to the bit, and every output of its heads from it on is NaN."""
+    H, G, d, dvv, n = 2, 1, 64, 64, 200
+    gen = torch.Generator().manual_seed(bad)
+    C = 2 * G * d + H * dvv
+    rows = rnd(gen, torch.float32, n, C + 2 * H + H * dvv).float()
+    args = [rnd(gen, torch.float32, C, 1), rnd(gen, torch.float32, H), rnd(gen, torch.float32, H),
+            1.0 + 0.1 * rnd(gen, torch.float32, dvv)]
+    ctx = SimpleNamespace(token_req=i32([0] * n), q_start=i32([0, n]), state_slot=i32([0]), n_reqs=1, n_decode=0,
+                          max_q_len=n)
+    outs = []
+    for junk in (False, True):
+        if junk:
+            rows[bad, G * d + 5] = float("nan")
+        proj = rows.cuda()
+        state = torch.zeros(1, ops.gated_delta_record(H, G, d, dvv, 1), device="cuda")
+        out = torch.empty(n, H * dvv, device="cuda", dtype=torch.bfloat16)
+        ops.gated_delta(proj, proj[:, C + H:], *[f32(a) for a in args], state, ctx, out, H, G, d, dvv, 1, 1e-6, 1e-5,
+                        head_decay=True, gate="silu")
+        outs.append(out)
+    before = bad // 16 * 16
+    assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0][:before], outs[1][:before])
+    assert bool(torch.isnan(outs[1][bad:]).all())
+
+
 def _ssm(gen, H, dvv, N, G, taps, ng, spread=1.0):
     m = dict(heads=H, vdim=dvv, state=N, groups=G, conv=taps, norm_groups=ng)
     C = H * dvv + 2 * G * N
