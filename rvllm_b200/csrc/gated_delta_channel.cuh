@@ -27,6 +27,10 @@
 //               out, the last state is the record
 //   gch_out     warp per (chunk, 16 tokens, head, 32 value columns): o
 //
+// A value that is not finite must not reach earlier tokens through a product with the zero that stands
+// for "later": gch_chunk takes such a value as 0 and notes its token.  From a bad key, value, decay or beta on
+// every output of the head is NaN, and so is its state; a bad query's own output is.
+//
 // Everything is float32: operands enter the bfloat16 products as three parts each (chunks.cuh), six of
 // the nine products.  What one kernel leaves for another's products lies in the order in which a
 // warp's fragments hold it, 16 bytes a lane, so that it goes from memory to registers as it is.
@@ -54,6 +58,7 @@ struct GhArgs {
     unsigned *K, *Q;                         // [3][d / 16][4][32][4], [3][4][d / 16][32][4]
     unsigned *S, *U;                         // [dv / 16][3][2][UP][32][4], [dv / 16][3][2][2][32][4]
     float *Pm, *V, *dec;                     // [64][64] (i >= j), [dv][64], [d]
+    int4 *bad;                               // the first token that is not finite (64: none), the queries that are not
 };
 
 __device__ __forceinline__ float gh_exp2(float x) {
@@ -62,6 +67,16 @@ __device__ __forceinline__ float gh_exp2(float x) {
     return y;
 }
 
+// Whether x can be taken into three parts; if not it is 0 from here on.
+__device__ __forceinline__ bool gh_clean(float& x) {
+    const bool ok = fabsf(x) <= 3.3895313e38f;            // the largest bfloat16
+    if (!ok) x = 0.f;
+    return ok;
+}
+__device__ __forceinline__ bool gh_clean(float4& v) {
+    const bool a = gh_clean(v.x), b = gh_clean(v.y), c = gh_clean(v.z), e = gh_clean(v.w);
+    return a && b && c && e;
+}
 // Four of them, on a 4-byte boundary.
 __device__ __forceinline__ void gh_lost(const bf16* p, float (&x)[4]) {
     const float2 a = lm_pair(*(const unsigned*)p), b = lm_pair(*(const unsigned*)(p + 2));
@@ -104,9 +119,14 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
     bf16* kt = (bf16*)ks;                                 // then [3][64][LD]: k e^(B)
     bf16* vt = kt + 3 * 64 * LD;                          // and [3][64][LV]: v
     __shared__ float beta[64];
-    __shared__ int at[2];
+    __shared__ int at[2], bad;                            // the first token with a value that is not finite
+    __shared__ unsigned bad_q[2];                         // the tokens whose query is not
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, dv = g.dv, LV = dv + 8;
     const int item = blockIdx.x, h = blockIdx.y, kh = h / (g.H / g.G);
+    if (tid == 0) {
+        bad = 64;
+        bad_q[0] = bad_q[1] = 0u;
+    }
     lm_locate(g.q_start, g.state_slot, g.first_req, g.n_reqs, item, at);
     const int t0 = at[0], L = at[1];
     rv_pdl_wait();
@@ -129,12 +149,22 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         for (int u = 0; u < EACH; ++u) {
             const int x = tid + u * GH_THREADS, j = x / (d / 4), c = (x - j * (d / 4)) * 4;
             if (x >= 64 * (d / 4)) continue;
+            if (!gh_clean(q[u])) atomicOr(&bad_q[j >> 5], 1u << (j & 31));
+            if (!gh_clean(k[u])) atomicMin(&bad, j);
+            // (a decay that is -inf forgets all, as it should)
+            if (l[u].x != l[u].x || l[u].y != l[u].y || l[u].z != l[u].z || l[u].w != l[u].w) {
+                l[u] = zero;
+                atomicMin(&bad, j);
+            }
             *(float4*)(qs + j * LD + c) = q[u];
             *(float4*)(ks + j * LD + c) = k[u];
             *(float4*)(bs + j * LD + c) = l[u];
         }
-        if (tid < 64)
-            beta[tid] = tid < L ? 1.f / (1.f + expf(-g.proj[(size_t)(t0 + tid) * g.P + g.C + h])) : 0.f;
+        if (tid < 64) {
+            float b = tid < L ? 1.f / (1.f + expf(-g.proj[(size_t)(t0 + tid) * g.P + g.C + h])) : 0.f;
+            if (!gh_clean(b)) atomicMin(&bad, tid);
+            beta[tid] = b;
+        }
     }
     __syncthreads();
     {   // unit norms: eight lanes a token
@@ -150,7 +180,10 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
             nq += __shfl_xor_sync(0xffffffffu, nq, o);
             nk += __shfl_xor_sync(0xffffffffu, nk, o);
         }
-        const float iq = 1.f / sqrtf((float)d) / sqrtf(nq + g.unit_eps), ik = 1.f / sqrtf(nk + g.unit_eps);
+        float iq = 1.f / sqrtf((float)d) / sqrtf(nq + g.unit_eps), ik = 1.f / sqrtf(nk + g.unit_eps);
+        // (a row of zeros without an epsilon: beyond the chunk's end it is no token)
+        if (!gh_clean(iq) && j < L && (tid & 7) == 0) atomicOr(&bad_q[j >> 5], 1u << (j & 31));
+        if (!gh_clean(ik) && j < L && (tid & 7) == 0) atomicMin(&bad, j);
         for (int c = (tid & 7) * 4; c < d; c += 32) {
             float4 q = *(const float4*)(qs + j * LD + c), k = *(const float4*)(ks + j * LD + c);
             q.x *= iq; q.y *= iq; q.z *= iq; q.w *= iq;
@@ -276,7 +309,7 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         }
     }
     __syncthreads();
-    gc_inverse<GH_THREADS, true>(As, Xs);
+    gc_inverse<GH_THREADS, false>(As, Xs);
     // q e^(B) and k e^(B): a thread has a lane's place in a fragment, rows j, j + 8 and channels c, c + 1,
     // c + 8, c + 9; k e^(B_L - B): channels c, c + 8 and tokens j, j + 1, j + 8, j + 9
     constexpr int SLOTS = 4 * UNITS * 32, OWN = (SLOTS + GH_THREADS - 1) / GH_THREADS;
@@ -335,8 +368,9 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
 #pragma unroll 4
         for (int x = tid; x < 64 * vq; x += GH_THREADS) {
             const int j = x / vq, c = (x - j * vq) * 4;
-            const float4 v = j < L ? *(const float4*)(base + (size_t)j * g.C + 2 * g.G * d + h * dv + c)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 v = j < L ? *(const float4*)(base + (size_t)j * g.C + 2 * g.G * d + h * dv + c)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!gh_clean(v)) atomicMin(&bad, j);
             uint2 p[3];
             lm_split(v.x, v.y, p[0].x, p[1].x, p[2].x);
             lm_split(v.z, v.w, p[0].y, p[1].y, p[2].y);
@@ -345,6 +379,7 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         }
     }
     __syncthreads();
+    if (tid == 0) g.bad[ih] = make_int4(bad, (int)bad_q[0], (int)bad_q[1], 0);
     // W and T V: a warp has 16 tokens and every fourth 16 columns, two of them at a time
     const int rg = warp & 3;
     unsigned a[4][3][4];
@@ -444,6 +479,7 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
             S[i][e] = mine ? Sg[(size_t)(ca + (e >> 1) * 8) * d + row + 8 * i + (e & 1)] : 0.f;
     uint4 w[3][UP], k[3][4];
     float2 v[2], keep[2];
+    int bad = LA_C;
     auto get_w = [&](size_t ih) {
         const unsigned* W = g.W + ih * 3 * 8 * UP * 128 + lane * 4;
 #pragma unroll
@@ -463,6 +499,7 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
             for (int kk = 0; kk < 4; ++kk) k[s][kk] = *(const uint4*)(K + ((s * UNITS + warp) * 4 + kk) * 128);
         keep[0] = *(const float2*)(g.dec + ih * d + row);
         keep[1] = *(const float2*)(g.dec + ih * d + row + 8);
+        bad = g.bad[ih].x;
     };
     const size_t step = g.H;
     size_t ih = (size_t)first_item * g.H + h;
@@ -537,7 +574,8 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    S[i][e] = fmaf(e & 1 ? keep[i].y : keep[i].x, S[i][e], (l[2][i][e] + l[1][i][e]) + l[0][i][e]);
+                    S[i][e] = bad < LA_C ? __int_as_float(0x7fc00000)
+                                         : fmaf(e & 1 ? keep[i].y : keep[i].x, S[i][e], (l[2][i][e] + l[1][i][e]) + l[0][i][e]);
         }
         if (c + 1 < n) get_k(ih + step);
     }
@@ -630,6 +668,19 @@ __global__ void __launch_bounds__(128) gch_out_kernel(const GhArgs g, float* __r
             product(a, b, e);
         }
     }
+    const int4 bad = g.bad[ih];
+    const unsigned bad_q = row_a & 32 ? (unsigned)bad.z : (unsigned)bad.y;
+    const float nan = __int_as_float(0x7fc00000);
+    if (row_a >= bad.x || (bad_q >> (row_a & 31) & 1u))
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) o[x][t][0] = o[x][t][1] = nan;
+    if (row_b >= bad.x || (bad_q >> (row_b & 31) & 1u))
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int t = 0; t < 2; ++t) o[x][t][2] = o[x][t][3] = nan;
     float* dst = o_out + ((size_t)t0 * g.H + h) * dv + 16 * cb0 + (lane & 3) * 2;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
@@ -652,7 +703,7 @@ static bool gh_sizes_ok(int H, int G, int d, int dv) {
     return d % 16 == 0 && d <= 128 && dv % 16 == 0 && (2 * G * d + H * dv) % 4 == 0 && gh_chunk_smem(d, dv) <= 220 * 1024;
 }
 struct GhScratch {
-    long long rows, logs, W, K, Q, S, U, Pm, V, dec, total;   // in floats, every part a multiple of four
+    long long rows, logs, W, K, Q, S, U, Pm, V, dec, bad, total;   // in floats, every part a multiple of four
 };
 static GhScratch gh_layout(int n_tokens, long long items, int H, int d, int dv, int C) {
     const long long ih = items * H, units = d / 16, up = (units + 1) / 2;
@@ -667,7 +718,8 @@ static GhScratch gh_layout(int n_tokens, long long items, int H, int d, int dv, 
     s.Pm = s.U + ih * (dv / 16) * 3 * 2 * 2 * 128;
     s.V = s.Pm + ih * 64 * 64;
     s.dec = s.V + ih * dv * 64;
-    s.total = s.dec + ih * d;
+    s.bad = s.dec + ih * d;
+    s.total = s.bad + ih * 4;
     return s;
 }
 
@@ -700,6 +752,7 @@ static int gh_run(GhArgs g, const float* filt, float* state, long long rec, int 
     g.Pm = scratch + lay.Pm;
     g.V = scratch + lay.V;
     g.dec = scratch + lay.dec;
+    g.bad = (int4*)(scratch + lay.bad);
     const long long count = (long long)(n_tokens - first_token) * g.H * g.d;
     rv_launch(gch_logs_kernel, dim3((unsigned)((count + 1023) / 1024)), dim3(256), 0, s, g, scratch + lay.logs, first_token, count);
     RV_CHECK_LAUNCH("gated_delta decays");

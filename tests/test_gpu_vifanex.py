@@ -408,6 +408,42 @@ def test_gated_delta_channel_chunks_behind_a_token_that_forgets(ops, d, log_deca
     assert errors[0] < errors[1] + 4 * 2.0 ** -24, errors
 
 
+@pytest.mark.parametrize("junk", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", ["query", "key", "value", "beta", "decay"])
+def test_gated_delta_channel_chunks_bad_values_and_earlier_tokens(ops, what, junk):
+    """A value that is not finite in the middle of a chunk: every token before it, and every head it is
+    no part of, comes out as without it, to the bit, state included.  A bad query costs its own
+    tokens (the convolution's taps), anything else the head's outputs from there on and its state.
+    (beta is a sigmoid and an infinite decay forgets: an infinity is a value like others there.)"""
+    if junk == float("inf") and what in ("beta", "decay"):
+        pytest.skip("finite after the gate")
+    H, G, d, dv, taps, T, at = 4, 2, 64, 48, 3, 400, 64 + 37
+    g = torch.Generator().manual_seed(len(what))
+    proj, low, filt, a_log, dt_bias, norm_w = delta_case(g, T, H, G, d, dv, taps)
+    C = 2 * G * d + H * dv
+    # (query and key head 1 serve heads 2 and 3)
+    column, heads = {"query": (d + 3, (2, 3)), "key": (G * d + d + 3, (2, 3)), "value": (2 * G * d + dv + 5, (1,)),
+                     "beta": (C + 3, (3,)), "decay": (2 * d + 7, (2,))}[what]
+    got = []
+    for bad in (False, True):
+        p, l = proj.clone(), low.clone()
+        if bad:
+            (l if what == "decay" else p)[at, column] = junk
+        ys, state = run_delta(ops, [(p, l)], (T,), H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, 1e-5,
+                              torch.bfloat16, [0])
+        got.append((ys[0].reshape(T, H, dv), state[0, (taps - 1) * C:].reshape(H, dv, d)))
+    (y0, s0), (y1, s1) = got
+    assert bool(torch.isfinite(y0).all()) and bool(torch.isfinite(s0).all())
+    behind = at + taps - 1 + 1 if what == "query" else T
+    for h in range(H):
+        if h not in heads:
+            assert torch.equal(y0[:, h], y1[:, h]) and torch.equal(s0[h], s1[h])
+            continue
+        assert torch.equal(y0[:at, h], y1[:at, h]) and torch.equal(y0[behind:, h], y1[behind:, h])
+        assert bool(torch.isnan(y1[at:behind, h]).all())
+        assert torch.equal(s0[h], s1[h]) if what == "query" else bool(torch.isnan(s1[h]).all())
+
+
 def test_gated_delta_order_within_a_token(ops):
     """Decay, then the correction with the decayed state, then the read-out of the written
     state: one head, two tokens, numbers worked by the plain step."""
