@@ -23,6 +23,10 @@
 // The rows are float32 and stay so: operands enter the bfloat16 products as three parts each
 // (chunks.cuh), six of the nine products, which reach a float32's last bits.
 //
+// A value that is not finite reaches no earlier token: mlc_out takes it as 0, and the head's outputs from its
+// token on are NaN, as are those of all later chunks by the memory.  (Weights of later tokens are 0 by choice, not
+// by a product, so keys and gates need no such care; a bad query is its own row.)
+//
 // The scan is a chain of some 64 instructions a token; here the only chain is mlc_scan's one
 // multiply-add a chunk, and mlc_out, the longest kernel (33 of 52 us for portions of 492 and 1,309
 // tokens), waits for its loads (30 % of a scheduler's cycles issue; its products keep the tensor pipe
@@ -100,8 +104,10 @@ __global__ void __launch_bounds__(1024) mlc_gates_kernel(const MlChunk g) {
             if (lane >= o) incl += up;
         }
         if (lane == 31) part[0][warp] = incl;
+        // (the sum before this pair, not the sum minus the pair: its second gate may be a NaN)
+        double before = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) before = 0.;
         __syncthreads();
-        double before = incl - F[1];
         for (int w = 0; w < warp; ++w) before += part[0][w];
         F[0] += before;
         F[1] += before;
@@ -140,6 +146,13 @@ __global__ void __launch_bounds__(1024) mlc_gates_kernel(const MlChunk g) {
     if (tid == 0) *m_rec = (float)m0;
 }
 
+// Whether all four can be taken into three parts; if not they are 0 from here on.
+__device__ __forceinline__ bool mlc_clean(float4& v) {
+    const bool ok = fabsf(v.x) <= 3.3895313e38f && fabsf(v.y) <= 3.3895313e38f && fabsf(v.z) <= 3.3895313e38f &&
+                    fabsf(v.w) <= 3.3895313e38f;              // the largest bfloat16
+    if (!ok) v = make_float4(0.f, 0.f, 0.f, 0.f);
+    return ok;
+}
 // Four neighbouring float32 values times f as three parts, to `dst`, `dst + step` and `dst + 2 step`.
 __device__ __forceinline__ void mlc_put4(bf16* dst, int step, float4 x, float f) {
     uint2 p[3];
@@ -285,9 +298,10 @@ __global__ void mlc_out_kernel(const MlChunk g) {
     bf16* vs = ss;
     __shared__ double at_[LA_C], ct[LA_C];
     __shared__ float f0[LA_C], em[LA_C], qn[LA_C], sq[4][LA_C], n0[16 * D16];
-    __shared__ int at[4];
+    __shared__ int at[4], bad;                   // bad: the first token with a value that is not finite
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rg = warp & 3, cg = warp >> 2;
     const int item = blockIdx.x, h = blockIdx.y;
+    if (tid == 0) bad = LA_C;
     mlc_locate(g, item, at);
     const int t0 = at[0], L = at[1];
     rv_pdl_wait();
@@ -394,7 +408,11 @@ __global__ void mlc_out_kernel(const MlChunk g) {
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                if (to[u] >= 0) mlc_put4(vs + to[u], LA_C * LV, in[u], 1.f);
+                if (to[u] >= 0) {
+                    // (an earlier token's weight of it is 0, and 0 times it must be 0)
+                    if (!mlc_clean(in[u])) atomicMin(&bad, to[u] / LV);
+                    mlc_put4(vs + to[u], LA_C * LV, in[u], 1.f);
+                }
         }
     }
     const int row_a = 16 * rg + (lane >> 2), row_b = row_a + 8;      // this thread's tokens
@@ -479,7 +497,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
             const int t = e ? row_b : row_a;
             if (t >= L) continue;
             const float2 gt = *(const float2*)(gate + (size_t)t * g.stride + c);
-            const float r = e ? rb : ra;
+            const float r = t >= bad ? __int_as_float(0x7fc00000) : e ? rb : ra;
             *(unsigned*)(out + ((size_t)(t0 + t) * g.H + h) * dv + c) =
                 pack_bf16(__fdividef(o[i][2 * e] * r * w0, 1.f + expf(-gt.x)),
                           __fdividef(o[i][2 * e + 1] * r * w1, 1.f + expf(-gt.y)));

@@ -365,6 +365,40 @@ def test_matrix_memory_chunks(ops, sizes, strong):
             assert abs(float(recd[H * (dv + 1) * d + h]) - mx) < 1e-5 * max(1.0, abs(mx))
 
 
+@pytest.mark.parametrize("junk", [float("nan"), float("inf")])
+@pytest.mark.parametrize("what", ["query", "key", "value", "gate"])
+def test_matrix_memory_chunks_bad_values_and_earlier_tokens(ops, what, junk):
+    """A value that is not finite in the middle of a chunk: every token before it and the other head
+    come out as without it, to the bit.  A bad query costs its own token, anything else the head's
+    outputs from there on.  (Input and forget gates are capped: an infinity is a value like others.)"""
+    if what == "gate" and junk == float("inf"):
+        pytest.skip("finite after the cap")
+    H, d, dv, n, at = 2, 64, 80, 230, 64 + 37
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn(n, 2 * H * d + 2 * H * dv + 2 * H, generator=g)
+    column = {"query": d + 3, "key": H * d + d + 3, "value": 2 * H * d + dv + 5, "gate": 2 * H * d + H * dv + 3}[what]
+    args = [torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda() + 3.0,
+            1.0 + 0.1 * torch.randn(H * dv, generator=g).cuda()]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(token_req=i32([0] * n), q_start=i32([0, n]), state_slot=i32([0]), n_reqs=1, n_decode=0)
+    outs, was = [], ops.mlstm_mode
+    try:
+        ops.mlstm_mode = "chunks"
+        for bad in (False, True):
+            if bad:
+                x[at, column] = junk
+            state = torch.zeros(1, ops.mlstm_record(H, d, dv), device="cuda")
+            out = torch.empty(n, H * dv, device="cuda", dtype=torch.bfloat16)
+            ops.mlstm(x.cuda(), *args, state, ctx, out, H, d, dv, 5.0, 1e-5)
+            outs.append(out.reshape(n, H, dv))
+    finally:
+        ops.mlstm_mode = was
+    assert bool(torch.isfinite(outs[0]).all()) and torch.equal(outs[0][:, 0], outs[1][:, 0])
+    behind = at + 1 if what == "query" else n
+    assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][behind:], outs[1][behind:])
+    assert bool(torch.isnan(outs[1][at:behind, 1]).all())
+
+
 def test_matrix_memory_alone_and_beside_a_long_portion(ops):
     """A request of 100 tokens goes token by token alone and in chunks beside one of 500: the same
     record within the float32 bound of the chunk form, the same output within bfloat16's."""
