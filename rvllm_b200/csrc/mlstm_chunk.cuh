@@ -18,7 +18,7 @@
 //   mlc_scan    over the chunks of a request one after another, elementwise: the memory before every
 //               chunk takes the place of the chunk's sum, the last one is the record
 //   mlc_out     block per (chunk, head): scores, both terms, the division, the head's norm, weight
-//               and gate
+//               and gate (divided, as in mlstm_finish, not multiplied by reciprocals)
 //
 // The rows are float32 and stay so: operands enter the bfloat16 products as three parts each
 // (chunks.cuh), six of the nine products, which reach a float32's last bits.
@@ -34,6 +34,10 @@
 // 4 x 512 tokens of 16 heads 191 -> 95, keys of 128 442 -> 93.
 #pragma once
 #include "chunks.cuh"
+
+// Threads of a block of mlc_state (two a value column) and mlc_out (128 for 64 columns) at most: values of
+// 256.  Stated as a bound, so that the registers of that many always fit.
+#define MLC_THREADS 512
 
 struct MlChunk {
     const float *rows, *bi, *bf, *norm_w;
@@ -163,7 +167,7 @@ __device__ __forceinline__ void mlc_put4(bf16* dst, int step, float4 x, float f)
 }
 // A warp has 16 columns of the values by all d rows.
 template <int D16>
-__global__ void mlc_state_kernel(const MlChunk g) {
+__global__ void __launch_bounds__(MLC_THREADS) mlc_state_kernel(const MlChunk g) {
     rv_pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int d = 16 * D16, LK = d + 8;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(128) mlc_scan_kernel(const MlChunk g) {
 // Four warps have 16 tokens each; as many groups of four as there are 64 columns.  The values take the
 // memory's place in shared memory once it has been read.
 template <int D16>
-__global__ void mlc_out_kernel(const MlChunk g) {
+__global__ void __launch_bounds__(MLC_THREADS) mlc_out_kernel(const MlChunk g) {
     rv_pdl_launch_dependents();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int d = 16 * D16, LK = d + 8;
@@ -459,14 +463,14 @@ __global__ void mlc_out_kernel(const MlChunk g) {
         den_a += __shfl_xor_sync(0xffffffffu, den_a, x);
         den_b += __shfl_xor_sync(0xffffffffu, den_b, x);
     }
-    const float by_a = q_scale / (fmaxf(fabsf(fmaf(fa, qn[row_a], den_a) * q_scale), em[row_a]) + 1e-6f);
-    const float by_b = q_scale / (fmaxf(fabsf(fmaf(fb, qn[row_b], den_b) * q_scale), em[row_b]) + 1e-6f);
+    den_a = fmaxf(fabsf(fmaf(fa, qn[row_a], den_a) * q_scale), em[row_a]) + 1e-6f;
+    den_b = fmaxf(fabsf(fmaf(fb, qn[row_b], den_b) * q_scale), em[row_b]) + 1e-6f;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            o[i][e] *= by_a;
-            o[i][2 + e] *= by_b;
+            o[i][e] = o[i][e] * q_scale / den_a;
+            o[i][2 + e] = o[i][2 + e] * q_scale / den_b;
             ss_a = fmaf(o[i][e], o[i][e], ss_a);
             ss_b = fmaf(o[i][2 + e], o[i][2 + e], ss_b);
         }
@@ -485,7 +489,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
         ss_a += sq[x][row_a];
         ss_b += sq[x][row_b];
     }
-    const float ra = 1.f / sqrtf(ss_a / (float)dv + g.eps), rb = 1.f / sqrtf(ss_b / (float)dv + g.eps);
+    const float ra = sqrtf(ss_a / (float)dv + g.eps), rb = sqrtf(ss_b / (float)dv + g.eps);
     const float* gate = base + 2 * g.H * d + g.H * dv + 2 * g.H + h * dv;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -499,8 +503,7 @@ __global__ void mlc_out_kernel(const MlChunk g) {
             const float2 gt = *(const float2*)(gate + (size_t)t * g.stride + c);
             const float r = t >= bad ? __int_as_float(0x7fc00000) : e ? rb : ra;
             *(unsigned*)(out + ((size_t)(t0 + t) * g.H + h) * dv + c) =
-                pack_bf16(__fdividef(o[i][2 * e] * r * w0, 1.f + expf(-gt.x)),
-                          __fdividef(o[i][2 * e + 1] * r * w1, 1.f + expf(-gt.y)));
+                pack_bf16(o[i][2 * e] / r * w0 / (1.f + expf(-gt.x)), o[i][2 * e + 1] / r * w1 / (1.f + expf(-gt.y)));
         }
     }
 }
@@ -513,7 +516,7 @@ static size_t mlc_out_smem(int d, int dv) {
 // Sizes that the chunk form takes: bfloat16 output; heads in multiples of 16, keys up to 128, values up
 // to 256, within shared memory; rows and heads on 16-byte boundaries.
 static bool mlc_ok(const float* rows, int stride, int out_dtype, int H, int d, int dv, const void* out) {
-    return out_dtype == RV_DTYPE_BF16 && d % 16 == 0 && d <= 128 && dv % 16 == 0 && dv <= 256 &&
+    return out_dtype == RV_DTYPE_BF16 && d % 16 == 0 && d <= 128 && dv % 16 == 0 && 2 * dv <= MLC_THREADS &&
            stride % 4 == 0 && ((uintptr_t)rows & 15) == 0 && ((uintptr_t)out & 3) == 0 &&
            mlc_out_smem(d, dv) <= 224 * 1024 && mlc_state_smem(d, dv) <= 224 * 1024;
 }

@@ -302,7 +302,7 @@ def test_matrix_memory_kernel(ops, dtype, sizes):
 
 @pytest.mark.parametrize("strong", [False, True])
 @pytest.mark.parametrize("sizes", [(1, 16, 16), (2, 64, 128), (3, 48, 80), (1, 128, 64), (1, 112, 144),
-                                   (1, 32, 256)])
+                                   (1, 32, 256), (1, 64, 256), (1, 80, 208)])
 def test_matrix_memory_chunks(ops, sizes, strong):
     """The chunk form against the definition in float64: portions of one token and around one, two
     and seventeen chunks of 64 (and of more tokens than a round of the gates' sums), a request whose
@@ -397,6 +397,32 @@ def test_matrix_memory_chunks_bad_values_and_earlier_tokens(ops, what, junk):
     behind = at + 1 if what == "query" else n
     assert torch.equal(outs[0][:at], outs[1][:at]) and torch.equal(outs[0][behind:], outs[1][behind:])
     assert bool(torch.isnan(outs[1][at:behind, 1]).all())
+
+
+def test_matrix_memory_chunks_nearly_closed_gates(ops):
+    """Output gates whose divisor is beyond 2^126 leave what a division leaves: the chunk form's
+    outputs are the scan's within bfloat16's roundings, none of them 0."""
+    H, d, dv, n = 1, 32, 64, 70
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(n, 2 * H * d + 2 * H * dv + 2 * H, generator=g)
+    x[:, -H * dv:] = -87.8
+    args = [torch.randn(H, generator=g).cuda(), torch.randn(H, generator=g).cuda() + 3.0,
+            torch.full((H * dv,), 1e4, device="cuda")]
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(token_req=i32([0] * n), q_start=i32([0, n]), state_slot=i32([0]), n_reqs=1, n_decode=0)
+    outs, was = [], ops.mlstm_mode
+    try:
+        for mode in ("chunks", "tokens"):
+            ops.mlstm_mode = mode
+            out = torch.empty(n, H * dv, device="cuda", dtype=torch.bfloat16)
+            ops.mlstm(x.cuda(), *args, torch.zeros(1, ops.mlstm_record(H, d, dv), device="cuda"), ctx, out, H, d, dv,
+                      5.0, 1e-5)
+            outs.append(out.double().cpu())
+    finally:
+        ops.mlstm_mode = was
+    big = outs[1].abs() > 1e-35                              # (bfloat16 has eight bits from 1.2e-38 on)
+    assert int(big.sum()) > n * dv // 2
+    assert float(((outs[0] - outs[1]).abs() / outs[1].abs().clamp(min=1e-35))[big].max()) < 2.0 ** -7
 
 
 def test_matrix_memory_alone_and_beside_a_long_portion(ops):
