@@ -152,11 +152,13 @@ static cudaError_t gf_launch(const float* x, const float* w, float* y, int M, in
     constexpr int BM = 8 * TMG, BN = 4 * TNG;
     const size_t smem = (size_t)GF_STAGES * (BM + BN) * GF_LD * sizeof(float);
     static_assert((size_t)GF_STAGES * (BM + BN) * GF_LD >= (size_t)BM * BN, "the tile fits the ring");
-    static bool raised = false;
-    if (!raised) {
+    // (the limit is a device's own: float32 products may be asked on another one than the first)
+    static bool raised[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !raised[dev]) {
         cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<TMG, TNG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        raised = true;
+        if (dev >= 0 && dev < 64) raised[dev] = true;
     }
     // K is split until there are three blocks a multiprocessor, 128 of K at least
     const int n_tiles = (N + BN - 1) / BN;
