@@ -343,8 +343,10 @@ def test_matrix_memory_chunks(ops, sizes, strong):
             ctx = SimpleNamespace(q_start=i32(starts), state_slot=i32(slots), token_req=i32(token_req),
                                   n_reqs=len(layout), n_decode=single)
             out = torch.full((x.shape[0], H * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+            before = ops.launches
             ops.mlstm(x, dev(torch.from_numpy(t["i.b"]).float()), dev(torch.from_numpy(t["f.b"]).float()),
                       dev(torch.from_numpy(t["norm"]).float()), state, ctx, out, H, d, dv, cap, eps)
+            assert ops.launches - before == (7 if single else 5)         # the chunk form's, and the scan's
             for ri, (r, n) in enumerate(layout):
                 if r:
                     got[r].append(out[starts[ri]:starts[ri + 1]].cpu())

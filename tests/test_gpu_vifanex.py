@@ -227,10 +227,11 @@ def plain_delta(proj, low, filt, a_log, dt_bias, norm_w, H, G, d, dv, eps):
     return y.reshape(T, H * dv), S
 
 
-def run_delta(ops, seqs, cuts, H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, eps, dtype, slots):
+def run_delta(ops, seqs, cuts, H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, eps, dtype, slots, forms=None):
     """The kernels on several requests at once, each cut into portions (cycled sizes, a
     request's next portion in every call until it is done), with a request that has no slot
-    and no tokens in every batch.  seqs: [(proj, low)] float64.  Returns (y per request, state)."""
+    and no tokens in every batch.  seqs: [(proj, low)] float64.  Returns (y per request, state).
+    `forms` receives, per call, the single tokens before the portions and whether these took chunks."""
     C = 2 * G * d + H * dv
     rec = ops.gated_delta_record(H, G, d, dv, taps)
     state = torch.full((max(slots) + 2, rec), float("nan"), device="cuda")
@@ -257,7 +258,13 @@ def run_delta(ops, seqs, cuts, H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, 
         q_start.append(q_start[-1])                            # the request without a slot
         ctx = SimpleNamespace(token_req=i32(token_req), q_start=i32(q_start),
                               state_slot=i32([slots[i] for i, _, _ in batch] + [-1]),
-                              n_reqs=len(batch) + 1)
+                              n_reqs=len(batch) + 1, n_decode=sum(n == 1 for _, _, n in batch),
+                              max_q_len=max(n for _, _, n in batch))
+        if forms is not None:
+            size = [ops.lib.rv_gated_delta_scratch(proj.shape[0], ctx.n_decode, ctx.n_reqs, H, G, d, dv, 0, c)
+                    for c in (0, 1)]
+            forms.append((ctx.n_decode, size[0] != size[1] and dtype == torch.bfloat16
+                          and ops.gated_delta_mode == "chunks" and ops._channel_chunks(ctx, proj.shape[0], H, d)))
         y = torch.full((proj.shape[0], H * dv), float("nan"), device="cuda", dtype=dtype)
         # wider rows than the kernel reads: what follows beta belongs to someone else
         wide = torch.cat([proj, torch.full((proj.shape[0], 3), float("nan"), dtype=proj.dtype)], dim=1)
@@ -350,9 +357,10 @@ def test_gated_delta_remembers_far_tokens(ops, sizes):
 @pytest.mark.parametrize("sizes", [(2, 1, 128, 128, 4), (4, 2, 16, 16, 3), (3, 1, 48, 80, 1), (2, 2, 112, 32, 2),
                                    (1, 1, 80, 144, 4)])
 def test_gated_delta_channel_chunks(ops, sizes, decays):
-    """The chunk form (bfloat16 output, portions of 256 tokens and more together) against the plain
-    rule in float64: requests that end at, one before and one after a chunk's and a block of 16's end,
-    one of a single token; decays that forget a channel within a few tokens (e^-20 a token, e^-1000
+    """The chunk form (bfloat16 output, a portion of more than 288 tokens) against the plain rule in
+    float64: requests that end at, one before and one after a chunk's and a block of 16's end, single
+    tokens before the portions, a record that a call in chunks leaves and the next one in chunks goes
+    on from; decays that forget a channel within a few tokens (e^-20 a token, e^-1000
     in a chunk) and decays of almost 1.  The records are float32 sums of operands in three exact
     parts: the bound of the token-by-token form."""
     H, G, d, dv, taps = sizes
@@ -363,16 +371,17 @@ def test_gated_delta_channel_chunks(ops, sizes, decays):
         a_log = a_log + 3.0
         dt_bias[::3] += 4.0
     seqs = []
-    for T in (321, 64, 127, 17, 1):
+    for T in (705, 64, 127, 17, 1):
         proj, low, *_ = delta_case(g, T, H, G, d, dv, taps)
         seqs.append((proj, low))
     want = [plain_delta(p.numpy(), l.numpy(), filt.numpy(), a_log.numpy(), dt_bias.numpy(),
                         norm_w.numpy(), H, G, d, dv, eps) for p, l in seqs]
     C = 2 * G * d + H * dv
-    for cuts in ((400,), (257, 48, 127, 16, 1)):
-        slots = [5, 2, 3, 0, 6]
+    for cuts, calls in (((400,), [(1, True), (0, True)]), ((300, 48, 127, 16, 1), [(1, True), (1, True), (0, False)])):
+        slots, forms = [5, 2, 3, 0, 6], []
         got, state = run_delta(ops, seqs, cuts, H, G, d, dv, taps, filt, a_log, dt_bias, norm_w, eps,
-                               torch.bfloat16, slots)
+                               torch.bfloat16, slots, forms)
+        assert forms == calls
         for i in range(len(seqs)):
             close(got[i], want[i][0], torch.bfloat16)
             S = state[slots[i], (taps - 1) * C:].reshape(H, dv, d).transpose(1, 2)
