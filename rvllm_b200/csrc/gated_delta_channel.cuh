@@ -16,7 +16,9 @@
 // every block of 16, forwards and backwards.  Only within a diagonal block an exponent is a difference of
 // two sums, which are large behind a token that forgets strongly; there a sum is a float32 and what its
 // additions lost (a bfloat16: some 2^-33 of it), so that the difference has its own float32 precision.  A
-// log decay below -192 counts as -192: either way the power, and every power across the token, is 0.
+// log decay below -192 counts as -192: either way the power, and every power across the token, is 0.  (One
+// token in sixteen with a log decay of -300: error of the state 1.2e-7, as token by token; with plain
+// differences 7.9e-6, and NaN behind a decay of -inf.)
 //
 //   gch_logs    log decays -> [n, H d]
 //   conv_silu   q | k | v pass the convolutions and silu -> rows [n, C] float32 (conv_silu.cuh)
@@ -702,6 +704,8 @@ static size_t gh_chunk_smem(int d, int dv) {
 static bool gh_sizes_ok(int H, int G, int d, int dv) {
     return d % 16 == 0 && d <= 128 && dv % 16 == 0 && (2 * G * d + H * dv) % 4 == 0 && gh_chunk_smem(d, dv) <= 220 * 1024;
 }
+// (Some 7.5 KB a token and head of 128 by 128, 3.6 times the form token by token: 490 MB for 8,192 tokens of 8 heads,
+// 980 MB of 16.)
 struct GhScratch {
     long long rows, logs, W, K, Q, S, U, Pm, V, dec, bad, total;   // in floats, every part a multiple of four
 };

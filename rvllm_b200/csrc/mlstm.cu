@@ -25,9 +25,10 @@
 //           multiply-adds into its rows and R into its part of the column's sum; the sums of
 //           sixteen tokens are added over the P lanes together -> num [N, H, dv + 1].  A
 //           column never meets another, so the columns of a head are spread over blocks, and a
-//           row's sums are formed token after token in the same order however a prompt was cut.
+//           row's sums are formed token after token in the same order however a prompt was cut
+//           (the chunk form's are not: it adds by chunks of 64 that begin where the portion does).
 //   finish  warp per (token, head): the division, the head's norm, weight and gate.
-// Portions of bfloat16 models whose sizes allow it take the chunk form on the tensor cores instead
+// Long portions of bfloat16 models whose sizes allow it take the chunk form on the tensor cores instead
 // (mlstm_chunk.cuh).
 // Plain reference: tests/plain_ops.py mlstm.
 #include "common.cuh"
@@ -412,7 +413,7 @@ extern "C" int rv_mlstm(const float* rows, int stride, const float* bi, const fl
         const int n = n_tokens - single;
         MlChunk g = {};
         g.rows = rows; g.bi = bi; g.bf = bf; g.norm_w = norm_w;
-        g.q_start = q_start; g.state_slot = state_slot; g.token_req = token_req;
+        g.q_start = q_start; g.state_slot = state_slot;
         g.state = state; g.rec = rec; g.out = out;
         g.stride = stride; g.first_req = single; g.n_reqs = n_reqs;
         g.H = H; g.d = d; g.dv = dv; g.cap = cap; g.eps = eps;

@@ -41,7 +41,7 @@
 
 struct MlChunk {
     const float *rows, *bi, *bf, *norm_w;
-    const int *q_start, *state_slot, *token_req;
+    const int *q_start, *state_slot;
     float* state;
     double *a, *c;               // [n, H]
     float *m, *em;               // [n, H]: the running maximum and e^-m

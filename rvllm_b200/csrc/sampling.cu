@@ -1,13 +1,14 @@
 // Sampling on the device: greedy argmax, and temperature with nucleus (top-p) filtering.
-// One block per row of float32 logits, so only token ids cross to the host.
+// Rows of float32 logits stay on the device, so only token ids cross to the host.
 //
 // argmax: the first maximum wins, NaN never wins, a row with nothing above -inf gives
 // 0 (the reference's argmax.cu:1-4 and src/sampler.rs:68-78).
 //
 // sample: a row with T <= 0 is greedy (as argmax).  Otherwise p_i = exp(l_i / T - max)
 // (src/sampler.rs:80-91); the nucleus is the set
-// {p_i >= tau} for the largest tau whose set has mass >= top_p * total, found by
-// bisection on the bit pattern of tau (positive floats order like their bits); tokens
+// {p_i >= tau} for the largest tau whose set has mass >= top_p * total, found by the bit
+// pattern of tau (positive floats order like their bits): rows up to 131,072 values by three
+// rounds of a histogram, a cluster of blocks a row, longer ones by bisection, a block a row; tokens
 // tied with the last kept one are kept (the reference keeps a sorted prefix,
 // src/sampler.rs:93-117).  The draw u in [0,1) is a counter-based hash of (seed,
 // counter), so a request's stream depends on nothing else in the batch; the token is the
@@ -365,10 +366,10 @@ __device__ __forceinline__ int rv_pick_bin(const unsigned* count, const unsigned
     return found;                                        // (a cluster barrier comes before the next round)
 }
 
-// MANY rows: four blocks a multiprocessor (64 registers), so that more rows are worked at once; few
+// MANY rows (up to 32 values a thread): four blocks a multiprocessor (64 registers), so that more rows are worked at once; few
 // rows have registers for all loads in flight (8 rows: 22 against 25 us; 64 rows: 51 against 40).
 template <int V, bool MANY>
-__global__ void __launch_bounds__(RV_SAMPLE_CT, MANY && V <= 32 ? 4 : 2) sample_cluster_kernel(
+__global__ void __launch_bounds__(RV_SAMPLE_CT, MANY ? 4 : 2) sample_cluster_kernel(
     const float* __restrict__ logits, const float* __restrict__ temperature,
     const float* __restrict__ top_p, const long long* __restrict__ seed,
     const long long* __restrict__ counter, int* __restrict__ out, int vocab, int rows) {
@@ -616,7 +617,9 @@ extern "C" int rv_sample(const float* logits, const float* temperature, const fl
         const cudaError_t e = each <= 16 ? RV_SAMPLE_CASE(16)
                               : each <= 24 ? RV_SAMPLE_CASE(24)
                               : each <= 32 ? RV_SAMPLE_CASE(32)
-                              : each <= 40 ? RV_SAMPLE_CASE(40) : RV_SAMPLE_CASE(64);
+                              : each <= 40
+                                  ? rv_sample_cluster<40, false>(logits, temperature, top_p, seed, counter, out, n_rows, vocab, blocks, s)
+                                  : rv_sample_cluster<64, false>(logits, temperature, top_p, seed, counter, out, n_rows, vocab, blocks, s);
 #undef RV_SAMPLE_CASE
         if (e != cudaSuccess) RV_FAIL("sample: %s", cudaGetErrorString(e));
     } else {
