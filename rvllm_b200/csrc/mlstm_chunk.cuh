@@ -18,7 +18,7 @@
 //   mlc_scan    over the chunks of a request one after another, elementwise: the memory before every
 //               chunk takes the place of the chunk's sum, the last one is the record
 //   mlc_out     block per (chunk, head): scores, both terms, the division, the head's norm, weight
-//               and gate (divided, as in mlstm_finish, not multiplied by reciprocals)
+//               and gate
 //
 // The rows are float32 and stay so: operands enter the bfloat16 products as three parts each
 // (chunks.cuh), six of the nine products, which reach a float32's last bits.
@@ -463,14 +463,17 @@ __global__ void __launch_bounds__(MLC_THREADS) mlc_out_kernel(const MlChunk g) {
         den_a += __shfl_xor_sync(0xffffffffu, den_a, x);
         den_b += __shfl_xor_sync(0xffffffffu, den_b, x);
     }
-    den_a = fmaxf(fabsf(fmaf(fa, qn[row_a], den_a) * q_scale), em[row_a]) + 1e-6f;
-    den_b = fmaxf(fabsf(fmaf(fb, qn[row_b], den_b) * q_scale), em[row_b]) + 1e-6f;
+    // (One division a row and products by it: a float32 rounding more than mlstm_finish's divisions, which
+    // the bfloat16 output's error against float64 does not show; dividing every value took mlc_out from 33
+    // to 37 us.  The gate is divided: its divisor goes beyond 2^126, where the fast division gives 0.)
+    const float by_a = q_scale / (fmaxf(fabsf(fmaf(fa, qn[row_a], den_a) * q_scale), em[row_a]) + 1e-6f);
+    const float by_b = q_scale / (fmaxf(fabsf(fmaf(fb, qn[row_b], den_b) * q_scale), em[row_b]) + 1e-6f);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            o[i][e] = o[i][e] * q_scale / den_a;
-            o[i][2 + e] = o[i][2 + e] * q_scale / den_b;
+            o[i][e] *= by_a;
+            o[i][2 + e] *= by_b;
             ss_a = fmaf(o[i][e], o[i][e], ss_a);
             ss_b = fmaf(o[i][2 + e], o[i][2 + e], ss_b);
         }
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(MLC_THREADS) mlc_out_kernel(const MlChunk g) {
         ss_a += sq[x][row_a];
         ss_b += sq[x][row_b];
     }
-    const float ra = sqrtf(ss_a / (float)dv + g.eps), rb = sqrtf(ss_b / (float)dv + g.eps);
+    const float ra = 1.f / sqrtf(ss_a / (float)dv + g.eps), rb = 1.f / sqrtf(ss_b / (float)dv + g.eps);
     const float* gate = base + 2 * g.H * d + g.H * dv + 2 * g.H + h * dv;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -503,7 +506,7 @@ __global__ void __launch_bounds__(MLC_THREADS) mlc_out_kernel(const MlChunk g) {
             const float2 gt = *(const float2*)(gate + (size_t)t * g.stride + c);
             const float r = t >= bad ? __int_as_float(0x7fc00000) : e ? rb : ra;
             *(unsigned*)(out + ((size_t)(t0 + t) * g.H + h) * dv + c) =
-                pack_bf16(o[i][2 * e] / r * w0 / (1.f + expf(-gt.x)), o[i][2 * e + 1] / r * w1 / (1.f + expf(-gt.y)));
+                pack_bf16(o[i][2 * e] * r * w0 / (1.f + expf(-gt.x)), o[i][2 * e + 1] * r * w1 / (1.f + expf(-gt.y)));
         }
     }
 }

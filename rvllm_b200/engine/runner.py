@@ -55,7 +55,9 @@ class ModelRunner:
         from ..parts.base import mixer_class
         limits, shallow = None, 0
         spec = self.model.spec
-        for call in spec.order if self.use_graphs else ():
+        # (all these kernels are for bfloat16: other models' steps pad to as few sizes as they can)
+        follow = self.use_graphs and self.model.dtype == torch.bfloat16
+        for call in spec.order if follow else ():
             m = spec.layers[call.layer].mixer
             rules = mixer_class(m.kind).launch_rules(m, self.ops)
             if rules[0] is not None:
