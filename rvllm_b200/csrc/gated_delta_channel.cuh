@@ -40,8 +40,8 @@
 // The scan by token is a chain of some 360 cycles a token; here it is two products and two barriers a
 // chunk (2.8 us, of which the products' issue is 0.8).  gch_chunk has one block of 512 threads a
 // multiprocessor (179 KB) and is a row of short phases, none of which fills the issue slots (36 %).
-// 8 heads of 128 by 128, one call: 2,048 tokens 440 -> 192 us, 559 + 1,489 tokens 370 -> 176,
-// 4 x 512 tokens of 16 heads 480 -> 308, keys of 64 305 -> 136, 512 tokens beside 31 single ones 261 -> 94.
+// 8 heads of 128 by 128, one call: 2,048 tokens 440 -> 201 us, 559 + 1,489 tokens 370 -> 183,
+// 4 x 512 tokens of 16 heads 480 -> 315, keys of 64 305 -> 140, 512 tokens beside 31 single ones 261 -> 96.
 #pragma once
 #include "gated_delta_chunk.cuh"
 

@@ -28,10 +28,10 @@
 // by a product, so keys and gates need no such care; a bad query is its own row.)
 //
 // The scan is a chain of some 64 instructions a token; here the only chain is mlc_scan's one
-// multiply-add a chunk, and mlc_out, the longest kernel (33 of 52 us for portions of 492 and 1,309
+// multiply-add a chunk, and mlc_out, the longest kernel (32 of 53 us for portions of 492 and 1,309
 // tokens), waits for its loads (30 % of a scheduler's cycles issue; its products keep the tensor pipe
-// 17 % busy).  8 heads of 64 by 128, one call: 2,048 tokens 283 -> 61 us, 492 + 1,309 tokens 182 -> 52,
-// 4 x 512 tokens of 16 heads 191 -> 95, keys of 128 442 -> 93.
+// 17 % busy).  8 heads of 64 by 128, one call: 2,048 tokens 283 -> 59 us, 492 + 1,309 tokens 182 -> 53,
+// 4 x 512 tokens of 16 heads 191 -> 98, keys of 128 442 -> 99.
 #pragma once
 #include "chunks.cuh"
 
