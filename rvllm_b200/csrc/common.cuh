@@ -53,6 +53,15 @@ __device__ __forceinline__ float rv_warp_max(float v) {
     return v;
 }
 
+// One lane of a warp whose lanes are all here.  What issues tcgen05 instructions is chosen so, by
+// a warp that comes there together: in a branch for `lane == 0` the compiler cannot keep their operands
+// in uniform registers and moves them one by one, some 80 cycles an instruction (25 this way).
+__device__ __forceinline__ bool rv_elect() {
+    unsigned one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
+
 // Sum over a block of up to 1024 threads; every thread gets the result.
 // `scratch` is shared memory for 33 floats.
 __device__ __forceinline__ float rv_block_sum(float v, float* scratch) {

@@ -20,6 +20,7 @@
 // one (131 rows 13824 x 1536 188 -> 209, 2,048 rows 1,377 -> 2,111), see rv_gemm_f32_better.
 // Operands in three bfloat16 parts on mma.sync were measured too: 131 rows 13824 x 1536 147 us, but
 // slower than the library below 96 rows and above 144, and than this at N = 1536.
+// From 768 of K on gemm_f32_split.cu is the faster one; this one is left with K of 512 to 764.
 // Its sums are nearer to float64 (relative error 2 - 4e-7 at these sizes, the library's 3e-7 - 1.5e-6).
 // Plain reference: tests/plain_ops.py linear.
 #include "common.cuh"

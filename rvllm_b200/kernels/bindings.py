@@ -51,6 +51,7 @@ class CudaOps:
         self.lib.rv_paged_attention_decode_scratch_bytes.restype = c_longlong
         self.lib.rv_gemm_tiled_bytes.restype = c_longlong
         self.lib.rv_gated_delta_scratch.restype = c_longlong
+        self.lib.rv_gemm_f32_split_scratch.restype = c_longlong
         self.lib.rv_mlstm_scratch.restype = c_longlong
         self.lib.rv_linear_attention_scratch.restype = c_longlong
         self.lib.rv_state_space_scratch.restype = c_longlong
@@ -303,7 +304,7 @@ class CudaOps:
                 self._gemm_status(device).zero_()
             raise KernelError(f"a kernel gave up waiting on an mbarrier (code {code}: 1-4 "
                               f"gemm_tcgen05, 12 decode attention, 21 prefill attention, 31-34 "
-                              f"grouped experts); its output is not valid")
+                              f"grouped experts, 41-45 float32 products); its output is not valid")
 
     def check_status(self) -> None:
         """Raise if a kernel recorded that one of its bounded waits ran out (this
@@ -354,16 +355,33 @@ class CudaOps:
         return qkv
 
     def _float32_product(self, x, w, out_dtype) -> bool:
-        """Whether x . w^T goes to this library's float32 kernel (few rows, or few columns).  What
-        the kernel cannot see from its pointers is looked at here: operands that do not fit one
-        another, that lie on another device or that want gradients are the library's."""
+        """Whether x . w^T may go to one of this library's float32 kernels.  What a kernel cannot
+        see from its pointers is looked at here: operands that do not fit one another, that lie on
+        another device or that want gradients are the library's."""
         return (x.dtype == torch.float32 and out_dtype == torch.float32 and self.gemm_mode != "cublas"
                 and x.dim() == 2 and w.dim() == 2 and x.shape[1] == w.shape[1]
                 and x.get_device() == w.get_device() == torch.cuda.current_device()
                 and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))
                 and x.is_contiguous() and w.is_contiguous()
-                and (x.data_ptr() | w.data_ptr()) % 16 == 0
-                and self.lib.rv_gemm_f32_better(x.shape[0], w.shape[0], x.shape[1]) != 0)
+                and (x.data_ptr() | w.data_ptr()) % 16 == 0)
+
+    @staticmethod
+    def _split_better(m: int, n: int, k: int) -> bool:
+        # It was the faster one at all sizes that were measured (K 512 to 8,192, 256 to 65,536 columns, 1 to
+        # 2,048 rows; 1.2 to 5 times the faster of the others) but for a few of up to 16 rows that were even.
+        # Which of the small ones stay where they were is pinned by tests of the other kernel.
+        return k % 4 == 0 and k >= 768 and n >= (256 if m <= 32 else 1024)
+
+    def _linear_split(self, x, w):
+        """y = x . w^T, float32, as sums of TF32 products (gemm_f32_split.cu)."""
+        (m, k), n = x.shape, w.shape[0]
+        y = torch.empty((m, n), dtype=torch.float32, device=x.device)
+        parts = torch.empty(self.lib.rv_gemm_f32_split_scratch(c_int(m), c_int(k)), dtype=torch.float32,
+                            device=x.device)
+        self._check(self.lib.rv_gemm_f32_split(
+            _ptr(x), _ptr(w), _ptr(y), _ptr(parts), _ptr(self._gemm_status(x.device)), c_int(m), c_int(n),
+            c_int(k), self._stream()), "gemm_f32_split")
+        return y
 
     def linear(self, x, w, bias=None, out_dtype=None):
         out_dtype = out_dtype or x.dtype
@@ -375,7 +393,10 @@ class CudaOps:
             return torch.empty((0, w.shape[0]), dtype=out_dtype, device=x.device)
         if self._small_product(x, w, out_dtype):
             y = self.linear_tcgen05(x, w, out_dtype)
-        elif self._float32_product(x, w, out_dtype):
+        elif self._float32_product(x, w, out_dtype) and self._split_better(x.shape[0], w.shape[0], x.shape[1]):
+            y = self._linear_split(x, w)
+        elif (self._float32_product(x, w, out_dtype)
+              and self.lib.rv_gemm_f32_better(x.shape[0], w.shape[0], x.shape[1])):
             y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
             self._check(self.lib.rv_gemm_f32(_ptr(x), _ptr(w), _ptr(y), c_int(x.shape[0]),
                                              c_int(w.shape[0]), c_int(x.shape[1]), self._stream()),

@@ -63,6 +63,42 @@ def test_float32_product_leaves_other_devices_and_gradients(ops):
     assert len(ops.calls) == 1
 
 
+@pytest.fixture
+def split_ops(ops):
+    ops.split = []
+    ops.lib.rv_gemm_f32_split_scratch = lambda m, k: 8
+    ops.lib.rv_gemm_f32_split = lambda *a: ops.split.append(a) or 0
+    ops._gemm_status = lambda device: torch.zeros(1, dtype=torch.int32)
+    return ops
+
+
+@pytest.mark.parametrize("m,n,k,taken", [
+    (1, 256, 768, True), (32, 256, 768, True), (33, 256, 768, False), (33, 1024, 768, True), (2048, 1024, 768, True),
+    (8, 255, 768, False), (8, 2048, 764, False), (8, 2048, 770, False)])
+def test_float32_product_of_parts_by_size(split_ops, m, n, k, taken):
+    split_ops.linear(on_device(m, k), on_device(n, k))
+    assert bool(split_ops.split) is taken and len(split_ops.split) + len(split_ops.calls) == 1
+
+
+def test_float32_product_of_parts_takes_what_fits(split_ops):
+    """Operands with other strides, of other types, at other addresses, on other devices or that want
+    gradients stay with the library; what it refuses stays refused."""
+    x, w = on_device(8, 1024), on_device(512, 1024)
+    for a, b in ((on_device(1024, 8).t(), w), (x, on_device(1024, 512).t()), (on_device(8, 2048)[:, ::2], w),
+                 (on_device(8 * 1024 + 1)[1:].view(8, 1024), w), (x, on_device(512, 1024, number=1)),
+                 (x, on_device(512, 1024, grad=True)), (x.double(), w.double())):
+        y = split_ops.linear(a, b)
+        assert not split_ops.split and not split_ops.calls
+        assert torch.allclose(torch.Tensor(y.detach().float()), torch.Tensor((a @ b.t()).detach().float()), atol=1e-3)
+    for a, b in ((x, on_device(512, 2048)), (on_device(2, 8, 1024), w), (x, on_device(2, 512, 1024))):
+        with pytest.raises((RuntimeError, ValueError)):
+            split_ops.linear(a, b)
+    assert not split_ops.split
+    split_ops.linear(x, w)
+    split_ops.linear(x, w.bfloat16())                       # cast, then multiplied
+    assert len(split_ops.split) == 2
+
+
 class Cuda(OnDevice):
     is_cuda = True
 

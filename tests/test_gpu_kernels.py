@@ -664,6 +664,57 @@ def test_gemm_f32(ops, M, N, K):
     assert float((y.double().cpu() - ref).norm() / ref.norm()) < 1e-6
 
 
+@pytest.mark.parametrize("M,N,K", [
+    # one chunk of K and a K that fills none, columns that fill no tile, every number of rows' tiles from
+    # one row to a full tile and one row more, K shared by one to eight blocks, two and three row tiles,
+    # rows that are split in portions
+    (1, 256, 768), (15, 300, 4), (17, 130, 100), (33, 257, 772), (49, 129, 3000), (65, 4608, 1536), (96, 128, 8192),
+    (113, 1000, 1028), (128, 13824, 768), (131, 1536, 6912), (160, 1030, 2048), (161, 1024, 800), (400, 2048, 2052),
+    (1000, 260, 16384)])
+def test_gemm_f32_split(ops, M, N, K):
+    """The float32 product from TF32 parts against float64.  A part's bits that are not read are below
+    2^-23 of an operand and the product that is left out below 2^-22 of the whole: 2^-21 a term.  A chunk's
+    twelve sums lose up to two units in the last place each (2^-23), the K / 32 chunks and eight blocks half
+    a unit each: (K / 32 + 64) 2^-24 of the sum of the terms' magnitudes, whatever the order."""
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g)
+    w = torch.randn(N, K, generator=g) * 0.05
+    x[M // 2, K // 3] = 40.0
+    w[N // 5, K // 3] = 3.0
+    x, w = x.cuda(), w.cuda()
+    before = ops.launches
+    y = ops._linear_split(x, w)
+    assert ops.launches == before + 1
+    if ops._split_better(M, N, K):
+        assert torch.equal(y, ops.linear(x, w))
+    ref = x.double() @ w.double().t()
+    ops.check_status()
+    bound = (K / 32 + 64) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert bool(((y.double() - ref).abs() <= bound).all())
+    assert float((y.double() - ref).norm() / ref.norm()) < 5e-7
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 300, 1028), (161, 1024, 800)])
+def test_gemm_f32_split_of_what_is_not_finite(ops, M, N, K):
+    """Infinite values, values that are none and values whose first part rounds up to infinity reach the
+    outputs that they belong to, as multiply-adds bring them there, and no others."""
+    g = torch.Generator().manual_seed(M)
+    x = torch.randn(M, K, generator=g)
+    w = torch.randn(N, K, generator=g) * 0.05
+    x[0, 7], x[1, 30], x[2, K - 1], x[3, 5] = float("inf"), float("nan"), 3.4028234e38, -float("inf")
+    w[4], w[5, 7], w[6, 3], w[7, 9] = 0.0, 0.0, float("inf"), float("nan")
+    w[:, K - 1] *= 1e-3
+    x, w = x.cuda(), w.cuda()
+    y = ops._linear_split(x, w)
+    ops.check_status()
+    ref = (x.double() @ w.double().t()).float()
+    assert torch.equal(torch.isnan(y), torch.isnan(ref))
+    assert torch.equal(torch.isinf(y) & (y > 0), torch.isinf(ref) & (ref > 0))
+    fin = torch.isfinite(ref)
+    bound = (K + 64) * 2.0 ** -24 * (x.nan_to_num(0, 0, 0).double().abs() @ w.nan_to_num(0, 0, 0).double().abs().t())
+    assert bool(((y.double() - ref.double()).abs() <= bound)[fin].all())
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 4608, 1536), (64, 1536, 6912)])
 def test_gemm_f32_of_a_matrix_made_just_before(ops, M, N, K):
     """The matrix may be what the launch before writes: a bfloat16 one is cast for float32 rows, and
