@@ -34,7 +34,7 @@
 //
 // Roles: warps 0-3 are the 128 rows; warp 4 brings Q (one 3-D TMA copy: [tokens, heads, 64])
 // and the key and value tiles (one 3-D TMA copy per page) into rings of two stages, keys and
-// values each as soon as their stage is free; thread 0 of warp 5 issues the MMAs -- S of the
+// values each as soon as their stage is free; warp 5 issues the MMAs -- S of the
 // next tile as soon as every row has read the current S out of TMEM.  Roles that wait do not
 // share a warp: a spinning lane starves the other lanes of its warp.  Only mbarriers
 // synchronise the roles inside the loop ("keys arrived", "values arrived", "S ready", "S
@@ -119,8 +119,8 @@ __device__ __forceinline__ void at_mma(unsigned tmem_d, unsigned long long a_des
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void at_tmem_ld16(unsigned taddr, float (&r)[16]) {
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem_base = tmem_base_smem;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
     const unsigned tmem_s = tmem_base, tmem_o = tmem_base + AT_KEYS;
 
     if (warp == 4) {
@@ -375,24 +375,28 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
             while (!ok && clock64() - t0 < AT_WAIT_CYCLES) ok = at_mbar_try_wait(&q_bar, 0);
         }
     } else if (warp == 5) {
-        // ---- MMA issuer (thread 0 of the sixth warp) ----------------------------------------
+        // ---- MMA issuer: the sixth warp walks the tiles together, one lane issues ------------
         // S = Q K^T of tile n + 1 is issued as soon as every row has read S of tile n out of
         // TMEM, so it runs while the rows do their softmax; O += P V of tile n when its P is
         // written.  instruction descriptors: D float32, A and B bfloat16; N >> 3 at bit 17,
         // M >> 4 at bit 24; bit 16: B is MN-major (V lies [key][dim]).
-        if (lane == 0) {
-            const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) |
-                                      ((unsigned)(AT_KEYS >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
-            const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                      ((unsigned)(64 >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
-            auto give_up = [&]() {
-                if (!failed) { failed = 1; atomicCAS(status, 0, 21); }
-            };
-            auto issue_qk = [&](int n) {
-                const int s = n % AT_STAGES;
-                if (!failed && !at_mbar_wait(&k_full[s], (unsigned)(n / AT_STAGES) & 1u, &failed)) give_up();
-                if (!failed) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) |
+                                  ((unsigned)(AT_KEYS >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
+        const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
+                                  ((unsigned)(64 >> 3) << 17) | ((unsigned)(AT_ROWS >> 4) << 24);
+        bool live = true;                                   // the same in every lane
+        auto wait = [&](unsigned long long* bar, unsigned parity) {
+            if (!live || __all_sync(0xffffffffu, at_mbar_wait(bar, parity, &failed))) return;
+            live = false;
+            if (lane == 0 && !failed) { failed = 1; atomicCAS(status, 0, 21); }
+            __syncwarp();
+        };
+        auto issue_qk = [&](int n) {
+            const int s = n % AT_STAGES;
+            wait(&k_full[s], (unsigned)(n / AT_STAGES) & 1u);
+            if (live) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (rv_elect()) {
+                if (live) {
                     const unsigned long long a0 = at_desc(q_tile);
                     const unsigned long long b0 = at_desc(kv_ring + (size_t)s * AT_TILES * TILE);
 #pragma unroll
@@ -400,21 +404,24 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
                         at_mma(tmem_s, a0 + (k >> 2) * (AT_ROWS * 128 >> 4) + 2 * (k & 3),
                                b0 + (k >> 2) * (HALF * 2 >> 4) + 2 * (k & 3), idesc_qk, k != 0);
                 }
-                if (!SAME) at_commit(&k_empty[s]);                  // the key stage is free again
+                if (!SAME) at_commit(&k_empty[s]);                // the key stage is free again
                 at_commit(&s_bar);
-            };
-            if (!at_mbar_wait(&q_bar, 0, &failed)) give_up();
-            issue_qk(0);
-            for (int n = 0; n < n_tiles; ++n) {
-                const int s = n % AT_STAGES;
-                if (n + 1 < n_tiles) {
-                    if (!failed && !at_mbar_wait(&s_read, (unsigned)n & 1u, &failed)) give_up();
-                    issue_qk(n + 1);
-                }
-                if (!failed && !at_mbar_wait(&p_ready, (unsigned)n & 1u, &failed)) give_up();
-                if (!SAME && !failed && !at_mbar_wait(&v_full[s], (unsigned)(n / AT_STAGES) & 1u, &failed)) give_up();
-                if (!failed) {
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            __syncwarp();
+        };
+        wait(&q_bar, 0);
+        issue_qk(0);
+        for (int n = 0; n < n_tiles; ++n) {
+            const int s = n % AT_STAGES;
+            if (n + 1 < n_tiles) {
+                wait(&s_read, (unsigned)n & 1u);
+                issue_qk(n + 1);
+            }
+            wait(&p_ready, (unsigned)n & 1u);
+            if (!SAME) wait(&v_full[s], (unsigned)(n / AT_STAGES) & 1u);
+            if (live) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (rv_elect()) {
+                if (live) {
                     const unsigned long long a0 = at_desc(p_tile);
                     const unsigned long long b0 = at_desc(kv_ring + (size_t)s * AT_TILES * TILE + (SAME ? 0 : TILE));
 #pragma unroll
@@ -426,9 +433,10 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
                                    b0 + (unsigned long long)(x * (HALF * 2 >> 4) + k * (16 * 128 >> 4)),
                                    idesc_pv, (n | k) != 0);
                 }
-                at_commit(SAME ? &k_empty[s] : &v_empty[s]);        // the value stage is free again
+                at_commit(SAME ? &k_empty[s] : &v_empty[s]);      // the value stage is free again
                 at_commit(&pv_bar);
             }
+            __syncwarp();
         }
     } else {
         // ---- rows: thread `tid` owns row tid = token * G + head ---------------------------

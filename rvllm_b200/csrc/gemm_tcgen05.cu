@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(128) gemm_tcgen05_kernel(
     // The next kernel of the stream may start its own preamble now.  This kernel's wait
     // for the previous one comes later: W does not depend on it, only x and y do.
     rv_pdl_launch_dependents();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tile = blockIdx.x, split = blockIdx.y, splits = gridDim.y;
     const int kb0 = (int)((long long)kblocks * split / splits);
     const int kb1 = (int)((long long)kblocks * (split + 1) / splits);
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(128) gemm_tcgen05_kernel(
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem_base = tmem_base_smem;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
 
     if (warp == 0 && lane == 0) {
         // ---- producer: TMA copies of W and x tiles ------------------------------------
@@ -190,35 +190,40 @@ __global__ void __launch_bounds__(128) gemm_tcgen05_kernel(
                 ok = mbar_try_wait(&full_bar[s], (i / stages) & 1);
             if (!ok && !failed) { failed = 1; atomicCAS(status, 0, 2); }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer -------------------------------------------------------------------
+    } else if (warp == 1) {
+        // ---- MMA issuer: the warp walks the stages together, one lane issues -------------------
         rv_pdl_wait();     // the bounded waits below start only when the previous kernel is done
         // instruction descriptor: D float32, A and B bfloat16, both K-major, N = n_pad, M = 128
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                ((unsigned)(n_pad >> 3) << 17) | ((unsigned)(RV_GEMM_BM >> 4) << 24);
         for (int i = 0; i < nst; ++i) {
             const int s = i % stages;
-            if (!mbar_wait(&full_bar[s], (i / stages) & 1, &failed)) {
-                if (!failed) { failed = 1; atomicCAS(status, 0, 3); }
+            if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], (i / stages) & 1, &failed))) {
+                if (lane == 0 && !failed) { failed = 1; atomicCAS(status, 0, 3); }
+                __syncwarp();
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int cnt = min(kbs, nkb - i * kbs);
+            if (rv_elect()) {
 #pragma unroll
-            for (int j = 0; j < kbs; ++j) {
-                if (j >= cnt) break;
-                const unsigned long long a0 = smem_desc_sw128(w_tiles + s * w_bytes + j * w_tile);
-                const unsigned long long b0 = smem_desc_sw128(x_tiles + s * x_bytes + j * x_tile);
+                for (int j = 0; j < kbs; ++j) {
+                    if (j >= cnt) break;
+                    const unsigned long long a0 = smem_desc_sw128(w_tiles + s * w_bytes + j * w_tile);
+                    const unsigned long long b0 = smem_desc_sw128(x_tiles + s * x_bytes + j * x_tile);
 #pragma unroll
-                for (int k = 0; k < RV_GEMM_BK / 16; ++k)      // 32 bytes per K = 16 step
-                    tcgen05_mma_f16(tmem_base, a0 + 2 * k, b0 + 2 * k, idesc, (i | j | k) != 0);
+                    for (int k = 0; k < RV_GEMM_BK / 16; ++k)      // 32 bytes per K = 16 step
+                        tcgen05_mma_f16(tmem_base, a0 + 2 * k, b0 + 2 * k, idesc, (i | j | k) != 0);
+                }
+                tcgen05_commit(&empty_bar[s]);              // frees the stage when the MMAs are done
             }
-            tcgen05_commit(&empty_bar[s]);                  // frees the stage when the MMAs are done
+            __syncwarp();
         }
-        tcgen05_commit(&accum_bar);                         // arrives when every MMA above is done
-        // this thread alone polls for the accumulator; the other 127 sleep at the block
-        // barrier below instead of competing with the two working threads for issue slots
-        if (!failed && !mbar_wait(&accum_bar, 0, &failed) && !failed) {
+        if (rv_elect()) tcgen05_commit(&accum_bar);         // arrives when every MMA above is done
+        __syncwarp();
+        // this warp alone polls for the accumulator; the others sleep at the block barrier
+        // below instead of competing with the working warps for issue slots
+        if (!__all_sync(0xffffffffu, mbar_wait(&accum_bar, 0, &failed)) && lane == 0 && !failed) {
             failed = 1;
             atomicCAS(status, 0, 4);
         }

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(128, 2) moe_grouped_kernel(
     rv_pdl_wait();                       // the list of tiles is written by an earlier kernel
     if ((int)blockIdx.y >= n_tiles[0]) return;
     const int expert = tile_expert[blockIdx.y], row0 = tile_row0[blockIdx.y];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tile = blockIdx.x;
     const int w_row = expert * n_out + tile * MT * MG_BM;
     unsigned tmem_cols = 32;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(128, 2) moe_grouped_kernel(
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem_base = tmem_base_smem;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
 
     if (warp == 0 && lane == 0) {
         // ---- producer ------------------------------------------------------------------------
@@ -223,29 +223,35 @@ __global__ void __launch_bounds__(128, 2) moe_grouped_kernel(
                 ok = mbar_try_wait(&full_bar[s], (i / stages) & 1);
             if (!ok && !failed) { failed = 1; atomicCAS(status, 0, 32); }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer: D float32, A and B bfloat16, both K-major, N = TN, M = 128 --------------
+    } else if (warp == 1) {
+        // ---- MMA issuer (the warp walks the stages together, one lane issues): D float32, A and B
+        // bfloat16, both K-major, N = TN, M = 128 ----------------------------------------------
         const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(TN >> 3) << 17) |
                                ((unsigned)(MG_BM >> 4) << 24);
         for (int i = 0; i < kblocks; ++i) {
             const int s = i % stages;
-            if (!mbar_wait(&full_bar[s], (i / stages) & 1, &failed)) {
-                if (!failed) { failed = 1; atomicCAS(status, 0, 33); }
+            if (!__all_sync(0xffffffffu, mbar_wait(&full_bar[s], (i / stages) & 1, &failed))) {
+                if (lane == 0 && !failed) { failed = 1; atomicCAS(status, 0, 33); }
+                __syncwarp();
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned long long b0 = smem_desc_sw128(x_tiles + s * x_tile);
-            for (int m = 0; m < MT; ++m) {
-                const unsigned long long a0 = smem_desc_sw128(w_tiles + s * w_tile + m * w_half);
+            if (rv_elect()) {
+                const unsigned long long b0 = smem_desc_sw128(x_tiles + s * x_tile);
+                for (int m = 0; m < MT; ++m) {
+                    const unsigned long long a0 = smem_desc_sw128(w_tiles + s * w_tile + m * w_half);
 #pragma unroll
-                for (int k = 0; k < MG_BK / 16; ++k)
-                    tcgen05_mma_f16(tmem_base + (unsigned)(m * TN), a0 + 2 * k, b0 + 2 * k, idesc,
-                                    (i | k) != 0);
+                    for (int k = 0; k < MG_BK / 16; ++k)
+                        tcgen05_mma_f16(tmem_base + (unsigned)(m * TN), a0 + 2 * k, b0 + 2 * k, idesc,
+                                        (i | k) != 0);
+                }
+                tcgen05_commit(&empty_bar[s]);
             }
-            tcgen05_commit(&empty_bar[s]);
+            __syncwarp();
         }
-        tcgen05_commit(&accum_bar);
-        if (!failed && !mbar_wait(&accum_bar, 0, &failed) && !failed) {
+        if (rv_elect()) tcgen05_commit(&accum_bar);
+        __syncwarp();
+        if (!__all_sync(0xffffffffu, mbar_wait(&accum_bar, 0, &failed)) && lane == 0 && !failed) {
             failed = 1;
             atomicCAS(status, 0, 34);
         }
