@@ -685,25 +685,41 @@ struct LaArgs {
 
 // The tensor-core forms exist for bfloat16 rows.
 template <int CH>
-static int la_tensor_launch(const float* rows, const LaArgs& a, int what, dim3 grid, float* kv, float* dec,
+static int la_tensor_launch(const float* rows, const LaArgs& a, int what, unsigned items, float* kv, float* dec,
                             float* num, cudaStream_t s) {
-    (void)rows; (void)a; (void)what; (void)grid; (void)kv; (void)dec; (void)num; (void)s;
+    (void)rows; (void)a; (void)what; (void)items; (void)kv; (void)dec; (void)num; (void)s;
     RV_FAIL("linear_attention: float32 rows on the tensor cores");
 }
 template <int CH>
-static int la_tensor_launch(const bf16* rows, const LaArgs& a, int what, dim3 grid, float* kv, float* dec,
+static int la_tensor_launch(const bf16* rows, const LaArgs& a, int what, unsigned items, float* kv, float* dec,
                             float* num, cudaStream_t s) {
-    if (what == 0) {
-        const size_t smem = lm_state_smem();
-        LA_SMEM(la_state_mma_kernel<CH>, smem)
-        rv_launch(la_state_mma_kernel<CH>, grid, dim3(128), smem, s, rows, a.stride, a.lr, a.tk, (const float*)a.z,
-                  a.log_decay, a.q_start, a.state_slot, a.n_decode, a.n_reqs, kv, dec, a.H, a.d, a.dv, a.act);
+    const int tiles_d = (a.d + LA_T - 1) / LA_T, tiles_v = (a.dv + LA_T - 1) / LA_T;
+    if constexpr (CH == LA_CHANNEL) {
+        if (what == 0) {
+            const size_t smem = lm_state_smem();
+            LA_SMEM(la_state_mma_kernel, smem)
+            rv_launch(la_state_mma_kernel, dim3(items, a.H, tiles_d * tiles_v), dim3(128), smem, s, rows, a.stride, a.lr,
+                      (const float*)a.z, a.q_start, a.state_slot, a.n_decode, a.n_reqs, kv, dec, a.H, a.d, a.dv, a.act);
+        } else {
+            const size_t smem = lm_out_smem(a.d);
+            LA_SMEM(la_out_mma_kernel, smem)
+            rv_launch(la_out_mma_kernel, dim3(items, a.H, tiles_v), dim3(128), smem, s, rows, a.stride, a.lr,
+                      (const float*)a.z, a.q_start, a.state_slot, a.n_decode, a.n_reqs, (const float*)kv, num, a.H, a.d,
+                      a.dv, a.act, a.q_scale);
+        }
+    } else if (what == 0) {
+        const size_t smem = lm_state_heads_smem();
+        const int tiles = (a.d + 127) / 128 * tiles_v, heads = lm_heads(a.lr.share, (long long)items * a.H * tiles);
+        LA_SMEM(la_state_heads_kernel<CH>, smem)
+        rv_launch(la_state_heads_kernel<CH>, dim3(items, a.H / heads, tiles), dim3(128), smem, s, rows, a.stride, a.lr,
+                  a.tk, a.log_decay, a.q_start, a.state_slot, a.n_decode, a.n_reqs, kv, a.H, a.d, a.dv, a.act, heads);
     } else {
-        const size_t smem = lm_out_smem(CH == LA_CHANNEL, a.d);
-        LA_SMEM(la_out_mma_kernel<CH>, smem)
-        rv_launch(la_out_mma_kernel<CH>, grid, dim3(128), smem, s, rows, a.stride, a.lr, a.tk, (const float*)a.z,
-                  a.log_decay, a.q_start, a.state_slot, a.n_decode, a.n_reqs, (const float*)kv, num, a.H, a.d, a.dv,
-                  a.act, a.q_scale);
+        const size_t smem = lm_out_heads_smem(a.d);
+        const int heads = lm_heads(a.lr.share, (long long)items * a.H * tiles_v);
+        LA_SMEM(la_out_heads_kernel<CH>, smem)
+        rv_launch(la_out_heads_kernel<CH>, dim3(items, a.H / heads, tiles_v), dim3(128), smem, s, rows, a.stride, a.lr,
+                  a.tk, a.log_decay, a.q_start, a.state_slot, a.n_decode, a.n_reqs, (const float*)kv, num, a.H, a.d,
+                  a.dv, a.act, a.q_scale, heads);
     }
     return 0;
 }
@@ -720,7 +736,7 @@ static int la_portions(const T* rows, const LaArgs& a, float* num, float* kv, fl
                       1.4426950408889634f / a.tau, a.q_start, a.state_slot, a.n_decode, a.n_reqs, width);
             RV_CHECK_LAUNCH("linear_attention_decay");
         }
-        if (la_tensor_launch<CH>(rows, a, 0, g1, kv, dec, num, s)) return 1;
+        if (la_tensor_launch<CH>(rows, a, 0, items, kv, dec, num, s)) return 1;
     } else {
         const size_t smem = (size_t)((CH == LA_CHANNEL ? 3 : 2) * LA_C * LA_LD + 4 * 64) * sizeof(float);
         auto kernel = la_state_kernel<T, CH>;
@@ -740,7 +756,7 @@ static int la_portions(const T* rows, const LaArgs& a, float* num, float* kv, fl
                   a.n_decode, kv, dec, a.state, a.H, a.d, a.dv);
     RV_CHECK_LAUNCH("linear_attention_scan");
     if (a.tensor) {
-        if (la_tensor_launch<CH>(rows, a, 1, g3, kv, dec, num, s)) return 1;
+        if (la_tensor_launch<CH>(rows, a, 1, items, kv, dec, num, s)) return 1;
     } else {
         const size_t smem = (size_t)((CH == LA_CHANNEL ? 6 : 3) * LA_DK * LA_LD + 2 * LA_C * LA_LD +
                                      (CH == LA_CHANNEL ? (LA_NG + 1 + LA_NG * LA_NG) * (LA_DK + 1) : 0)) * sizeof(float);
