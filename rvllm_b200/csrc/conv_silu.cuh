@@ -19,6 +19,12 @@ __device__ __forceinline__ void cs_load(const float* p, float (&x)[V]) {
     }
 }
 
+// A quotient that is rounded to bfloat16 need not be correct to the last bit of a float32.
+template <typename T>
+__device__ __forceinline__ float cs_silu(float x) {
+    return sizeof(T) == 4 ? x / (1.f + expf(-x)) : __fdividef(x, 1.f + __expf(-x));
+}
+
 // TAPS 0: any number, `taps`.
 template <typename T, int TAPS, int TT, int V>
 __global__ void __launch_bounds__(128) conv_silu_kernel(
@@ -92,9 +98,27 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(
 #pragma unroll
         for (int e = 0; e < V; ++e) {
             acc[e] += b[e];
-            acc[e] = acc[e] / (1.f + expf(-acc[e]));
+            acc[e] = cs_silu<T>(acc[e]);
         }
         la_store<T, V>(out + (size_t)t * C + c, acc);
+    }
+}
+
+// Channel c's inputs move on: its record of taps - 1 becomes the last of (old record | this step's `qlen` rows
+// from `in` on, P apart), oldest first.  What a place receives lies behind it, so eight are read
+// before any of their places is written.
+__device__ __forceinline__ void cs_move_on(float* record, const float* in, int P, int qlen, int C, int taps, int c) {
+    for (int i0 = 0; i0 < taps - 1; i0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int idx = qlen - (taps - 1) + i0 + u;  // among this step's rows; negative: older
+            if (i0 + u < taps - 1)
+                v[u] = idx >= 0 ? in[(size_t)idx * P + c] : record[(size_t)(taps - 1 + idx) * C + c];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + u < taps - 1) record[(size_t)(i0 + u) * C + c] = v[u];
     }
 }
 
