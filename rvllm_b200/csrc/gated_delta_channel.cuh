@@ -12,7 +12,8 @@
 // A channel may forget by e^-100 within a chunk, so e^(B_i) and e^(-B_j) are never formed apart.  A and P
 // are made in blocks of 16 by 16 tokens: below the diagonal blocks the decay from j to i passes the
 // first token of i's block, e^(from there to i) and e^(from j to there), neither above 1, go to the two
-// operands of a product; within a diagonal block every pair's own power is taken.  The sums start anew in
+// operands of a product; within a diagonal block the second eight tokens meet the first eight in the same way, and
+// every pair's own power is taken within those.  The sums start anew in
 // every block of 16, forwards and backwards.  Only within a diagonal block an exponent is a difference of
 // two sums, which are large behind a token that forgets strongly; there a sum is a float32 and what its
 // additions lost (a bfloat16: some 2^-33 of it), so that the difference has its own float32 precision.  A
@@ -39,7 +40,8 @@
 //
 // The scan by token is a chain of some 360 cycles a token; here it is two products and two barriers a
 // chunk (2.8 us, of which the products' issue is 0.8).  gch_chunk has one block of 512 threads a
-// multiprocessor (179 KB) and is a row of short phases, none of which fills the issue slots (36 %).
+// multiprocessor (179 KB) and is a row of short phases (thousand cycles: loads 4, norms and sums 4, A and P 14, the
+// inverse 7, what scan and out multiply with 7, W and T V 5); 264 such blocks take 57 us.
 // 8 heads of 128 by 128, one call: 2,048 tokens 440 -> 201 us, 559 + 1,489 tokens 370 -> 183,
 // 4 x 512 tokens of 16 heads 480 -> 315, keys of 64 305 -> 140, 512 tokens beside 31 single ones 261 -> 96.
 #pragma once
@@ -221,15 +223,16 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
     }
     __syncthreads();
     float* Pm = g.Pm + ih * 64 * 64;
-    if (warp < 9) {
-        // diagonal blocks: 36 tiles of two by two tokens each, two lanes a tile
-        const int unit = tid >> 1, J = unit / 36, ti = unit - 36 * J;
+    if (warp < 10) {
+        // blocks of eight on the diagonal: 10 tiles of two by two tokens each, four lanes a tile, whose
+        // loads meet few banks twice (two lanes a tile of blocks of sixteen: 23,000 cycles a chunk beside the products of the other blocks, 13,600 so)
+        const int unit = tid >> 2, J = unit / 10, ti = unit - 10 * J;
         int a = 0;
         while ((a + 1) * (a + 2) / 2 <= ti) ++a;
-        const int i0 = 16 * J + 2 * a, j0 = 16 * J + 2 * (ti - a * (a + 1) / 2);
+        const int i0 = 8 * J + 2 * a, j0 = 8 * J + 2 * (ti - a * (a + 1) / 2);
         float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, p[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 2
-        for (int c = (tid & 1) * 4; c < d; c += 8) {
+        for (int c = (tid & 3) * 4; c < d; c += 16) {
             float ki[2][4], qi[2][4], bi[2][4], kj[2][4], bj[2][4], li[2][4], lj[2][4];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -256,18 +259,54 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
         for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                s[i][j] += __shfl_xor_sync(0xffffffffu, s[i][j], 1);
-                p[i][j] += __shfl_xor_sync(0xffffffffu, p[i][j], 1);
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    s[i][j] += __shfl_xor_sync(0xffffffffu, s[i][j], o);
+                    p[i][j] += __shfl_xor_sync(0xffffffffu, p[i][j], o);
+                }
                 const int r = i0 + i, t = j0 + j;
-                if ((tid & 1) == 0) As[r * 65 + t] = t < r ? beta[r] * s[i][j] : 0.f;
-                else Pm[r * 64 + t] = t <= r ? p[i][j] : 0.f;       // (beyond the diagonal: no power of a sum)
+                if ((tid & 3) == 0) As[r * 65 + t] = t < r ? beta[r] * s[i][j] : 0.f;
+                if ((tid & 3) == 1) Pm[r * 64 + t] = t <= r ? p[i][j] : 0.f;        // (beyond the diagonal: no power of a sum)
             }
-    } else if (warp < 15) {
+        // the blocks of eight below those, a pair's a warp: tokens 8 .. 15 of sixteen against 0 .. 7, keys in
+        // the product's first eight rows and queries in the others, the decay by way of token 7
+        if (warp < 4) {
+            const int I = 16 * warp, r = I + 8 + (lane >> 2), j = I + (lane >> 2);
+            float y[3][4] = {};
+#pragma unroll 2
+            for (int kk = 0; kk < UNITS; ++kk) {
+                unsigned f[3][4], b[3][2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int c = 16 * kk + e * 8 + (lane & 3) * 2;
+                    const float2 m = *(const float2*)(bs + (I + 7) * LD + c), ml = lm_pair(*(const unsigned*)(ls + (I + 7) * (d + 2) + c)),
+                                 x = *(const float2*)(bs + r * LD + c), xl = lm_pair(*(const unsigned*)(ls + r * (d + 2) + c)),
+                                 z = *(const float2*)(bs + j * LD + c), zl = lm_pair(*(const unsigned*)(ls + j * (d + 2) + c)),
+                                 k = *(const float2*)(ks + r * LD + c), q = *(const float2*)(qs + r * LD + c),
+                                 kj = *(const float2*)(ks + j * LD + c);
+                    const float fx = gh_exp2((x.x - m.x) + (xl.x - ml.x)), fy = gh_exp2((x.y - m.y) + (xl.y - ml.y));
+                    lm_split(k.x * fx, k.y * fy, f[0][2 * e], f[1][2 * e], f[2][2 * e]);
+                    lm_split(q.x * fx, q.y * fy, f[0][2 * e + 1], f[1][2 * e + 1], f[2][2 * e + 1]);
+                    lm_split(kj.x * gh_exp2((m.x - z.x) + (ml.x - zl.x)), kj.y * gh_exp2((m.y - z.y) + (ml.y - zl.y)),
+                             b[0][e], b[1][e], b[2][e]);
+                }
+#pragma unroll
+                for (int z = 0; z < 3; ++z)
+#pragma unroll
+                    for (int x = 2; x >= z; --x) mma_bf16(y[x], f[z], b[x - z][0], b[x - z][1]);
+            }
+            const int t = I + (lane & 3) * 2;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) As[r * 65 + t + e] = beta[r] * ((y[2][e] + y[1][e]) + y[0][e]);
+            *(float2*)(Pm + r * 64 + t) = make_float2((y[2][2] + y[1][2]) + y[0][2], (y[2][3] + y[1][3]) + y[0][3]);
+        }
+    } else {
         // a block below the diagonal a warp: (1, 0), (2, 0), (2, 1), (3, 0), (3, 1), (3, 2)
-        const int w = warp - 9, I = w == 0 ? 1 : w < 3 ? 2 : 3, J = w - I * (I - 1) / 2;
+        const int w = warp - 10, I = w == 0 ? 1 : w < 3 ? 2 : 3, J = w - I * (I - 1) / 2;
         const int ra = 16 * I + (lane >> 2), ja = 16 * J + (lane >> 2);
+        const float over1 = J < 1 && I > 1, over2 = J < 2 && I > 2;     // whole blocks between the two
         float s[2][4] = {}, p[2][4] = {};
-#pragma unroll 1
+#pragma unroll 2
         for (int kk = 0; kk < UNITS; ++kk) {
             unsigned ak[3][4], aq[3][4], b[3][4];
 #pragma unroll
@@ -283,11 +322,8 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
             for (int e = 0; e < 4; ++e) {                 // tokens ja, ja + 8; a pair of channels, and eight on
                 const int j = ja + (e >> 1) * 8, c = 16 * kk + (e & 1) * 8 + (lane & 3) * 2;
                 float2 x = *(const float2*)(fs + j * LD + c);
-                for (int M = J + 1; M < I; ++M) {
-                    const float2 m = *(const float2*)(tot + M * d + c);
-                    x.x += m.x;
-                    x.y += m.y;
-                }
+                const float2 m1 = *(const float2*)(tot + d + c), m2 = *(const float2*)(tot + 2 * d + c);
+                x = make_float2(fmaf(over2, m2.x, fmaf(over1, m1.x, x.x)), fmaf(over2, m2.y, fmaf(over1, m1.y, x.y)));
                 const float2 k = *(const float2*)(ks + j * LD + c);
                 lm_split(k.x * gh_exp2(x.x), k.y * gh_exp2(x.y), b[0][e], b[1][e], b[2][e]);
             }
@@ -302,13 +338,12 @@ __global__ void __launch_bounds__(GH_THREADS) gch_chunk_kernel(const GhArgs g) {
                 As[r * 65 + t + 1] = beta[r] * s[i][2 * e + 1];
                 *(float2*)(Pm + r * 64 + t) = make_float2(p[i][2 * e], p[i][2 * e + 1]);
             }
-    } else {
-        for (int c = lane; c < d; c += 32) {
-            const float t[4] = {tot[c], tot[d + c], tot[2 * d + c], tot[3 * d + c]};
-            pre[c] = 0.f; pre[d + c] = t[0]; pre[2 * d + c] = t[0] + t[1]; pre[3 * d + c] = (t[0] + t[1]) + t[2];
-            post[3 * d + c] = 0.f; post[2 * d + c] = t[3]; post[d + c] = t[3] + t[2]; post[c] = (t[3] + t[2]) + t[1];
-            g.dec[ih * d + c] = gh_exp2(((t[0] + t[1]) + t[2]) + t[3]);
-        }
+    }
+    for (int c = GH_THREADS - 1 - tid; c < d; c += GH_THREADS) {
+        const float t[4] = {tot[c], tot[d + c], tot[2 * d + c], tot[3 * d + c]};
+        pre[c] = 0.f; pre[d + c] = t[0]; pre[2 * d + c] = t[0] + t[1]; pre[3 * d + c] = (t[0] + t[1]) + t[2];
+        post[3 * d + c] = 0.f; post[2 * d + c] = t[3]; post[d + c] = t[3] + t[2]; post[c] = (t[3] + t[2]) + t[1];
+        g.dec[ih * d + c] = gh_exp2(((t[0] + t[1]) + t[2]) + t[3]);
     }
     __syncthreads();
     gc_inverse<GH_THREADS, false>(As, Xs);
