@@ -39,7 +39,7 @@
 // warp's fragments hold it, 16 bytes a lane, so that it goes from memory to registers as it is.
 //
 // The scan by token is a chain of some 360 cycles a token; here it is two products and two barriers a
-// chunk (2.8 us, of which the products' issue is 0.8).  gch_chunk has one block of 512 threads a
+// chunk (2.4 us, of which the products' issue is 0.8).  gch_chunk has one block of 512 threads a
 // multiprocessor (179 KB) and is a row of short phases (thousand cycles: loads 4, norms and sums 4, A and P 14, the
 // inverse 7, what scan and out multiply with 7, W and T V 5); 264 such blocks take 57 us.
 // 8 heads of 128 by 128, one call: 2,048 tokens 440 -> 201 us, 559 + 1,489 tokens 370 -> 183,
@@ -543,9 +543,8 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
     get_w(ih);
     get_k(ih);
     for (int c = 0; c < n; ++c, ih += step) {
-        // the state before the chunk, for the products here and for gch_out
+        // the state before the chunk
         if (mine) {
-            unsigned* to = g.S + (ih * col_blocks + cb) * 3 * 2 * UP * 128 + (warp >> 1) * 128 + lane * 4 + (warp & 1) * 2;
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 unsigned x[3], y[3];
@@ -556,13 +555,13 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
                     bf16* p = ss + (s * GC_COLS + ca + 8 * e) * LK + row;
                     *(unsigned*)p = x[s];
                     *(unsigned*)(p + 8) = y[s];
-                    *(uint2*)(to + (s * 2 + e) * UP * 128) = make_uint2(x[s], y[s]);
                 }
             }
         }
         __syncthreads();
         // (W S)^T for this warp's eight tokens
         float y[3][4] = {};
+        uint4 left[3];
 #pragma unroll
         for (int kk = 0; kk < UNITS; ++kk) {
             unsigned a[3][4];
@@ -576,8 +575,27 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
                     const uint4 b = w[x - z][kk >> 1];
                     mma_bf16(y[x], a[z], kk & 1 ? b.z : b.x, kk & 1 ? b.w : b.y);
                 }
+            // for gch_out: its operand of columns 8 e.. and 32 rows of the state is half of what two such
+            // fragments hold, so a warp that has both leaves it, 16 bytes a lane
+            const int e = warp & 1;
+            if (warp >> 1 == kk >> 1 && kk >> 1 < UP) {
+                if (!(kk & 1)) {
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) left[s] = make_uint4(e ? a[s][1] : a[s][0], e ? a[s][3] : a[s][2], 0u, 0u);
+                } else {
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) {
+                        left[s].z = e ? a[s][1] : a[s][0];
+                        left[s].w = e ? a[s][3] : a[s][2];
+                    }
+                }
+            }
         }
-        unsigned* to = g.U + (ih * col_blocks + cb) * 3 * 2 * 2 * 128 + (warp >> 2) * 128 + lane * 4 + (warp & 3);
+        if (warp >> 1 < UP) {
+            unsigned* to = g.S + (ih * col_blocks + cb) * 3 * 2 * UP * 128 + ((warp & 1) * UP + (warp >> 1)) * 128 + lane * 4;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) *(uint4*)(to + s * 2 * UP * 128) = left[s];
+        }
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             unsigned x[3];
@@ -586,11 +604,20 @@ __global__ void __launch_bounds__(256) gch_scan_kernel(const GhArgs g, float* __
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
                 *(unsigned*)(us + (s * GC_COLS + ca + 8 * e) * GC_LT + tok) = x[s];
-                to[(s * 2 + e) * 2 * 128] = x[s];
             }
         }
         if (c + 1 < n) get_w(ih + step);
         __syncthreads();
+        if (warp < 4) {                                   // U in the same way, 32 tokens and 8 columns a warp
+            unsigned* to = g.U + (ih * col_blocks + cb) * 3 * 2 * 2 * 128 + ((warp & 1) * 2 + (warp >> 1)) * 128 + lane * 4;
+            const bf16* from = us + (8 * (warp & 1) + ca) * GC_LT + 32 * (warp >> 1) + (lane & 3) * 2;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const bf16* f = from + s * GC_COLS * GC_LT;
+                *(uint4*)(to + s * 2 * 2 * 128) = make_uint4(*(const unsigned*)f, *(const unsigned*)(f + 8),
+                                                             *(const unsigned*)(f + 16), *(const unsigned*)(f + 24));
+            }
+        }
         if (mine) {
             float l[3][2][4] = {};
 #pragma unroll
