@@ -19,6 +19,9 @@
 // values are the keys (a latent row): a tile is copied once and its stage is free when P V is
 // done, and the ring has three stages.
 //
+// Several blocks may share the key tiles of one block of query tokens (`nsplit`): a cluster of up to four,
+// whose unnormalised rows meet in distributed shared memory, or up to 16 through memory and a merge kernel.
+//
 // Head size 64: 65 KB of shared memory and 128 TMEM columns per block: three blocks share an SM,
 // so one block's softmax overlaps the others' copies and MMAs; 128: 113 KB (97 KB with RV_SAME) and
 // 256 columns, two blocks.
@@ -175,6 +178,47 @@ __device__ __forceinline__ unsigned long long at_desc(const void* tile) {
     return addr | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
+#define AT_THREADS 192
+#define AT_MAX_CLUSTER 4            // blocks that share a block's key tiles and meet in distributed shared memory
+__device__ __forceinline__ void at_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// What block `rank` of the cluster has where `local` is.
+__device__ __forceinline__ void at_cluster_load(const void* local, int rank, float2& v) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at_smem(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(remote) : "memory");
+}
+__device__ __forceinline__ void at_cluster_load(const void* local, int rank, float4& v) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at_smem(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+}
+// Four columns of a row from its parts (unnormalised, with offset and sum), in order.
+template <int HD, int PARTS>
+__device__ __forceinline__ void at_store_parts(const float2 (&ml)[PARTS], const float4 (&v)[PARTS], const float* sinks,
+                                               int head, bf16* dst) {
+    float M = -INFINITY;
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p)
+        if (ml[p].y > 0.f) M = fmaxf(M, ml[p].x);
+    float L = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p) {
+        if (ml[p].y > 0.f) {                                    // something visible in this part
+            const float w = at_exp2(ml[p].x - M);
+            L += ml[p].y * w;
+            o.x += v[p].x * w; o.y += v[p].y * w; o.z += v[p].z * w; o.w += v[p].w * w;
+        }
+    }
+    if (sinks && L > 0.f) L += at_exp2(sinks[head] * 1.4426950408889634f - M);   // once
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * inv, o.y * inv);
+    const __nv_bfloat162 hi = __floats2bfloat162_rn(o.z * inv, o.w * inv);
+    *(uint2*)dst = make_uint2(*(const unsigned*)&lo, *(const unsigned*)&hi);
+}
 // What the warps meet at: static memory, but for heads of 128 with values of their own.  Two of their
 // blocks would be 256 bytes more than a multiprocessor has, so there it lies in what the tiles'
 // alignment leaves of the dynamic memory (32 / 8 heads, 2,048 tokens: 89 us with one block a
@@ -203,6 +247,7 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
     int first_req, int num_heads, int num_kv_heads, int q_block, int page_size, float scale_log2,
     int window, int* __restrict__ status, int nsplit, float* __restrict__ part_o,
     float2* __restrict__ part_ml, const float* __restrict__ sinks) {
+    const bool clustered = nsplit > 1 && part_o == nullptr;
     static_assert(HD == 64 || HD == 128, "128-byte swizzle rows: 64 dimensions each");
     constexpr bool SAME = RV_SAME != 0;
     constexpr int HALVES = HD / 64;
@@ -230,8 +275,8 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
     const int t_all = key_lo / AT_KEYS, t_hi = p_last / AT_KEYS;
     const int per_part = (t_hi - t_all + nsplit) / nsplit;        // ceil(tiles / nsplit)
     const int t_lo = t_all + part * per_part;                      // this block's first tile
-    if (t_lo > t_hi) return;                                    // a part without tiles
-    const int n_tiles = min(t_hi, t_lo + per_part - 1) - t_lo + 1;
+    if (t_lo > t_hi && !clustered) return;                      // a part without tiles
+    const int n_tiles = max(0, min(t_hi, t_lo + per_part - 1) - t_lo + 1);
     const int page_shift = 31 - __clz(page_size);
     const int ppt = AT_KEYS >> page_shift;                      // pages per tile (1..16)
     const unsigned page_bytes = (unsigned)page_size * HD * 2u;
@@ -285,7 +330,12 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
     const unsigned tmem_base = __shfl_sync(0xffffffffu, tmem_base_smem, 0);
     const unsigned tmem_s = tmem_base, tmem_o = tmem_base + AT_KEYS;
 
-    if (warp == 4) {
+    // clustered: the parts' rows, [128][HD + 4] over the tiles, and their offsets and sums
+    float* rows_o = (float*)base;
+    float2* rows_ml = (float2*)(rows_o + AT_ROWS * (HD + 4));
+    if (n_tiles == 0) {                                         // (clustered: the others have tiles)
+        if (tid < AT_ROWS) rows_ml[tid] = make_float2(-INFINITY, 0.f);
+    } else if (warp == 4) {
         // ---- producer warp: Q once, then keys and values, each as soon as its stage is free.
         // A key stage is free when its S = Q K^T is done, a value stage when its P V is done,
         // so the keys run ahead of the values.  The warp polls both "stage free" barriers
@@ -557,7 +607,17 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
         if (__all_sync(0xffffffffu, done && !failed)) {         // one answer per warp: the reads
                                                                 // below are warp-wide
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (nsplit > 1) {
+            if (clustered) {
+                rows_ml[m] = make_float2(m_run, l_run);
+#pragma unroll
+                for (int c = 0; c < HD; c += 16) {
+                    float v[16];
+                    at_tmem_ld16(tmem_o + lane_base + (unsigned)c, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4)
+                        *(float4*)(rows_o + m * (HD + 4) + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
+            } else if (nsplit > 1) {
                 // this part's rows as they stand: O unnormalised, the offset and the sum
                 const size_t slot = (((size_t)r_local * gridDim.y + blockIdx.y) * gridDim.x + g) * nsplit + part;
                 float* po = part_o + (slot * AT_ROWS + m) * HD;
@@ -594,9 +654,12 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
                 }
             }
             }
-        } else if (!failed) {
-            failed = 1;
-            atomicCAS(status, 0, 21);
+        } else {
+            if (!failed) {
+                failed = 1;
+                atomicCAS(status, 0, 21);
+            }
+            if (clustered) rows_ml[m] = make_float2(-INFINITY, 0.f);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -605,6 +668,28 @@ __global__ void __launch_bounds__(HD == 64 ? 192 : 256, HD == 64 ? 3 : 2) paged_
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                      "r"(TMEM));
     }
+    if (!clustered) return;
+    // ---- the cluster's parts put together, in order: a block has every nsplit-th row -------------
+    at_cluster_sync();                                          // every part's rows are there
+    constexpr int CH = HD / 4;
+    for (int i = part * AT_THREADS + tid; i < n_tok * G * CH; i += nsplit * AT_THREADS) {
+        const int m = i / CH, c = (i - m * CH) * 4, tok = m / G, head = m - tok * G;
+        float2 ml[AT_MAX_CLUSTER];
+        float4 v[AT_MAX_CLUSTER];
+#pragma unroll
+        for (int p = 0; p < AT_MAX_CLUSTER; ++p) {
+            ml[p] = make_float2(-INFINITY, 0.f);
+            v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p < nsplit) {
+                at_cluster_load(rows_ml + m, p, ml[p]);
+                at_cluster_load(rows_o + m * (HD + 4) + c, p, v[p]);
+            }
+        }
+        at_store_parts<HD, AT_MAX_CLUSTER>(ml, v, sinks, g * G + head,
+                                           out + (size_t)(qs + q0 + tok) * num_heads * HD + (size_t)(g * G + head) * HD + c);
+    }
+    __syncwarp();
+    at_cluster_sync();                                          // nobody leaves while its rows are read
 }
 
 // The parts of a block of query tokens put together, in order.  A thread owns four columns of
@@ -648,26 +733,8 @@ __global__ void __launch_bounds__(16 * (HD / 4)) paged_attention_prefill_merge_k
         v[p] = there ? *(const float4*)(part_o + ((slot0 + p) * AT_ROWS + m) * HD + c)
                      : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    float M = -INFINITY;
-#pragma unroll
-    for (int p = 0; p < AT_MAX_PARTS; ++p)
-        if (ml[p].y > 0.f) M = fmaxf(M, ml[p].x);
-    float L = 0.f;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int p = 0; p < AT_MAX_PARTS; ++p) {
-        if (ml[p].y > 0.f) {                                    // something visible in this part
-            const float w = at_exp2(ml[p].x - M);
-            L += ml[p].y * w;
-            o.x += v[p].x * w; o.y += v[p].y * w; o.z += v[p].z * w; o.w += v[p].w * w;
-        }
-    }
-    if (sinks && L > 0.f) L += at_exp2(sinks[g * G + head] * 1.4426950408889634f - M);   // once
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-    bf16* dst = out + (size_t)(qs + q0 + tok) * num_heads * HD + (size_t)(g * G + head) * HD + c;
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x * inv, o.y * inv);
-    const __nv_bfloat162 hi = __floats2bfloat162_rn(o.z * inv, o.w * inv);
-    *(uint2*)dst = make_uint2(*(const unsigned*)&lo, *(const unsigned*)&hi);
+    at_store_parts<HD, AT_MAX_PARTS>(ml, v, sinks, g * G + head,
+                                     out + (size_t)(qs + q0 + tok) * num_heads * HD + (size_t)(g * G + head) * HD + c);
 }
 
 // ---- host side ----------------------------------------------------------------------------
@@ -749,6 +816,31 @@ static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window
     return parts < 1 ? 1 : parts;
 }
 
+// The same within a cluster: the parts meet in distributed shared memory, so they need no scratch and no
+// launch behind them, and whole prompts gain too.  `parts` is what sharing out through memory would take;
+// `blocks` are those with tokens, at the most.
+// Up to eight such parts become two to four blocks of a cluster, as many as fit the GPU at once: us through
+// memory / in a cluster, 32 / 8 heads of 64: 512 tokens after 700 25.6 / 20.0, 512 after 1,500 32.8 / 27.6, 256
+// after 2,000 24.2 / 20.3; 16 latent heads of 128: 512 after 1,500 36.6 / 22.9, 1,000 after 1,000 43.6 / 32.8; 32 / 8 heads
+// of 128: 256 after 2,000 39.9 / 26.2.  With more parts (64 tokens after 4,000: 14.5 / 23.7) or very few blocks (128 after 1,000
+// of 16 / 8 heads: 14.7 / 15.2) memory is the better way.
+// Prompts without earlier tokens are a triangle of blocks, the longest of which is the time where they do
+// not fill the GPU: us alone / in clusters of two, 16 / 8 heads of 64, 1,000 tokens 21.0 / 17.6, 2,048 37.8 / 30.6, 3,000 (376
+// blocks) 54.7 / 52.2, 4 x 512 (8 tiles deep) 16.3 / 21.6; 32 / 8 heads: 700 16.8 / 15.8, 1,000 (256 blocks) 22.5 / 25.4; 16 latent
+// heads, 1,000 tokens 24.4 / 21.6, 1,500 (188 blocks) 32.7 / 33.8.  Of four: 16 / 8 heads 512 tokens 13.3 / 11.5, 700 16.2 / 13.5,
+// 1,000 21.0 / 22.0.
+static int at_cluster(long long blocks, int parts, int tiles, int n_sms) {
+    const long long places = (RV_HD == 64 ? 3ll : 2ll) * n_sms;
+    if (parts > 1) {
+        int c = parts < AT_MAX_CLUSTER ? parts : AT_MAX_CLUSTER;
+        while (c > 2 && blocks * c > places) --c;
+        return parts > 8 || 2 * blocks * c < n_sms ? 1 : c;
+    }
+    if (tiles >= 8 && 5 * blocks <= places) return 4;
+    if (tiles >= 11 && 8 * blocks <= places * (tiles >= 20 ? 5 : 4)) return 2;
+    return 1;
+}
+
 static int at_configure(size_t smem) {
     static bool configured = false;
     if (configured) return 0;
@@ -802,16 +894,33 @@ extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
     if (at_configure(smem)) return 1;
     const int nqb = (max_q_len + q_block - 1) / q_block;
     const long long blocks = (long long)num_kv_heads * nqb * n_reqs;
-    const int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;
+    int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;
     if ((long long)n_reqs * (parts > AT_ROWS / 16 ? parts : AT_ROWS / 16) > 65535)
         return at_fail("paged_attention_prefill_tcgen05: too many requests");
     float* part_o = (float*)scratch;
     float2* part_ml = (float2*)((char*)scratch + (size_t)blocks * parts * AT_ROWS * RV_HD * 4);
-    rv_launch(paged_attention_prefill_tcgen05_kernel<RV_HD>, dim3(num_kv_heads, nqb, n_reqs * parts),
-              dim3(192), smem, (cudaStream_t)stream, map_q, map_k, map_v, block_table, max_blocks,
-              q_start, ctx_lens, (bf16*)out, first_req, num_heads, num_kv_heads, q_block, page_size,
-              scale * 1.4426950408889634f, window, status, parts, part_o, part_ml, sinks);
-    cudaError_t e = cudaGetLastError();
+    const long long real = (long long)num_kv_heads * (n_tokens / q_block + n_reqs);
+    int depth = (max_ctx_len + AT_KEYS - 1) / AT_KEYS;
+    if (window > 0 && window / AT_KEYS + 2 < depth) depth = window / AT_KEYS + 2;
+    const int cluster = n_sms > 0 ? at_cluster(blocks < real ? blocks : real, parts, depth, n_sms) : 1;
+    if (cluster > 1) parts = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(num_kv_heads, nqb, n_reqs * parts * cluster);
+    cfg.blockDim = dim3(AT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = rv_pdl_enabled();
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = cluster;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, paged_attention_prefill_tcgen05_kernel<RV_HD>, map_q, map_k, map_v, block_table,
+                                       max_blocks, q_start, ctx_lens, (bf16*)out, first_req, num_heads, num_kv_heads,
+                                       q_block, page_size, scale * 1.4426950408889634f, window, status, parts * cluster,
+                                       cluster > 1 ? (float*)nullptr : part_o, part_ml, sinks);
     if (e != cudaSuccess) return at_fail(cudaGetErrorString(e));
     if (parts > 1) {
         rv_launch(paged_attention_prefill_merge_kernel<RV_HD>,

@@ -880,6 +880,50 @@ def test_prefill_attention_blocks_a_multiprocessor(ops, head_dim, same, blocks):
         torch.cuda.get_device_properties(0).shared_memory_per_multiprocessor
 
 
+@pytest.mark.parametrize("hd,heads,kv,lens,ctxs,window", [
+    # whole prompts in clusters of four and of two, just over one part's tiles; parts that become clusters
+    # of two, three and four; a second request of which most blocks have no tokens; blocks of the
+    # cluster without tiles (fewer tiles than blocks); a window; latent rows
+    (64, 16, 8, [449], [449], None), (64, 16, 8, [700], [700], None), (64, 16, 8, [1000], [1000], None),
+    (64, 32, 8, [512], [1212], None), (64, 32, 8, [128], [1128], None), (64, 32, 8, [256], [2256], None),
+    (64, 16, 8, [300, 700], [300, 700], None), (64, 16, 8, [700, 3], [700, 700], None), (64, 16, 8, [1000], [1500], 700),
+    (128, 16, 1, [1000], [1000], None), (128, 16, 1, [512], [2012], None), (128, 32, 8, [256], [2256], None),
+    (128, 16, 1, [1000], [1500], 640)])
+def test_prefill_attention_in_clusters(ops, hd, heads, kv, lens, ctxs, window):
+    """Blocks that share a block's key tiles and meet in distributed shared memory, against float64.  P and
+    the outputs are rounded to bfloat16 (2^-9 of each at the most, of both signs): 2^-8 of the outputs' norm."""
+    g = torch.Generator().manual_seed(sum(lens) + hd)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, lens, ctxs, heads, kv, hd, 16)
+    same = kv == 1
+    if same:
+        vc = kc
+    N = sum(lens)
+    k, v = kc.cuda(), None
+    v = k if same else vc.cuda()
+    out = torch.empty(N, heads * hd, dtype=torch.bfloat16, device="cuda")
+    sinks = torch.randn(heads, generator=g).cuda() if window else None
+    ops.paged_attention(q.cuda(), heads, kv, hd, k, v, to_cuda(ctx), to_cuda(group), hd ** -0.5, window, out, sinks=sinks)
+    ops.check_status()
+    a = 0
+    for r, (n, c) in enumerate(zip(lens, ctxs)):
+        at = torch.arange(c)
+        page = group.block_table[r].cpu().long()[at // 16]
+        rows = lambda t: t.cpu()[page, at % 16].double().cuda()                          # noqa: E731
+        kk, vv = rows(kc), rows(vc)
+        qq = q[a:a + n, :heads * hd].view(n, heads, hd).double().cuda()
+        pos = torch.arange(c - n, c, device="cuda")[:, None]
+        key = torch.arange(c, device="cuda")[None]
+        hidden = (key > pos) | (key <= pos - window if window else key < 0)
+        for h in range(heads):
+            s = (qq[:, h] @ kk[:, h * kv // heads].T * hd ** -0.5).masked_fill(hidden, -float("inf"))
+            if sinks is not None:
+                s = torch.cat([s, sinks[h].double().expand(n, 1)], 1)
+            w = torch.softmax(s, -1)[:, :c] @ vv[:, h * kv // heads]
+            got = out[a:a + n, h * hd:(h + 1) * hd].double()
+            assert float((got - w).norm() / w.norm()) < 2.0 ** -8, (r, h)
+        a += n
+
+
 def test_prefill_attention_tcgen05_is_used(ops):
     """The default choice takes the tcgen05 kernel where it applies (its launch is counted by
     its own library) and refuses nothing it cannot do: other head sizes go to the mma kernel."""
