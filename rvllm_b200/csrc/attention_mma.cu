@@ -34,6 +34,7 @@
 #include "attention_pooled.cuh"
 #include "common.cuh"
 #include "mma_bf16.cuh"
+#include "stream_shares.cuh"
 
 #ifndef RV_HD
 #error "compile with -DRV_HD=<head size>"
@@ -602,19 +603,23 @@ __global__ void __launch_bounds__(NW * 32) paged_attention_decode_mma_kernel(
 #ifdef RV_STREAM
 // ---------------------------------------------------------------------------------
 // Decode as a stream (head size 64, pages of 8, 16, 32 or 64 tokens).  One persistent block
-// per SM; each of its six warps is a pipeline of its own.  A warp takes work items --
-// (request, key/value head, split of 128 or 256 keys) -- round robin, brings the item's key
-// and value tiles (64 keys) from the pages into its private ring of two stages with TMA (one
+// per SM; each of its six warps is a pipeline of its own, with an even share of the step's key tiles
+// (stream_shares.cuh; the heads of a page, which lie side by side in memory, are read at about the same
+// time).  A warp brings its run of tiles (64 keys) from the pages into its private ring of two stages with TMA (one
 // 3-D tensor copy per page, box [page_size tokens, one head, 64 dims], 128-byte swizzle,
-// completion counted on an mbarrier of the stage) and walks them with the online softmax.
-// The copy of the next tile -- of the next item, when this one ends -- is in flight while a
-// tile is computed, the block table entries and the context length of the item after the one
-// being loaded are fetched one item ahead, and its query rows arrive by cp.async; so the warp
-// never waits for a chain of dependent loads, and no warp waits for another.  Only tiles
-// that hold keys of the item are copied; a page past the context is zero-filled.  Every
+// completion counted on an mbarrier of the stage) and walks them with the online softmax; where
+// the run leaves a request, the rows so far go to memory as one of the request's segments, which
+// paged_attention_merge_segments_kernel (attention_simt.cu) puts together in order.
+// Splits of 128 or 256 keys, dealt out in turns, left some warps twice the others' work, and a replay's also
+// splits without keys.  Us with the merge, 32 / 8 heads, splits / runs: 8 requests of some 2,300 keys 14.2 / 13.0,
+// 31 of 950 20.7 / 17.9, 64 of 3,100 80.3 / 73.4 (5.6 TB/s), 8 of 240 7.3 / 5.3.
+// The copy of the next tile -- of the next segment, when this one ends -- is in flight while a
+// tile is computed, the block table entries are fetched one piece (up to 32 pages) ahead of
+// the one being loaded, and a segment's query rows arrive by cp.async; so the warp
+// never waits for a chain of dependent loads, and no warp waits for another.  A page past the
+// context is zero-filled.  Every
 // mbarrier wait is bounded (RV_STREAM_WAIT_CYCLES clock cycles); when one runs out the warp
 // records code 12 in `status`, waits (bounded) for its copies in flight and leaves.
-#define RV_STREAM_WARPS 6
 #define RV_STREAM_STAGES 2
 #define RV_STREAM_WAIT_CYCLES 400000000ll   // about 0.2 s: far beyond any real wait
 
@@ -661,7 +666,7 @@ __device__ __forceinline__ void st_tma_page(void* dst, const CUtensorMap* map, i
 
 // What the computing side needs to know of an item whose tiles are on their way.
 struct StreamMeta {
-    int r, g, m0, split, key_lo, key_hi, t_first, t_last;
+    int r, g, m0, place, key_lo, key_hi, t_first, t_last;
 };
 
 template <int HD>
@@ -670,8 +675,8 @@ paged_attention_decode_stream_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
     const bf16* __restrict__ q, int q_stride, const int* __restrict__ block_table, int max_blocks,
     const int* __restrict__ ctx_lens, float* __restrict__ part_o, float2* __restrict__ part_ml,
-    int max_splits, int item_tiles, int num_heads, int num_kv_heads, int page_size,
-    float scale_log2, int window, int n_reqs, int* __restrict__ status) {
+    int max_ctx, int teams, int num_heads, int num_kv_heads,
+    int page_size, float scale_log2, int window, int n_reqs, int* __restrict__ status) {
     rv_pdl_launch_dependents();     // the wait comes after the first look at the block table
     static_assert(HD == 64, "the stream kernel's stages are 128-byte rows");
     constexpr int LD = HD + 8;                                      // query rows stay padded
@@ -689,12 +694,10 @@ paged_attention_decode_stream_kernel(
     const int G = num_heads / num_kv_heads;
     const int tiles_per_head = (G + 15) / 16;
     const int heads_tiles = num_kv_heads * tiles_per_head;
-    const long long total = (long long)n_reqs * max_splits * heads_tiles;
-    const int nb = gridDim.x, b = blockIdx.x;
+    const int nw = gridDim.x * W;                                   // warps
     const int page_shift = 31 - __clz(page_size);                   // a power of two (host check)
     const int ppt = RV_BN >> page_shift;                            // pages per tile
-    const int ppi = ppt * item_tiles;                               // pages per item (<= 32)
-    const int item_keys = item_tiles * RV_BN;
+    const int piece_tiles = 32 / ppt;                               // tiles whose pages a warp's lanes hold
     const unsigned page_bytes = (unsigned)page_size * HD * 2u;
 
     if (lane == 0) {
@@ -708,72 +711,112 @@ paged_attention_decode_stream_kernel(
     const float ln2 = 0.6931471805599453f;
 
     // ---- the loading side -----------------------------------------------------------------
-    long long lk = 0;                 // this warp's next item is number (lk * W + w) * nb + b
-    int n_live = 0;                   // items with keys met so far (index into meta_q and my_q)
-    bool l_more = true;               // items left to look at
-    int l_t = 0, l_last = -1, l_t0 = 0, l_g = 0, l_page = -1;
-    int nx_clen = 0, nx_page = -1;    // context length and this lane's page of item lk, fetched ahead
-    // fetch the length and the block table entries of item `it` (no use of them yet)
-    auto fetch_ahead = [&](long long it) {
-        nx_clen = 0;
+    int n_live = 0;                   // segments met so far (index into meta_q and my_q)
+    int l_t = 0, l_last = -1, l_t0 = 0, l_g = 0, l_page = -1;   // the piece being loaded
+    // the cursor, one piece ahead
+    int c_unit = w * gridDim.x + blockIdx.x, c_run = 0, c_ht = 0;    // unit: (run, head)
+    int c_r = 0, c_t = 0, c_end = -1, c_left = 0;
+    bool c_new = false;
+    RvStreamShares sh(ctx_lens, n_reqs, window, max_ctx, teams);
+    const long long units = sh.total ? (long long)sh.used * heads_tiles : 0;
+    int nx_r = 0, nx_t = 0, nx_cnt = 0, nx_clen = 0, nx_page = -1;  // the cursor's piece, fetched ahead
+    bool nx_new = false;
+    int nx_ht = 0, nx_run = 0, nx_end = 0;
+    auto fetch_ahead = [&]() {
+        nx_cnt = 0;
+        if (c_left == 0) {                                          // the next unit's run
+            if (c_unit >= units) return;
+            c_run = c_unit / heads_tiles;
+            c_ht = c_unit - c_run * heads_tiles;
+            c_unit += nw;
+            const int from = sh.run_start(c_run);
+            int before = 0;                                         // tiles of the requests before
+            for (int at = 0;; at += 32) {
+                if (at >= n_reqs) return;                           // (there is such a request)
+                if (sh.grp != at) sh.load_group(at);
+                const int n = sh.tiles_of(sh.grp_len);
+                int upto = n;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, upto, d);
+                    if (lane >= d) upto += v;
+                }
+                const unsigned past = __ballot_sync(0xffffffffu, before + upto > from);
+                if (past) {
+                    const int j = __ffs(past) - 1;
+                    const int start = before + __shfl_sync(0xffffffffu, upto - n, j);
+                    const int clen = __shfl_sync(0xffffffffu, sh.grp_len, j);
+                    c_r = at + j;
+                    c_t = sh.first_tile(clen) + from - start;
+                    c_end = (clen - 1) / RV_BN;
+                    break;
+                }
+                before += __shfl_sync(0xffffffffu, upto, 31);
+            }
+            c_left = sh.run_start(c_run + 1) - from;
+            c_new = true;
+        } else if (c_t > c_end) {                                   // the run goes on in another request
+            int n = 0, clen = 0;
+            while (n == 0) {
+                if (++c_r >= n_reqs) {
+                    c_left = 0;
+                    return;
+                }
+                if (c_r >= sh.grp + 32) sh.load_group(sh.grp + 32);
+                clen = __shfl_sync(0xffffffffu, sh.grp_len, c_r - sh.grp);
+                n = sh.tiles_of(clen);
+            }
+            c_t = sh.first_tile(clen);
+            c_end = (clen - 1) / RV_BN;
+            c_new = true;
+        }
+        nx_clen = __shfl_sync(0xffffffffu, sh.grp_len, c_r - sh.grp);
+        nx_cnt = min(min(c_left, c_end - c_t + 1), piece_tiles);
+        nx_r = c_r; nx_t = c_t; nx_new = c_new; nx_ht = c_ht; nx_run = c_run;
+        nx_end = min(c_end, c_t + c_left - 1);                      // the segment's last tile
+        const int blk = c_t * ppt + lane;
         nx_page = -1;
-        if (it >= total) return;
-        const long long rest = it / heads_tiles;
-        const int split = (int)(rest % max_splits), r = (int)(rest / max_splits);
-        nx_clen = ctx_lens[r];
-        const int blk = ((split * item_keys) >> page_shift) + lane;
-        if (lane < ppi && blk < max_blocks) nx_page = block_table[(size_t)r * max_blocks + blk];
+        if (lane < nx_cnt * ppt && blk < max_blocks && (blk << page_shift) < nx_clen)
+            nx_page = block_table[(size_t)c_r * max_blocks + blk];
+        c_t += nx_cnt;
+        c_left -= nx_cnt;
+        c_new = false;
     };
-    fetch_ahead((lk * W + w) * nb + b);   // index arrays of the step: not the previous kernel's
+    fetch_ahead();                         // index arrays of the step: not the previous kernel's
     rv_pdl_wait();                         // keys, values and queries are the previous kernels'
     int n_loaded = 0, n_consumed = 0;
 
-    // move to the next item that has keys; false when there is none
-    auto next_load_item = [&]() -> bool {
-        while (l_more) {
-            const long long it = (lk * W + w) * nb + b;
-            if (it >= total) {
-                l_more = false;
-                break;
-            }
-            const int clen = nx_clen, page = nx_page;
-            ++lk;
-            fetch_ahead((lk * W + w) * nb + b);
-            const int ht = (int)(it % heads_tiles);
-            const long long rest = it / heads_tiles;
-            const int split = (int)(rest % max_splits), r = (int)(rest / max_splits);
-            if (clen == 0) continue;
-            const int p = clen - 1;
-            const int key_lo = max(window > 0 ? max(0, p - window + 1) : 0, split * item_keys);
-            const int key_hi = min(p, split * item_keys + item_keys - 1);
-            if (key_lo > key_hi) continue;
-            const int g = ht / tiles_per_head, m0 = (ht % tiles_per_head) * 16;
-            l_g = g;
-            l_t0 = split * item_tiles;
-            l_t = key_lo / RV_BN;
-            l_last = key_hi / RV_BN;
-            l_page = (lane < ppi && ((split * item_keys + (lane << page_shift)) < clen)) ? page : -1;
+    // move to the next piece; false when there is none
+    auto next_piece = [&]() -> bool {
+        if (nx_cnt == 0) return false;
+        l_t0 = l_t = nx_t;
+        l_last = nx_t + nx_cnt - 1;
+        l_page = nx_page;
+        l_g = nx_ht / tiles_per_head;
+        if (nx_new) {
+            const int m0 = (nx_ht - l_g * tiles_per_head) * 16;
             if (lane == 0) {
                 StreamMeta& m = meta_q[w][n_live & 3];
-                m.r = r; m.g = g; m.m0 = m0; m.split = split;
-                m.key_lo = key_lo; m.key_hi = key_hi; m.t_first = l_t; m.t_last = l_last;
+                m.r = nx_r; m.g = l_g; m.m0 = m0; m.place = nx_run + nx_r;
+                m.key_lo = window > 0 ? max(0, nx_clen - window) : 0;
+                m.key_hi = nx_clen - 1; m.t_first = nx_t; m.t_last = nx_end;
             }
-            // its query rows, by cp.async into the slot of this item's parity
+            // its query rows, by cp.async into the slot of this segment's parity
             bf16* Qs = my_q + (size_t)(n_live & 1) * 16 * LD;
             const int rows = min(16, G - m0);
             for (int i = lane; i < 16 * (HD / 8); i += 32) {
                 const int m = i / (HD / 8), ch = i - m * (HD / 8);
                 const bool valid = m < rows;
-                const bf16* src = q + (size_t)r * q_stride +
-                                  (size_t)(g * G + m0 + (valid ? m : 0)) * HD + ch * 8;
+                const bf16* src = q + (size_t)nx_r * q_stride +
+                                  (size_t)(l_g * G + m0 + (valid ? m : 0)) * HD + ch * 8;
                 cp_async_16(Qs + m * LD + ch * 8, src, valid);
             }
             cp_async_commit();
             ++n_live;
-            __syncwarp();
-            return true;
         }
-        return false;
+        fetch_ahead();
+        __syncwarp();
+        return true;
     };
     // copy the load cursor's tile into the next stage; the stage is free (the caller knows)
     auto issue_tile = [&]() {
@@ -812,14 +855,14 @@ paged_attention_decode_stream_kernel(
     };
     auto fill = [&]() {
         while (n_loaded - n_consumed < S) {
-            if (l_t > l_last && !next_load_item()) break;
+            if (l_t > l_last && !next_piece()) break;
             issue_tile();
         }
     };
 
     // ---- the computing side -----------------------------------------------------------------
     fill();
-    int n_done = 0;                   // items finished (index into meta_q and my_q)
+    int n_done = 0;                   // segments finished (index into meta_q and my_q)
     bool failed = false;
     while (n_consumed < n_loaded && !failed) {
         __syncwarp();
@@ -862,14 +905,14 @@ paged_attention_decode_stream_kernel(
         l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
         const int col = (lane & 3) * 2;
         if (ok_a) {
-            const size_t slot = ((size_t)m.r * num_heads + m.g * G + row_a) * max_splits + m.split;
+            const size_t slot = (size_t)(m.g * G + row_a) * (teams + n_reqs) + m.place;
 #pragma unroll
             for (int i = 0; i < HD / 8; ++i)
                 *(float2*)(part_o + slot * HD + i * 8 + col) = make_float2(o[i][0], o[i][1]);
             if ((lane & 3) == 0) part_ml[slot] = make_float2(m_a * ln2, l_a);
         }
         if (ok_b) {
-            const size_t slot = ((size_t)m.r * num_heads + m.g * G + row_b) * max_splits + m.split;
+            const size_t slot = (size_t)(m.g * G + row_b) * (teams + n_reqs) + m.place;
 #pragma unroll
             for (int i = 0; i < HD / 8; ++i)
                 *(float2*)(part_o + slot * HD + i * 8 + col) = make_float2(o[i][2], o[i][3]);
@@ -1121,9 +1164,7 @@ extern "C" int RV_SYM(rv_paged_attention_decode_mma)(
     return 0;
 }
 
-// Decode as a stream (one persistent block per SM); same scratch layout as
-// rv_paged_attention_decode_mma with the split that rv_paged_attention_decode_stream_split
-// names (128 or 256 keys: the smaller one when the larger would leave warps without work).
+// Decode as a stream (one persistent block per SM).
 // Needs head size 64 and pages of 8, 16, 32 or 64 tokens; `total_slots` = pages * page_size
 // of the cache tensors.  `status` receives code 12 when a bounded wait runs out.
 #ifdef RV_STREAM
@@ -1154,38 +1195,27 @@ static int kv_map(CUtensorMap* map, const void* cache, long long total_slots, in
     return 0;
 }
 
-extern "C" int RV_SYM(rv_paged_attention_decode_stream_split)(int n_reqs, int max_ctx_len,
-                                                              int num_heads, int num_kv_heads,
-                                                              int n_sms) {
-    if (num_kv_heads <= 0 || n_sms <= 0) return RV_SPLIT;
-    const int G = num_heads / num_kv_heads;
-    const long long items = (long long)n_reqs * ((max_ctx_len + RV_SPLIT - 1) / RV_SPLIT) *
-                            num_kv_heads * ((G + 15) / 16);
-    return items < 3ll * RV_STREAM_WARPS * n_sms ? RV_SPLIT / 2 : RV_SPLIT;
-}
-
+// Writes the requests' segments for rv_paged_attention_merge_segments (places: stream_shares.cuh).
 extern "C" int RV_SYM(rv_paged_attention_decode_stream)(
     const void* q, int q_stride, const void* k_cache, const void* v_cache, long long total_slots,
     const int* block_table, int max_blocks, const int* ctx_lens, void* scratch,
     long long scratch_bytes, int n_reqs, int max_ctx_len, int num_heads, int num_kv_heads,
-    int page_size, float scale, int window, int split_keys, int n_sms, int* status, void* stream) {
+    int page_size, float scale, int window, int n_sms, int* status, void* stream) {
     if (n_reqs == 0) return 0;
     if (num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || n_reqs < 0 || n_sms <= 0)
         return fail("paged_attention_decode_stream: bad sizes");
     if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64)
         return fail("paged_attention_decode_stream: pages of 8, 16, 32 or 64 tokens only");
-    if (split_keys != RV_SPLIT && split_keys != RV_SPLIT / 2)
-        return fail("paged_attention_decode_stream: splits of 128 or 256 keys only");
     if (((uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q) % 16 || (q_stride % 8))
         return fail("paged_attention_decode_stream: caches and query rows must be 16-byte aligned");
-    int max_splits = (max_ctx_len + split_keys - 1) / split_keys;
-    if (max_splits < 1) max_splits = 1;
-    const size_t slots = (size_t)n_reqs * num_heads * max_splits;
-    if ((long long)(slots * RV_VD * 4 + slots * 8) > scratch_bytes)
+    static_assert(RV_STREAM_TILE == RV_BN && RV_VD == 64, "the shares' tiles and rows");
+    const int teams = rv_stream_teams(num_heads, num_kv_heads, n_sms), keys = rv_stream_keys(max_ctx_len);
+    if (rv_stream_bytes(n_reqs, num_heads, teams) > scratch_bytes)
         return fail("paged_attention_decode_stream: scratch too small");
-    const int G = num_heads / num_kv_heads;
-    const int tiles_per_head = (G + 15) / 16;
-    const long long total = (long long)n_reqs * max_splits * num_kv_heads * tiles_per_head;
+    const long long tiles = (long long)n_reqs * (keys / RV_BN);
+    if (tiles > 0x7fffffffll) return fail("paged_attention_decode_stream: too many keys");
+    // as many blocks as there may be runs
+    const long long runs = (tiles < teams ? tiles : teams) * rv_stream_heads(num_heads, num_kv_heads);
     const size_t ring_bytes = (size_t)RV_STREAM_WARPS * RV_STREAM_STAGES * 2 * RV_BN * RV_HD * sizeof(bf16);
     const size_t q_bytes = (size_t)RV_STREAM_WARPS * 2 * 16 * (RV_HD + 8) * sizeof(bf16);
     const size_t smem = ring_bytes + q_bytes + 1024;
@@ -1199,15 +1229,14 @@ extern "C" int RV_SYM(rv_paged_attention_decode_stream)(
     CUtensorMap map_k, map_v;
     if (kv_map(&map_k, k_cache, total_slots, num_kv_heads, page_size)) return 1;
     if (kv_map(&map_v, v_cache, total_slots, num_kv_heads, page_size)) return 1;
-    long long blocks = (total + RV_STREAM_WARPS - 1) / RV_STREAM_WARPS;
+    long long blocks = (runs + RV_STREAM_WARPS - 1) / RV_STREAM_WARPS;
     if (blocks > n_sms) blocks = n_sms;
     float* part_o = (float*)scratch;
-    float2* part_ml = (float2*)((char*)scratch + slots * RV_VD * 4);
+    float2* part_ml = (float2*)(part_o + (size_t)num_heads * (teams + n_reqs) * RV_VD);
     rv_launch(paged_attention_decode_stream_kernel<RV_HD>, dim3((unsigned)blocks),
               dim3(RV_STREAM_WARPS * 32), smem, (cudaStream_t)stream, map_k, map_v,
-              (const bf16*)q, q_stride, block_table, max_blocks, ctx_lens, part_o, part_ml,
-              max_splits, split_keys / RV_BN, num_heads, num_kv_heads, page_size,
-              scale * 1.4426950408889634f, window, n_reqs, status);
+              (const bf16*)q, q_stride, block_table, max_blocks, ctx_lens, part_o, part_ml, keys, teams,
+              num_heads, num_kv_heads, page_size, scale * 1.4426950408889634f, window, n_reqs, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(cudaGetErrorString(e));
     return 0;

@@ -29,6 +29,7 @@
 // Plain reference: tests/plain_ops.py paged_attention.
 #include "attention_pooled.cuh"
 #include "common.cuh"
+#include "stream_shares.cuh"
 
 #define RV_ATTN_MAX_DPL 16     // head sizes up to 512: up to 16 dimensions per lane
 #define RV_ATTN_GT 4           // query heads of a group handled together in decode
@@ -379,6 +380,72 @@ __global__ void paged_attention_merge_kernel(const float* __restrict__ part_o,
     }
 }
 
+// The same for the segments of the stream kernel (stream_shares.cuh; value heads of 64).  A warp has a head, a lane
+// two dimensions; where the request's segments lie is worked out before the wait.
+template <typename T>
+__global__ void __launch_bounds__(128) paged_attention_merge_segments_kernel(
+    const float2* __restrict__ part_o, const float2* __restrict__ part_ml, const int* __restrict__ ctx_lens,
+    T* __restrict__ out, int teams, int n_reqs, int num_heads, int window, int max_ctx,
+    const float* __restrict__ sinks) {
+    rv_pdl_launch_dependents();
+    constexpr int GROUP = 16;
+    constexpr bool kFast = sizeof(T) == 2;
+    const int r = blockIdx.y, h = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (h >= num_heads) {
+        rv_pdl_wait();
+        return;
+    }
+    const int clen = ctx_lens[r];                 // the step's index array: before the wait
+    const float sink = sinks ? sinks[h] : -INFINITY;      // a constant of the layer
+    RvStreamShares sh(ctx_lens, n_reqs, window, max_ctx, teams);
+    int start = 0;
+    for (int at = 0; at < r; at += 32) {
+        if (sh.grp != at) sh.load_group(at);
+        start += __reduce_add_sync(0xffffffffu, at + lane < r ? sh.tiles_of(sh.grp_len) : 0);
+    }
+    const int tiles = sh.tiles_of(clen);
+    const int run0 = tiles ? sh.run_of(start) : 0;
+    const int n = tiles ? sh.run_of(start + tiles - 1) - run0 + 1 : 0;
+    rv_pdl_wait();
+    T* o = out + ((size_t)r * num_heads + h) * 64 + lane * 2;
+    if (n == 0) {                                 // nothing to see; more than the launch was told of
+        const float v = clen == 0 ? 0.f : NAN;
+        rv_store(o, v);
+        rv_store(o + 1, v);
+        return;
+    }
+    const size_t base = (size_t)h * (teams + n_reqs) + run0 + r;
+    float M = sink, L = sinks ? 1.f : 0.f;        // the sink counts once, here
+    float2 O = make_float2(0.f, 0.f);
+    // sixteen at a time: a group's loads are independent
+    for (int sb = 0; sb < n; sb += GROUP) {
+        const int cnt = min(GROUP, n - sb);
+        float2 ml = lane < cnt ? part_ml[base + sb + lane] : make_float2(-INFINITY, 0.f);
+        float2 po[GROUP];
+#pragma unroll
+        for (int i = 0; i < GROUP; ++i)
+            po[i] = i < cnt ? part_o[(base + sb + i) * 32 + lane] : make_float2(0.f, 0.f);
+        float mg = fmaxf(M, ml.x);
+#pragma unroll
+        for (int d = 16; d; d >>= 1) mg = fmaxf(mg, __shfl_xor_sync(0xffffffffu, mg, d));
+        if (mg == -INFINITY) continue;
+        const float keep = rv_exp<kFast>(M - mg);          // M = -inf -> 0
+        const float w = ml.y > 0.f ? rv_exp<kFast>(ml.x - mg) : 0.f;
+        L = L * keep + rv_warp_sum(ml.y * w);
+        O.x *= keep;
+        O.y *= keep;
+#pragma unroll
+        for (int i = 0; i < GROUP; ++i) {
+            const float wi = __shfl_sync(0xffffffffu, w, i);
+            O.x += po[i].x * wi;
+            O.y += po[i].y * wi;
+        }
+        M = mg;
+    }
+    rv_store(o, L > 0.f ? O.x / L : 0.f);
+    rv_store(o + 1, L > 0.f ? O.y / L : 0.f);
+}
+
 // ---------------------------------------------------------------------------------
 static int check_attention_sizes(const char* name, int num_heads, int num_kv_heads, int hd, int vd,
                                  int page_size, int dtype) {
@@ -532,6 +599,30 @@ extern "C" int rv_paged_attention_merge_ex(const void* scratch, const int* ctx_l
             sinks, 0, 0, 0)));
     RV_CHECK_LAUNCH("paged_attention_merge");
     return 0;
+}
+
+// The merge of the stream kernel's segments (bytes of scratch: rv_paged_attention_stream_scratch_bytes).
+extern "C" int rv_paged_attention_merge_segments(const void* scratch, const int* ctx_lens, void* out,
+                                                 int dtype, int n_reqs, int max_ctx_len, int num_heads,
+                                                 int num_kv_heads, int window, int n_sms, const float* sinks,
+                                                 void* stream) {
+    if (n_reqs == 0) return 0;
+    if (n_reqs < 0 || n_reqs > 65535 || num_heads <= 0 || num_kv_heads <= 0 || num_heads % num_kv_heads || n_sms <= 0)
+        RV_FAIL("paged_attention_merge: bad sizes");
+    const int teams = rv_stream_teams(num_heads, num_kv_heads, n_sms);
+    const float2* part_o = (const float2*)scratch;
+    const float2* part_ml = part_o + (size_t)num_heads * (teams + n_reqs) * 32;
+    RV_DISPATCH_DTYPE(dtype, "paged_attention_merge",
+        (rv_launch(paged_attention_merge_segments_kernel<T>, dim3((num_heads + 3) / 4, n_reqs), dim3(128), 0,
+            (cudaStream_t)stream, part_o, part_ml, ctx_lens, (T*)out, teams, n_reqs, num_heads, window,
+            rv_stream_keys(max_ctx_len), sinks)));
+    RV_CHECK_LAUNCH("paged_attention_merge");
+    return 0;
+}
+
+// Whatever the heads share (no launch has more teams than warps).
+extern "C" long long rv_paged_attention_stream_scratch_bytes(int n_reqs, int num_heads, int n_sms) {
+    return rv_stream_bytes(n_reqs, num_heads, n_sms * RV_STREAM_WARPS);
 }
 
 extern "C" int rv_paged_attention_merge(const void* scratch, const int* ctx_lens, void* out,

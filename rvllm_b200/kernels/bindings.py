@@ -49,6 +49,7 @@ class CudaOps:
         self.launches = 0
         self.lib.rv_last_error.restype = ctypes.c_char_p
         self.lib.rv_paged_attention_decode_scratch_bytes.restype = c_longlong
+        self.lib.rv_paged_attention_stream_scratch_bytes.restype = c_longlong
         self.lib.rv_gemm_tiled_bytes.restype = c_longlong
         self.lib.rv_gated_delta_scratch.restype = c_longlong
         self.lib.rv_gemm_f32_split_scratch.restype = c_longlong
@@ -71,9 +72,11 @@ class CudaOps:
         self.decode_split = int(os.environ.get("RVLLM_ATTN_DECODE_SPLIT", "256"))
         # "stream": one persistent block per SM whose warps each stream their work items'
         # tiles through a private ring; "block": one block per (request, head, split);
-        # "auto": the stream kernel from `stream_min_items` work items of 256 keys on
+        # "auto": the stream kernel from `stream_min_items` work items of 256 keys on, by default always (us
+        # block / stream, 32 / 8 heads: 1 request of 40 keys 6.4 / 4.2, of 4,000 9.8 / 6.3; 8 of some 240
+        # 10.0 / 4.4)
         self.decode_kernel = os.environ.get("RVLLM_ATTN_DECODE_KERNEL", "auto")
-        self.stream_min_items = int(os.environ.get("RVLLM_ATTN_STREAM_MIN_ITEMS", "384"))
+        self.stream_min_items = int(os.environ.get("RVLLM_ATTN_STREAM_MIN_ITEMS", "0"))
         self._sm_count = torch.cuda.get_device_properties(
             torch.cuda.current_device()).multi_processor_count
         # bfloat16 products with at most `gemm_small_m` tokens go to the tcgen05
@@ -495,6 +498,9 @@ class CudaOps:
         smallest split any of them uses, 128 keys)."""
         decode = int(self.lib.rv_paged_attention_decode_scratch_bytes(
             c_int(n_reqs), c_int(num_heads), c_int(head_dim), c_int(2 * max_ctx_len)))
+        if head_dim == 64:
+            decode = max(decode, int(self.lib.rv_paged_attention_stream_scratch_bytes(
+                c_int(n_reqs), c_int(num_heads), c_int(self._sm_count))))
         return max(decode, self._prefill_scratch_bytes(head_dim))
 
     def reserve_scratch(self, nbytes: int, device) -> None:
@@ -761,14 +767,11 @@ class CudaOps:
             items = (n_reqs * -(-max_ctx_len // 256) * num_kv_heads
                      * -(-(num_heads // num_kv_heads) // 16))
             stream = items >= self.stream_min_items
-        if stream:
-            split = getattr(lib, f"rv_paged_attention_decode_stream_split_hd{head_dim}")(
-                c_int(n_reqs), c_int(max_ctx_len), c_int(num_heads), c_int(num_kv_heads),
-                c_int(self._sm_count))
-        else:
-            split = self.decode_split
-        need = self.lib.rv_paged_attention_decode_scratch_bytes(
-            c_int(n_reqs), c_int(num_heads), c_int(vd), c_int(max_ctx_len * (256 // split)))
+        split = self.decode_split
+        need = int(self.lib.rv_paged_attention_stream_scratch_bytes(
+            c_int(n_reqs), c_int(num_heads), c_int(self._sm_count)) if stream
+            else self.lib.rv_paged_attention_decode_scratch_bytes(
+                c_int(n_reqs), c_int(num_heads), c_int(vd), c_int(max_ctx_len * (256 // split))))
         if scratch is None:
             scratch = self._scratch_buffer(need, qkv.device)
         win = c_int(window if window else 0)
@@ -780,12 +783,12 @@ class CudaOps:
                 c_int(block_table.shape[1]), _ptr(ctx_lens), _ptr(scratch),
                 c_longlong(scratch.numel() * scratch.element_size()), c_int(n_reqs),
                 c_int(max_ctx_len), c_int(num_heads), c_int(num_kv_heads), c_int(page_size),
-                c_float(scale), win, c_int(split), c_int(self._sm_count),
+                c_float(scale), win, c_int(self._sm_count),
                 _ptr(self._gemm_status(qkv.device)), self._stream()),
                 "paged_attention_decode_stream")
-            self._check(self.lib.rv_paged_attention_merge_ex(
+            self._check(self.lib.rv_paged_attention_merge_segments(
                 _ptr(scratch), _ptr(ctx_lens), _ptr(out), _code(out.dtype), c_int(n_reqs),
-                c_int(max_ctx_len), c_int(num_heads), c_int(head_dim), win, c_int(split),
+                c_int(max_ctx_len), c_int(num_heads), c_int(num_kv_heads), win, c_int(self._sm_count),
                 _ptr(sinks), self._stream()), "paged_attention_merge")
             return
         fn = getattr(lib, f"rv_paged_attention_decode_mma_{tag}")

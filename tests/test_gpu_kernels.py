@@ -293,6 +293,40 @@ def test_paged_attention(ops, dtype, case, standout):
     assert torch.allclose(out2.cpu().float(), ref.float(), **t)
 
 
+@pytest.mark.parametrize("reqs,nh,nkv,ps,window", [
+    (1, 4, 4, 16, None),          # a request over all runs
+    (3, 8, 2, 64, None),
+    (31, 4, 2, 16, None),
+    (70, 4, 2, 16, None),         # more requests than a warp looks up at once, several in a run
+    (70, 6, 2, 8, 129),
+    (33, 32, 1, 32, None),        # two teams' warps a key/value head
+    (9, 300, 300, 16, 100),       # more heads than a quarter of the warps: several runs a warp
+])
+def test_decode_stream_runs(ops, reqs, nh, nkv, ps, window):
+    """The stream kernel shares the step's tiles out in runs that end anywhere: contexts of all lengths around a
+    tile's and a run's edge, empty ones between them.  Bounds as in `test_paged_attention`."""
+    hd = 64
+    lens = [(1, 64, 700, 65, 3, 128, 129, 1500, 200, 63)[i % 10] if nh < 100 else 60 + 70 * i for i in range(reqs)]
+    g = torch.Generator().manual_seed(11)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, [1] * reqs, lens, nh, nkv, hd, ps, window)
+    for r in range(5, reqs, 13):
+        ctx.ctx_lens[r] = 0
+        group.block_table[r] = -1
+    ref = torch.zeros(reqs, nh * hd, dtype=torch.bfloat16)
+    PlainOps().paged_attention(q, nh, nkv, hd, kc, vc, ctx, group, 0.125, window, ref)
+    ref[ctx.ctx_lens == 0] = 0
+    out = torch.full((reqs, nh * hd), float("nan"), dtype=torch.bfloat16, device="cuda")
+    chosen = ops.decode_kernel
+    try:
+        ops.decode_kernel = "stream"
+        ops.paged_attention(q.cuda(), nh, nkv, hd, kc.cuda(), vc.cuda(), to_cuda(ctx), to_cuda(group), 0.125,
+                            window, out)
+        ops.check_status()
+    finally:
+        ops.decode_kernel = chosen
+    assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
+
+
 EDGE_CASES = [
     # q_len, context, window, page: where the window's first key `lo` of the last (and, for a
     # portion, of the first) query falls
