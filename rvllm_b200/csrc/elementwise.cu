@@ -5,6 +5,9 @@
 #include "common.cuh"
 
 static thread_local char g_error[512] = "";
+// See rv_whole_launch.
+extern "C" void rv_next_launch_whole() { rv_whole_launch() = 1; }
+
 extern "C" const char* rv_last_error() { return g_error; }
 void rv_set_error(const char* fmt, ...) {
     va_list ap;
