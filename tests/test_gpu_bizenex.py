@@ -306,6 +306,40 @@ def test_moe_select(ops, shape):
         assert abs(float(wts[t].sum()) - 1.0) < 1e-5
 
 
+@pytest.mark.parametrize("score", ["sigmoid", "softmax", "chosen"])
+@pytest.mark.parametrize("shape", [(16, 4, 4, 2, 2), (32, 32, 1, 1, 1), (32, 5, 8, 3, 1), (30, 7, 5, 3, 3), (2, 1, 2, 1, 2),
+                                   (17, 3, 1, 1, 1)])
+def test_moe_select_by_ranks(ops, shape, score):
+    """Up to 32 experts are chosen by ranks, more by taking the largest out in turn: the same with experts among
+    them that nobody chooses, for equal scores and scores that are not finite too."""
+    E, top, groups, keep, group_top = shape
+    modes = {"sigmoid": 0, "softmax": 1, "chosen": 2}
+    name = next(k for k, v in ops.SCORE_MODES.items() if v == modes[score])
+    g = torch.Generator().manual_seed(E + top)
+    n, size = 150, E // groups
+    logits = (torch.randn(n, E, generator=g) * 2).round(decimals=1)       # some are equal
+    logits[0] = 0.0
+    if top < E:
+        logits[1, E - 1] = -float("inf")
+    wide = size + 40
+    at = (torch.arange(E) // size) * wide + torch.arange(E) % size
+    more = torch.full((n, groups * wide), -1e30)
+    more[:, at] = logits
+    for bias in (None, torch.randn(E, generator=g) * 0.3):
+        out = []
+        for lg, b in ((logits, bias), (more, None if bias is None else torch.full((groups * wide,), -1e30).index_copy(
+                0, at, bias))):
+            ids = torch.empty(n, top, dtype=torch.int32, device="cuda")
+            wts = torch.empty(n, top, dtype=torch.float32, device="cuda")
+            ops.moe_select(dev(lg), groups, keep, group_top, 1e-20, ids, wts, score=name, route_scale=1.5,
+                           choice_bias=None if b is None else dev(b))
+            out.append((ids.cpu().long(), wts.cpu()))
+        assert torch.equal(at[out[0][0]], out[1][0])
+        # (a softmax's sum is of as many in another order: 2 ulp of the sum, the quotient and the weights' sum)
+        tol = dict(rtol=8 * 2.0 ** -24, atol=0) if score == "softmax" else dict(rtol=0, atol=0)
+        assert torch.allclose(out[0][1], out[1][1], **tol)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("shape", [(50, 5, 2, 5, 3), (96, 8, 3, 2, 1), (1024, 64, 6, 8, 3), (333, 9, 3, 1, 1),
                                    (256, 128, 8, 8, 4), (4000, 16, 4, 4, 2)])
