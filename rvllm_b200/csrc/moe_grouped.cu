@@ -3,11 +3,11 @@
 // on the 5th-generation tensor cores.
 //
 //   moe_sort      ids [N, top] -> a layout of rows in which expert e owns a stretch that
-//                 begins at a multiple of TN rows: sorted_token[row] = the pair's token (-1: a
-//                 filling row), pair_pos[pair] = its row, and the list of token tiles
-//                 (tile_expert, tile_row0, n_tiles).  Counts stay on the device, so a captured
+//                 begins at a multiple of TN rows: pair_pos[pair] = its row, and the list of token
+//                 tiles (tile_expert, tile_row0, n_tiles).  Counts stay on the device, so a captured
 //                 launch sequence serves any routing.
-//   moe_gather    xs[row] = x[sorted_token[row]] (zeros for filling rows).
+//   moe_gather    xs[pair_pos[pair]] = x[the pair's token].  Rows that fill a tile up stay as they are:
+//                 a row's sums are of its own values only, and nobody reads theirs.
 //   moe_grouped   out[row0 + t, n] = <xs[row0 + t], W[e][n]> for the rows of one token tile and
 //                 128 rows of W[e] per block: 128 rows of W are the M side of a tcgen05.mma
 //                 (cta_group::1, kind::f16, M = 128), the TN tokens its N side, the accumulator
@@ -36,64 +36,78 @@
 #define MG_SMEM_LIMIT (110 * 1024)     // two blocks an SM: one's epilogue beside the other's products
 #define MG_SMEM_MAX (200 * 1024)
 
-__global__ void moe_sort_kernel(const int* __restrict__ ids, int P, int E, int top, int TN,
-                                int rows_pad, int max_tiles, int* __restrict__ sorted_token,
-                                int* __restrict__ pair_pos, int* __restrict__ tile_expert,
-                                int* __restrict__ tile_row0, int* __restrict__ n_tiles) {
+// One block.  A pair's place among its expert's is counted with one addition a warp and expert (3,108 pairs of
+// 16 experts: 7.2 us with one a pair, twice, and the tiles listed by one thread).
+__global__ void __launch_bounds__(1024) moe_sort_kernel(
+    const int* __restrict__ ids, int P, int E, int TN, int max_tiles, int* __restrict__ pair_pos,
+    int* __restrict__ tile_expert, int* __restrict__ tile_row0, int* __restrict__ n_tiles) {
     rv_pdl_prologue();
     extern __shared__ int sm[];
-    int* cnt = sm;             // [E]
-    int* off = cnt + E;        // [E]
-    int* cur = off + E;        // [E]
-    for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = cur[e] = 0;
+    int* cnt = sm;             // [E] rows
+    int* off = cnt + E;        // [E] first row
+    int* first = off + E;      // [E] first tile
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < P; p += blockDim.x) {
-        const int e = ids[p];
-        if (e >= 0 && e < E) atomicAdd(&cnt[e], 1);
+#pragma unroll 4
+    for (int p0 = threadIdx.x - lane; p0 < P; p0 += blockDim.x) {
+        const int p = p0 + lane;
+        const int e = p < P ? ids[p] : -1;
+        const bool valid = e >= 0 && e < E;
+        const unsigned same = __match_any_sync(0xffffffffu, valid ? e : -1);
+        const int leader = __ffs(same) - 1;
+        int at = 0;
+        if (valid && lane == leader) at = atomicAdd(&cnt[e], __popc(same));
+        at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1u));
+        if (p < P) pair_pos[p] = valid ? at : e >= E ? -1 : 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int row = 0, tiles = 0;
-        for (int e = 0; e < E; ++e) {
-            off[e] = row;
-            const int nt = (cnt[e] + TN - 1) / TN;
-            for (int i = 0; i < nt && tiles < max_tiles; ++i) {
-                tile_expert[tiles] = e;
-                tile_row0[tiles] = row + i * TN;
-                ++tiles;
+    if (warp == 0) {
+        int tiles = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int nt = e0 + lane < E ? (cnt[e0 + lane] + TN - 1) / TN : 0;
+            int upto = nt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += v;
             }
-            row += nt * TN;
+            if (e0 + lane < E) {
+                first[e0 + lane] = tiles + upto - nt;
+                off[e0 + lane] = (tiles + upto - nt) * TN;
+            }
+            tiles += __shfl_sync(0xffffffffu, upto, 31);
         }
-        n_tiles[0] = tiles;
+        if (lane == 0) n_tiles[0] = min(tiles, max_tiles);
     }
-    for (int r = threadIdx.x; r < rows_pad; r += blockDim.x) sorted_token[r] = -1;
     __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        const int nt = (cnt[e] + TN - 1) / TN;
+        for (int i = 0; i < nt && first[e] + i < max_tiles; ++i) {
+            tile_expert[first[e] + i] = e;
+            tile_row0[first[e] + i] = off[e] + i * TN;
+        }
+    }
+#pragma unroll 4
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
         const int e = ids[p];
-        int pos = e >= E ? -1 : 0;
-        if (e >= 0 && e < E) {
-            pos = off[e] + atomicAdd(&cur[e], 1);
-            if (pos < rows_pad) sorted_token[pos] = p / top;
-        }
-        pair_pos[p] = pos;
+        if (e >= 0 && e < E) pair_pos[p] += off[e];
     }
 }
 
-// one warp per row; width a multiple of 8
-__global__ void moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ sorted_token,
-                                  bf16* __restrict__ xs, int rows, int W) {
-    rv_pdl_prologue();
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= rows) return;
-    const int t = sorted_token[warp];
-    uint4* dst = (uint4*)(xs + (size_t)warp * W);
-    if (t < 0) {
-        for (int i = lane; i < W / 8; i += 32) dst[i] = make_uint4(0, 0, 0, 0);
-        return;
+// one block per token; width a multiple of 8
+__global__ void moe_gather_kernel(const bf16* __restrict__ x, const int* __restrict__ pair_pos,
+                                  bf16* __restrict__ xs, int top, int rows, int W) {
+    rv_pdl_launch_dependents();
+    const int t = blockIdx.x;
+    rv_pdl_wait();
+    for (int i = threadIdx.x; i < W / 8; i += blockDim.x) {
+        const uint4 v = ((const uint4*)(x + (size_t)t * W))[i];
+        for (int k = 0; k < top; ++k) {
+            const int row = pair_pos[(size_t)t * top + k];
+            if (row >= 0 && row < rows) ((uint4*)(xs + (size_t)row * W))[i] = v;
+        }
     }
-    const uint4* src = (const uint4*)(x + (size_t)t * W);
-    for (int i = lane; i < W / 8; i += 32) dst[i] = src[i];
 }
 
 // one block per token; width a multiple of 8
@@ -358,12 +372,17 @@ static int grouped_product(const void* xs, const void* w, void* out, int* status
     if (make_map(&map_w, w, (long long)E * n_out, K, MG_BM)) return 1;
     if (make_map(&map_x, xs, rows, K, TN)) return 1;
     const int kblocks = (K + MG_BK - 1) / MG_BK;
-    // two tiles of W a block where there are many tokens an expert and rows of W enough
-    // (RVLLM_MOE_MT=1 or 2 forces it)
-    static int forced_mt = getenv("RVLLM_MOE_MT") ? atoi(getenv("RVLLM_MOE_MT")) : 0;
-    int MT = (TN >= 128 && n_out >= 4 * MG_BM) ? 2 : 1;
-    if (forced_mt == 1 || forced_mt == 2) MT = forced_mt;
-    static int smem_limit = getenv("RVLLM_MOE_SMEM_KB") ? atoi(getenv("RVLLM_MOE_SMEM_KB")) * 1024 : MG_SMEM_LIMIT;
+    // Two tiles of W a block where there are many tokens an expert, rows of W enough and, with that, more blocks
+    // than multiprocessors; else one, in a ring as deep as a multiprocessor's memory if there are no more blocks
+    // of it either (the tiles are those of even shares: the counts are not known here).  Us, 16 experts,
+    // 4 a token, n_out x K, two tiles / one / one in the deep ring: 256 tokens, 1024 x 1024 22.7 / 16.3 / 13.7,
+    // 2048 x 1024 25.8 / 22.3 / 26.3; 777, 1024 x 1024 21.4 / 15.8 / 21.9, 2048 x 1024 27.8 / 30.7 / 43;
+    // 2,048, 1024 x 1024 22.9 / 26.6 / 41.  (Tiles of 256 tokens, a block an SM: 777, 2048 x 1024 26.3, but 1,000
+    // 42.4 against 41.8, 2,048 60 against 47.)
+    const long long tiles = max_tiles - E + (E + 1) / 2;
+    const int w_tiles = (n_out + MG_BM - 1) / MG_BM, sms = rv_sm_count();
+    const int MT = TN >= 128 && n_out >= 4 * MG_BM && tiles * ((w_tiles + 1) / 2) > sms ? 2 : 1;
+    const int smem_limit = MT == 1 && tiles * w_tiles <= sms ? MG_SMEM_MAX : MG_SMEM_LIMIT;
     const int per_stage = MT * MG_BM * MG_BK * 2 + TN * MG_BK * 2;
     int stages = (smem_limit - 1024) / per_stage;
     if (stages > 6) stages = 6;
@@ -390,7 +409,7 @@ static int grouped_product(const void* xs, const void* w, void* out, int* status
 extern "C" long long rv_moe_grouped_scratch_bytes(int n_tokens, int top, int E, int W, int F, int TN) {
     const long long pairs = (long long)n_tokens * top;
     const long long rows = rv_moe_grouped_rows((int)pairs, E, TN);
-    const long long ints = rows + pairs + 2 * (rows / TN) + 4;
+    const long long ints = pairs + 2 * (rows / TN) + 4;
     return ((ints * 4 + 255) & ~255ll) + rows * ((long long)W * 2 + (long long)F * 2 + (long long)W * 2) + 256;
 }
 
@@ -419,21 +438,21 @@ extern "C" int rv_moe_experts_grouped(const void* x, const int* ids, const float
     const long long rows = rv_moe_grouped_rows((int)pairs, E, TN);
     const int max_tiles = (int)(rows / TN);
     if (max_tiles > 65535) RV_FAIL("moe_experts_grouped: too many token tiles");
-    int* sorted_token = (int*)scratch;
-    int* pair_pos = sorted_token + rows;
+    int* pair_pos = (int*)scratch;
     int* tile_expert = pair_pos + pairs;
     int* tile_row0 = tile_expert + max_tiles;
     int* n_tiles = tile_row0 + max_tiles;
-    const long long ints = rows + pairs + 2 * (long long)max_tiles + 4;
+    const long long ints = pairs + 2 * (long long)max_tiles + 4;
     bf16* xs = (bf16*)((char*)scratch + ((ints * 4 + 255) & ~255ll));
     bf16* act = xs + rows * W;
     bf16* ys = act + rows * F;
     cudaStream_t s = (cudaStream_t)stream;
     rv_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)3 * E * sizeof(int), s, ids, (int)pairs, E,
-              top, TN, (int)rows, max_tiles, sorted_token, pair_pos, tile_expert, tile_row0, n_tiles);
+              TN, max_tiles, pair_pos, tile_expert, tile_row0, n_tiles);
     RV_CHECK_LAUNCH("moe_sort");
-    rv_launch(moe_gather_kernel, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, s, (const bf16*)x,
-              (const int*)sorted_token, xs, (int)rows, W);
+    const int row_threads = W / 8 < 256 ? ((W / 8 + 31) / 32) * 32 : 256;
+    rv_launch(moe_gather_kernel, dim3(n_tokens), dim3(row_threads), 0, s, (const bf16*)x, (const int*)pair_pos,
+              xs, top, (int)rows, W);
     RV_CHECK_LAUNCH("moe_gather");
     if (grouped_product(xs, gate_up, act, status, tile_expert, tile_row0, n_tiles, rows, E,
                         act_mode == 2 ? F : 2 * F, W, TN, max_tiles,
@@ -442,7 +461,7 @@ extern "C" int rv_moe_experts_grouped(const void* x, const int* ids, const float
     if (grouped_product(act, down, ys, status, tile_expert, tile_row0, n_tiles, rows, E, W, F, TN,
                         max_tiles, 0, 0.f, 0.f, s))
         return 1;
-    rv_launch(moe_combine_kernel, dim3(n_tokens), dim3(W / 8 < 256 ? ((W / 8 + 31) / 32) * 32 : 256), 0,
+    rv_launch(moe_combine_kernel, dim3(n_tokens), dim3(row_threads), 0,
               s, (const bf16*)ys, (const int*)pair_pos, weights, (const bf16*)addend, (const bf16*)x,
               (bf16*)out, top, W);
     RV_CHECK_LAUNCH("moe_combine");
