@@ -611,8 +611,8 @@ __global__ void __launch_bounds__(NW * 32) paged_attention_decode_mma_kernel(
 // the run leaves a request, the rows so far go to memory as one of the request's segments, which
 // paged_attention_merge_segments_kernel (attention_simt.cu) puts together in order.
 // Splits of 128 or 256 keys, dealt out in turns, left some warps twice the others' work, and a replay's also
-// splits without keys.  Us with the merge, 32 / 8 heads, splits / runs: 8 requests of some 2,300 keys 14.2 / 13.0,
-// 31 of 950 20.7 / 17.9, 64 of 3,100 80.3 / 73.4 (5.6 TB/s), 8 of 240 7.3 / 5.3.
+// splits without keys.  Us with the merge, 32 / 8 heads, splits / runs: 8 requests of some 2,300 keys 14.2 / 11.6,
+// 31 of 950 20.7 / 16.2, 64 of 3,100 80.3 / 68.7 (5.9 TB/s), 8 of 240 7.3 / 4.4.
 // The copy of the next tile -- of the next segment, when this one ends -- is in flight while a
 // tile is computed, the block table entries are fetched one piece (up to 32 pages) ahead of
 // the one being loaded, and a segment's query rows arrive by cp.async; so the warp
