@@ -306,15 +306,13 @@ def test_moe_select(ops, shape):
         assert abs(float(wts[t].sum()) - 1.0) < 1e-5
 
 
-@pytest.mark.parametrize("score", ["sigmoid", "softmax", "chosen"])
-@pytest.mark.parametrize("shape", [(16, 4, 4, 2, 2), (32, 32, 1, 1, 1), (32, 5, 8, 3, 1), (30, 7, 5, 3, 3), (2, 1, 2, 1, 2),
+@pytest.mark.parametrize("score", ["sigmoid", "softmax", "softmax_chosen"])
+@pytest.mark.parametrize("shape", [(16, 4, 4, 2, 2), (32, 32, 1, 1, 1), (32, 5, 8, 3, 1), (30, 7, 5, 3, 3), (2, 1, 2, 1, 1),
                                    (17, 3, 1, 1, 1)])
 def test_moe_select_by_ranks(ops, shape, score):
     """Up to 32 experts are chosen by ranks, more by taking the largest out in turn: the same with experts among
     them that nobody chooses, for equal scores and scores that are not finite too."""
     E, top, groups, keep, group_top = shape
-    modes = {"sigmoid": 0, "softmax": 1, "chosen": 2}
-    name = next(k for k, v in ops.SCORE_MODES.items() if v == modes[score])
     g = torch.Generator().manual_seed(E + top)
     n, size = 150, E // groups
     logits = (torch.randn(n, E, generator=g) * 2).round(decimals=1)       # some are equal
@@ -331,7 +329,7 @@ def test_moe_select_by_ranks(ops, shape, score):
                 0, at, bias))):
             ids = torch.empty(n, top, dtype=torch.int32, device="cuda")
             wts = torch.empty(n, top, dtype=torch.float32, device="cuda")
-            ops.moe_select(dev(lg), groups, keep, group_top, 1e-20, ids, wts, score=name, route_scale=1.5,
+            ops.moe_select(dev(lg), groups, keep, group_top, 1e-20, ids, wts, score=score, route_scale=1.5,
                            choice_bias=None if b is None else dev(b))
             out.append((ids.cpu().long(), wts.cpu()))
         assert torch.equal(at[out[0][0]], out[1][0])
