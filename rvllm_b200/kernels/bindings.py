@@ -420,7 +420,7 @@ class CudaOps:
                 y = torch.mm(xp, w.t()).to(out_dtype)
             if y.shape[0] != m:
                 y = y[:m]
-            if torch.cuda.is_current_stream_capturing():
+            if y.is_cuda and torch.cuda.is_current_stream_capturing():
                 self.lib.rv_next_launch_whole()
         if bias is not None:
             self.add_bias(y, bias)
