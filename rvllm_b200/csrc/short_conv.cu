@@ -245,12 +245,15 @@ __global__ void short_conv_vec4_kernel(const T* __restrict__ proj, const float* 
     }
 }
 
-// Long prompt portions: a thread owns eight adjacent channels (one 16-byte access per bfloat16
-// row) of a chunk of 16 tokens and requests the rows of half a chunk (B, C and x of 8 tokens:
-// 24 independent loads; a quarter chunk in float32) before it uses any of them, so that enough bytes are in flight to
-// run at memory speed; the sums are formed in the same order as in the kernels above, so the
+// Portions: a thread owns eight adjacent channels (one 16-byte access per bfloat16
+// row) of R consecutive tokens and requests all that it reads (B, C and x of its tokens, the window before them and,
+// for the new state, the portion's last rows) before it uses any of it: a launch is one latency for the index
+// arrays and one for the rows (LOOP: several rounds of R tokens).  The blocks are those that have tokens, found from
+// `q_start`: blocks for every request as if it were the longest, 16 tokens each in two rounds, took 6.2 us in a replay
+// for a portion of 512 beside 31 single tokens of 1,024 channels, 3.3 now; four portions of some 33 float32 tokens of
+// 1,536 channels, token after token, 11.9 and 2.9.
+// The sums are formed in the same order as in the kernels above, so the
 // three give the same numbers.  Filters of at most 4 taps, widths that are a multiple of 8.
-#define RV_CONV_WIDE_CHUNK 16
 
 struct RvRaw8Bf16 { uint4 v; };
 struct RvRaw8F32 { float4 a, b; };
@@ -292,23 +295,42 @@ __device__ __forceinline__ void rv_conv_store8(float* p, const float (&v)[8]) {
     *(float4*)(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
 }
 
-template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) short_conv_wide_kernel(
+template <typename T, int TAPS, int R, bool LOOP>
+__global__ void __launch_bounds__(128) short_conv_rows_kernel(
     const T* __restrict__ proj, const float* __restrict__ filter, const float* __restrict__ in_bias,
     const float* __restrict__ conv_bias, float* __restrict__ state, const int* __restrict__ q_start,
     const int* __restrict__ state_slot, const int* __restrict__ start_pos, T* __restrict__ out,
-    int hidden) {
+    int hidden, int n_reqs, int rounds) {
     typedef typename RvRaw8<T>::type Raw;
-    constexpr int ROWS = sizeof(T) == 2 ? 8 : 4;       // rows requested together: 24 loads of 16 bytes
-    constexpr int HIST = TAPS - 1;
+    constexpr int HIST = TAPS - 1, H1 = HIST > 0 ? HIST : 1;
+    static_assert(R >= 2 && HIST <= R + 1, "a portion that one thread does not end has as many rows as the window");
     rv_pdl_launch_dependents();
+    // the request of this block's tokens: pieces of R tokens a round, request after request
+    const int piece = LOOP ? R * rounds : R;
+    int r = -1, t0 = 0, q0 = 0, qlen = 0;
+    for (int at = 0, before = 0; at < n_reqs; at += 32) {
+        const int lane = threadIdx.x & 31, mine = at + lane;
+        const int qs = mine < n_reqs ? q_start[mine] : 0, n = mine < n_reqs ? q_start[mine + 1] - qs : 0;
+        const int pieces = (n + piece - 1) / piece;
+        int upto = pieces;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += v;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, before + upto > (int)blockIdx.y);
+        if (past) {
+            const int j = __ffs(past) - 1;
+            r = at + j;
+            t0 = ((int)blockIdx.y - before - __shfl_sync(0xffffffffu, upto - pieces, j)) * piece;
+            q0 = __shfl_sync(0xffffffffu, qs, j);
+            qlen = __shfl_sync(0xffffffffu, n, j);
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
-    if (c >= hidden) return;
-    const int r = blockIdx.y;
-    const int q0 = q_start[r];
-    const int qlen = q_start[r + 1] - q0;
-    const int t0 = blockIdx.z * RV_CONV_WIDE_CHUNK;
-    if (t0 >= qlen) return;
+    if (r < 0 || c >= hidden) return;
     const int slot = state_slot[r];
     const bool has_state = slot >= 0 && start_pos[r] > 0 && HIST > 0;
     float* st = slot >= 0 ? state + (size_t)slot * HIST * hidden + c : nullptr;
@@ -336,43 +358,59 @@ __global__ void __launch_bounds__(128) short_conv_wide_kernel(
 #pragma unroll
         for (int i = 0; i < 8; ++i) o[i] = (b[i] + bb[i]) * (x[i] + bxb[i]);
     };
-    auto bx_at = [&](int rel, float (&o)[8]) {
-        const T* p = proj + (size_t)(q0 + rel) * stride + c;
-        bx_of(rv_conv_raw8(p), rv_conv_raw8(p + 2 * hidden), o);
-    };
     rv_pdl_wait();
-    float old[HIST > 0 ? HIST : 1][8], win[HIST > 0 ? HIST : 1][8];
+    const int last = min(piece, qlen - t0) - 1;
+    const T* p0 = proj + (size_t)(q0 + t0) * stride + c;
+    // the rows (past the portion's end the last one again, not used), the window's and the new state's
+    Raw rb[R], rc[R], rx[R], wb[H1], wx[H1], nb[H1], nx[H1];
+    float old[H1][8];
+    const bool ends_here = qlen <= piece;          // the new state is the window that this thread ends with
+    const bool moves = t0 == 0 && st && HIST > 0;
+    auto request = [&](int tb) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const T* p = p0 + (size_t)min(tb + j, last) * stride;
+            rb[j] = rv_conv_raw8(p);
+            rc[j] = rv_conv_raw8(p + hidden);
+            rx[j] = rv_conv_raw8(p + 2 * hidden);
+        }
+    };
+    request(0);
 #pragma unroll
     for (int k = 0; k < HIST; ++k) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) old[k][i] = win[k][i] = 0.f;
         const int rel = t0 - HIST + k;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) old[k][i] = 0.f;
         if (rel >= 0) {
-            bx_at(rel, win[k]);
+            const T* p = proj + (size_t)(q0 + rel) * stride + c;
+            wb[k] = rv_conv_raw8(p);
+            wx[k] = rv_conv_raw8(p + 2 * hidden);
         } else if (has_state) {
             const float* sp = st + (size_t)(HIST + rel) * hidden;
             const float4 a = *(const float4*)sp, b = *(const float4*)(sp + 4);
             old[k][0] = a.x; old[k][1] = a.y; old[k][2] = a.z; old[k][3] = a.w;
             old[k][4] = b.x; old[k][5] = b.y; old[k][6] = b.z; old[k][7] = b.w;
+        }
+        if (moves && !ends_here) {
+            const T* p = proj + (size_t)(q0 + qlen + k - HIST) * stride + c;
+            nb[k] = rv_conv_raw8(p);
+            nx[k] = rv_conv_raw8(p + 2 * hidden);
+        }
+    }
+    float win[H1][8];
+#pragma unroll
+    for (int k = 0; k < HIST; ++k) {
+        if (t0 - HIST + k >= 0) {
+            bx_of(wb[k], wx[k], win[k]);
+        } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) win[k][i] = old[k][i];
         }
     }
-    const int t1 = min(t0 + RV_CONV_WIDE_CHUNK, qlen);
-    for (int tb = t0; tb < t1; tb += ROWS) {
-        // every row of this part of the chunk is requested before the first is used (a row past
-        // the portion's end reads the last valid row again and is not used)
-        Raw rb[ROWS], rc[ROWS], rx[ROWS];
+    for (int tb = 0;;) {
 #pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-            const T* p = proj + (size_t)(q0 + min(tb + j, t1 - 1)) * stride + c;
-            rb[j] = rv_conv_raw8(p);
-            rc[j] = rv_conv_raw8(p + hidden);
-            rx[j] = rv_conv_raw8(p + 2 * hidden);
-        }
-#pragma unroll
-        for (int j = 0; j < ROWS; ++j) {
-            if (tb + j < t1) {
+        for (int j = 0; j < R; ++j) {
+            if (tb + j <= last) {
                 float bx[8], gate_c[8], res[8];
                 bx_of(rb[j], rx[j], bx);
                 rv_conv_unpack8(rc[j], gate_c);
@@ -384,32 +422,28 @@ __global__ void __launch_bounds__(128) short_conv_wide_kernel(
                     acc += flat[i * TAPS + HIST] * bx[i];
                     res[i] = (gate_c[i] + bc[i]) * (acc + cb[i]);
                 }
-                rv_conv_store8(out + (size_t)(q0 + tb + j) * hidden + c, res);
+                rv_conv_store8(out + (size_t)(q0 + t0 + tb + j) * hidden + c, res);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
 #pragma unroll
                     for (int k = 0; k + 1 < HIST; ++k) win[k][i] = win[k + 1][i];
-                    if (HIST > 0) win[HIST > 0 ? HIST - 1 : 0][i] = bx[i];
+                    if (HIST > 0) win[H1 - 1][i] = bx[i];
                 }
             }
         }
+        tb += R;
+        if (!LOOP || tb > last) break;
+        request(tb);
     }
-    if (t0 == 0 && st && HIST > 0) {
+    if (moves) {
 #pragma unroll
         for (int k = 0; k < HIST; ++k) {
-            const int w = qlen + k;                    // window row of the new state's row k
             float v[8];
+            if (ends_here) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = 0.f;
-            if (w >= HIST) {
-                bx_at(w - HIST, v);
-            } else {
-#pragma unroll
-                for (int kk = 0; kk < HIST; ++kk)
-                    if (kk == w) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] = old[kk][i];
-                    }
+                for (int i = 0; i < 8; ++i) v[i] = win[k][i];
+            } else {                                   // more than R >= 2 tokens: as many as the window's at least
+                bx_of(nb[k], nx[k], v);
             }
             float* sp = st + (size_t)k * hidden;
             *(float4*)sp = make_float4(v[0], v[1], v[2], v[3]);
@@ -418,29 +452,29 @@ __global__ void __launch_bounds__(128) short_conv_wide_kernel(
     }
 }
 
-template <typename T>
-static void short_conv_wide_launch(dim3 grid, cudaStream_t stream, const void* proj, const float* filter,
+template <typename T, int R, bool LOOP>
+static void short_conv_rows_launch(dim3 grid, cudaStream_t stream, const void* proj, const float* filter,
                                    const float* in_bias, const float* conv_bias, float* state,
                                    const int* q_start, const int* state_slot, const int* start_pos,
-                                   void* out, int hidden, int taps) {
-#define RV_CONV_WIDE_CASE(N)                                                                     \
+                                   void* out, int hidden, int taps, int n_reqs, int rounds) {
+#define RV_CONV_ROWS_CASE(N)                                                                     \
     case N:                                                                                      \
-        rv_launch(short_conv_wide_kernel<T, N>, grid, dim3(128), 0, stream, (const T*)proj, filter, \
-                  in_bias, conv_bias, state, q_start, state_slot, start_pos, (T*)out, hidden);   \
+        rv_launch(short_conv_rows_kernel<T, N, R, LOOP>, grid, dim3(128), 0, stream, (const T*)proj, filter, \
+                  in_bias, conv_bias, state, q_start, state_slot, start_pos, (T*)out, hidden, n_reqs, rounds); \
         break;
     switch (taps) {
-        RV_CONV_WIDE_CASE(1)
-        RV_CONV_WIDE_CASE(2)
-        RV_CONV_WIDE_CASE(3)
-        RV_CONV_WIDE_CASE(4)
+        RV_CONV_ROWS_CASE(1)
+        RV_CONV_ROWS_CASE(2)
+        RV_CONV_ROWS_CASE(3)
+        RV_CONV_ROWS_CASE(4)
     }
-#undef RV_CONV_WIDE_CASE
+#undef RV_CONV_ROWS_CASE
 }
 
 extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, const float* in_bias,
                              const float* conv_bias, float* state, const int* q_start,
                              const int* state_slot, const int* start_pos, void* out, int n_reqs,
-                             int max_q_len, int hidden, int taps, void* stream) {
+                             int n_tokens, int max_q_len, int hidden, int taps, void* stream) {
     if (n_reqs == 0) return 0;
     if (n_reqs < 0 || hidden <= 0 || max_q_len <= 0) RV_FAIL("short_conv: bad sizes");
     if (taps < 1 || taps > RV_CONV_MAX_TAPS)
@@ -452,22 +486,32 @@ extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, c
                          (!state || (uintptr_t)state % 16 == 0) &&
                          (!in_bias || (uintptr_t)in_bias % 16 == 0) &&
                          (!conv_bias || (uintptr_t)conv_bias % 16 == 0);
-    // long portions: the wide kernel (RVLLM_CONV_WIDE_FROM: portions of at least this many tokens)
-    static const int wide_from = [] {
+    // Portions: the kernel that requests its rows at once, with as few of them a thread as leave the chip full.
+    // Us, 3 taps: 543 bfloat16 tokens of 1,024 channels with 2 / 4 / 8 tokens a thread 3.29 / 3.26 / 3.40, 108 2.45 /
+    // 2.80 / 3.16, 600 of 2,048 channels 5.78 / 4.94 / 5.32, 2,000 of 1,536 10.8 / 8.5 / 9.0 and 8.9 in two rounds of 8;
+    // 131 float32 tokens of 1,536 2.90 / 3.26, 2,048 of 2,048 17.1 / 13.7, 12.4 in four rounds of 4 (a thread reads the
+    // window before its tokens once more, so long rows are better read in longer pieces).
+    static const int rows_from = [] {
         const char* e = getenv("RVLLM_CONV_WIDE_FROM");
-        return e && *e ? atoi(e) : 64;
+        return e && *e ? atoi(e) : 2;
     }();
-    if (taps <= RV_CONV_VEC_TAPS && hidden % 8 == 0 && aligned && max_q_len >= wide_from &&
+    if (taps <= RV_CONV_VEC_TAPS && hidden % 8 == 0 && aligned && max_q_len >= rows_from && n_tokens > 0 &&
         (uintptr_t)filter % 16 == 0) {
-        const int wchunks = (max_q_len + RV_CONV_WIDE_CHUNK - 1) / RV_CONV_WIDE_CHUNK;
-        if (wchunks > 65535) RV_FAIL("short_conv: batch too large for one launch");
-        dim3 wgrid((hidden / 8 + 127) / 128, n_reqs, wchunks);
-        RV_DISPATCH_DTYPE(dtype, "short_conv",
-                          (short_conv_wide_launch<T>(wgrid, (cudaStream_t)stream, proj, filter, in_bias,
-                                                     conv_bias, state, q_start, state_slot, start_pos,
-                                                     out, hidden, taps)));
-        RV_CHECK_LAUNCH("short_conv");
-        return 0;
+        const int wide = (hidden / 8 + 127) / 128, sms = rv_sm_count();
+        auto pieces = [&](int r) { return (long long)n_tokens / r + n_reqs; };    // as many as there may be
+        const bool half = dtype == RV_DTYPE_BF16, in_rounds = pieces(16) * wide >= (half ? 2 : 1) * sms;
+        const int r = in_rounds ? (half ? 8 : 4) : pieces(4) * wide >= sms ? 4 : 2;
+        const int rounds = in_rounds ? 16 / r : 1;
+        if (pieces(r * rounds) <= 65535) {
+            dim3 rgrid(wide, (unsigned)pieces(r * rounds));
+            RV_DISPATCH_DTYPE(dtype, "short_conv",
+                (in_rounds ? short_conv_rows_launch<T, sizeof(T) == 2 ? 8 : 4, true>
+                 : r == 4 ? short_conv_rows_launch<T, 4, false> : short_conv_rows_launch<T, 2, false>)(
+                    rgrid, (cudaStream_t)stream, proj, filter, in_bias, conv_bias, state, q_start, state_slot,
+                    start_pos, out, hidden, taps, n_reqs, rounds));
+            RV_CHECK_LAUNCH("short_conv");
+            return 0;
+        }
     }
     if (taps <= RV_CONV_VEC_TAPS && hidden % 4 == 0 && aligned) {
         dim3 vgrid((hidden / 4 + 127) / 128, n_reqs, chunks);

@@ -829,7 +829,7 @@ class CudaOps:
         self._check(self.lib.rv_short_conv(
             _ptr(proj), _code(proj.dtype), _ptr(filt), _ptr(in_bias), _ptr(conv_bias),
             _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), _ptr(ctx.start_pos), _ptr(out),
-            c_int(ctx.n_reqs), c_int(ctx.max_q_len), c_int(hidden), c_int(taps),
+            c_int(ctx.n_reqs), c_int(proj.shape[0]), c_int(ctx.max_q_len), c_int(hidden), c_int(taps),
             self._stream()), "short_conv")
 
     # ---- SwiGLU ----------------------------------------------------------------------

@@ -446,6 +446,34 @@ def test_short_conv(ops, dtype, taps, bias):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("taps,rest", [(3, 2600), (4, 2600), (2, 700), (4, 700)])
+def test_short_conv_pieces(ops, dtype, taps, rest):
+    """Pieces of 16 tokens in rounds (2,600 tokens of 1,032 channels) and of 4 at once (700), for more requests than
+    are looked up at a time and portions around a piece's and a window's length."""
+    g = torch.Generator().manual_seed(19)
+    hidden = 1032
+    q_lens = [1] * 25 + [2, 3, 4, 5, 8, 9, 15, 16, 17, 31, 33, rest, 16, 1]
+    n, R = sum(q_lens), len(q_lens)
+    start = [(0, 5, 1)[i % 3] for i in range(R)]
+    slots = [i if i % 7 else -1 for i in range(R)]
+    proj = rnd((n, 3 * hidden), dtype, g)
+    filt = rnd((hidden, taps), torch.float32, g, 0.5)
+    state = rnd((R, taps - 1, hidden), torch.float32, g)
+    q_start = [0]
+    for ql in q_lens:
+        q_start.append(q_start[-1] + ql)
+    ctx = SimpleNamespace(n_reqs=R, max_q_len=max(q_lens), q_start=torch.tensor(q_start, dtype=torch.int32),
+                          state_slot=torch.tensor(slots, dtype=torch.int32),
+                          start_pos=torch.tensor(start, dtype=torch.int32))
+    ref, ref_state = torch.empty(n, hidden, dtype=dtype), state.clone()
+    PlainOps().short_conv(proj, filt, None, None, ref_state, ctx, ref)
+    out, d_state = torch.full((n, hidden), float("nan"), dtype=dtype, device="cuda"), state.cuda()
+    ops.short_conv(proj.cuda(), filt.cuda(), None, None, d_state, to_cuda(ctx), out)
+    assert torch.allclose(out.cpu().float(), ref.float(), **tol(dtype))
+    assert torch.allclose(d_state.cpu(), ref_state, atol=1e-6, rtol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("taps", [3, 4])
 def test_short_conv_long_portion_equals_short_portions(ops, dtype, taps):
     """A portion of 150 tokens (the kernel for long portions: eight channels a thread, rows
