@@ -303,7 +303,9 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
     int hidden, int n_reqs, int rounds) {
     typedef typename RvRaw8<T>::type Raw;
     constexpr int HIST = TAPS - 1, H1 = HIST > 0 ? HIST : 1;
-    static_assert(R >= 2 && HIST <= R + 1, "a portion that one thread does not end has as many rows as the window");
+    // only a portion's first piece may look at the state, which its thread overwrites; and a portion that one
+    // thread does not end has as many rows as the window
+    static_assert(HIST <= R, "a piece is as long as the window before the next");
     rv_pdl_launch_dependents();
     // the request of this block's tokens: pieces of R tokens a round, request after request
     const int piece = LOOP ? R * rounds : R;
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
             if (ends_here) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = win[k][i];
-            } else {                                   // more than R >= 2 tokens: as many as the window's at least
+            } else {                                   // more tokens than a piece: as many as the window's at least
                 bx_of(nb[k], nx[k], v);
             }
             float* sp = st + (size_t)k * hidden;
@@ -459,7 +461,7 @@ static void short_conv_rows_launch(dim3 grid, cudaStream_t stream, const void* p
                                    void* out, int hidden, int taps, int n_reqs, int rounds) {
 #define RV_CONV_ROWS_CASE(N)                                                                     \
     case N:                                                                                      \
-        rv_launch(short_conv_rows_kernel<T, N, R, LOOP>, grid, dim3(128), 0, stream, (const T*)proj, filter, \
+        rv_launch(short_conv_rows_kernel<T, N, (N - 1 <= R ? R : 4), LOOP>, grid, dim3(128), 0, stream, (const T*)proj, filter, \
                   in_bias, conv_bias, state, q_start, state_slot, start_pos, (T*)out, hidden, n_reqs, rounds); \
         break;
     switch (taps) {
@@ -488,8 +490,8 @@ extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, c
                          (!conv_bias || (uintptr_t)conv_bias % 16 == 0);
     // Portions: the kernel that requests its rows at once, with as few of them a thread as leave the chip full.
     // Us, 3 taps: 543 bfloat16 tokens of 1,024 channels with 2 / 4 / 8 tokens a thread 3.29 / 3.26 / 3.40, 108 2.45 /
-    // 2.80 / 3.16, 600 of 2,048 channels 5.78 / 4.94 / 5.32, 2,000 of 1,536 10.8 / 8.5 / 9.0 and 8.9 in two rounds of 8;
-    // 131 float32 tokens of 1,536 2.90 / 3.26, 2,048 of 2,048 17.1 / 13.7, 12.4 in four rounds of 4 (a thread reads the
+    // 2.80 / 3.16, 600 of 2,048 channels 5.78 / 4.94 / 5.32, 2,000 of 1,536 10.8 / 8.5 / 9.0 and 8.9 in two rounds of 8
+    // (no fewer than the window has: two only up to 3 taps.)  131 float32 tokens of 1,536 2.90 / 3.26, 2,048 of 2,048 17.1 / 13.7, 12.4 in four rounds of 4 (a thread reads the
     // window before its tokens once more, so long rows are better read in longer pieces).
     static const int rows_from = [] {
         const char* e = getenv("RVLLM_CONV_WIDE_FROM");
@@ -500,7 +502,7 @@ extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, c
         const int wide = (hidden / 8 + 127) / 128, sms = rv_sm_count();
         auto pieces = [&](int r) { return (long long)n_tokens / r + n_reqs; };    // as many as there may be
         const bool half = dtype == RV_DTYPE_BF16, in_rounds = pieces(16) * wide >= (half ? 2 : 1) * sms;
-        const int r = in_rounds ? (half ? 8 : 4) : pieces(4) * wide >= sms ? 4 : 2;
+        const int r = in_rounds ? (half ? 8 : 4) : pieces(4) * wide >= sms || taps > 3 ? 4 : 2;
         const int rounds = in_rounds ? 16 / r : 1;
         if (pieces(r * rounds) <= 65535) {
             dim3 rgrid(wide, (unsigned)pieces(r * rounds));

@@ -513,6 +513,34 @@ def test_short_conv_long_portion_equals_short_portions(ops, dtype, taps):
     assert torch.allclose(whole_state.cpu(), ref_state, atol=1e-6, rtol=1e-6)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("taps", [2, 3, 4])
+def test_short_conv_state_of_short_portions(ops, dtype, taps):
+    """Many portions of one to five tokens over four steps: a piece of a portion must not see the state that another
+    piece has moved on (a piece shorter than the window would, now and then)."""
+    g = torch.Generator().manual_seed(23)
+    hidden, R = 2048, 60
+    filt = rnd((hidden, taps), torch.float32, g, 0.5)
+    ref_state = rnd((R, taps - 1, hidden), torch.float32, g)
+    state = ref_state.cuda()
+    for step in range(4):
+        q_lens = [1 + (i * 7 + step * 3) % 5 for i in range(R)]
+        q_start = [0]
+        for ql in q_lens:
+            q_start.append(q_start[-1] + ql)
+        n = q_start[-1]
+        ctx = SimpleNamespace(n_reqs=R, max_q_len=max(q_lens), q_start=torch.tensor(q_start, dtype=torch.int32),
+                              state_slot=torch.arange(R, dtype=torch.int32),
+                              start_pos=torch.full((R,), 9, dtype=torch.int32))
+        proj = rnd((n, 3 * hidden), dtype, g)
+        ref = torch.empty(n, hidden, dtype=dtype)
+        PlainOps().short_conv(proj, filt, None, None, ref_state, ctx, ref)
+        out = torch.empty(n, hidden, dtype=dtype, device="cuda")
+        ops.short_conv(proj.cuda(), filt.cuda(), None, None, state, to_cuda(ctx), out)
+        assert torch.allclose(out.cpu().float(), ref.float(), **tol(dtype))
+        assert torch.allclose(state.cpu(), ref_state, atol=1e-5, rtol=1e-5)
+
+
 def test_argmax_first_maximum_and_nan(ops):
     x = torch.randn(5, 1003)
     x[0, 17] = x[0, 900] = 9.0                 # tie: the first wins
