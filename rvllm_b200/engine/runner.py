@@ -17,6 +17,7 @@ from typing import Dict, Hashable, List, Optional, Sequence, Tuple
 
 import gc
 import os
+import threading
 import weakref
 
 import torch
@@ -373,8 +374,8 @@ class ModelRunner:
         return logits[torch.tensor(rows, device=logits.device, dtype=torch.long)]
 
 
-def _capture(graph, fn, pool=None):
-    """Capture `fn` into `graph`.  Python's cyclic garbage collector must not run meanwhile:
+def _capture(graph, fn, ops, pool=None):
+    """Capture `fn` into `graph`; `ops` knows meanwhile which thread's launches are captured.  Python's cyclic garbage collector must not run meanwhile:
     if it destroyed an older graph or freed device memory during the capture, the capture
     would be invalidated (and a graph destroyed from a destructor aborts the process), so
     garbage is collected before and collection is off during the capture."""
@@ -403,9 +404,11 @@ def _capture(graph, fn, pool=None):
                 graph.capture_begin(pool=pool)
             else:
                 graph.capture_begin()
+            ops.capture_thread = threading.get_ident()
             try:
                 out = fn()
             finally:
+                ops.capture_thread = None
                 graph.capture_end()
         torch.cuda.current_stream().wait_stream(_capture_stream)
         return out
@@ -460,7 +463,8 @@ class _DecodeGraph:
             graph = torch.cuda.CUDAGraph()
             self.capturing = True
             try:
-                self.logits = _capture(graph, lambda: model.forward(ctx, views), self.runner.graph_pool())
+                self.logits = _capture(graph, lambda: model.forward(ctx, views), model.ops,
+                                       self.runner.graph_pool())
             finally:
                 self.capturing = False
             self.graph = graph
@@ -516,7 +520,8 @@ class _MixedGraph:
             graph = torch.cuda.CUDAGraph()
             self.capturing = True
             try:
-                self.logits = _capture(graph, lambda: model.forward(ctx, views), self.runner.graph_pool())
+                self.logits = _capture(graph, lambda: model.forward(ctx, views), model.ops,
+                                       self.runner.graph_pool())
             finally:
                 self.capturing = False
             self.graph = graph
@@ -562,7 +567,7 @@ class _ShapeGraph:
             self.capturing = True
             try:
                 self.logits = _capture(
-                    graph, lambda: runner.model.forward(ctx, runner.cache.views()),
+                    graph, lambda: runner.model.forward(ctx, runner.cache.views()), runner.model.ops,
                     runner.graph_pool())
             finally:
                 self.capturing = False

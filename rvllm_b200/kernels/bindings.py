@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -36,6 +37,8 @@ def _ptr(t):
 
 class CudaOps:
     name = "cuda"
+
+    capture_thread = None               # whose launches the engine is capturing
 
     def __init__(self, verbose_build: bool = True):
         if not torch.cuda.is_available():
@@ -420,7 +423,8 @@ class CudaOps:
                 y = torch.mm(xp, w.t()).to(out_dtype)
             if y.shape[0] != m:
                 y = y[:m]
-            if y.is_cuda and torch.cuda.is_current_stream_capturing():
+            # (a thread's number beside the engine's: asking the driver takes a part of a microsecond)
+            if self.capture_thread is not None and self.capture_thread == threading.get_ident():
                 self.lib.rv_next_launch_whole()
         if bias is not None:
             self.add_bias(y, bias)
