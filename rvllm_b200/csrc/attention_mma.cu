@@ -88,13 +88,15 @@ __device__ __forceinline__ float capped_log2(float s, float cap_arg, float cap_o
 template <bool EXT>
 __device__ __forceinline__ float tile_exp2(float x) { return EXT ? fast_exp2(x) : exp2f(x); }
 
-template <int HD, bool SW = false, bool EXT = false>
+// REST: what bfloat16 leaves of P is multiplied too.  1: by the product's rows 8 .. 15, where the warp has up to
+// eight rows of its own (`lo_b` and the like are not looked at); 2: by a second product, to `rest`.
+template <int HD, bool SW = false, bool EXT = false, int REST = 0>
 __device__ __forceinline__ void attend_tile(const unsigned (&qf)[HD / 16][4], const bf16* kt,
                                             const bf16* vt, int tile_key0, int lane, int lo_a,
                                             int hi_a, int lo_b, int hi_b, float scale_log2,
                                             float& m_a, float& m_b, float& l_a, float& l_b,
                                             float (&o)[RV_VD / 8][4], float cap_arg = 0.f,
-                                            float cap_out = 0.f) {
+                                            float cap_out = 0.f, float (*rest)[4] = nullptr) {
     constexpr int KSTEPS = HD / 16, VD = RV_VD;
     // S = Q K^T for 16 rows x 64 keys
     float s[RV_BN / 8][4];
@@ -153,19 +155,24 @@ __device__ __forceinline__ void attend_tile(const unsigned (&qf)[HD / 16][4], co
             for (int e = 0; e < 2; ++e) {
                 const int key = key0 + i * 8 + e;
                 s[i][e] = (key >= lo_a && key <= hi_a) ? s[i][e] * scale_log2 : -INFINITY;
-                s[i][2 + e] = (key >= lo_b && key <= hi_b) ? s[i][2 + e] * scale_log2 : -INFINITY;
                 mx_a = fmaxf(mx_a, s[i][e]);
-                mx_b = fmaxf(mx_b, s[i][2 + e]);
+                if (REST != 1) {
+                    s[i][2 + e] = (key >= lo_b && key <= hi_b) ? s[i][2 + e] * scale_log2 : -INFINITY;
+                    mx_b = fmaxf(mx_b, s[i][2 + e]);
+                }
             }
         }
     }
     mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1));
     mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
-    mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
-    mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
+    if (REST != 1) {
+        mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1));
+        mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
+    }
     const float mn_a = fmaxf(m_a, mx_a), mn_b = fmaxf(m_b, mx_b);
     const float off_a = mn_a == -INFINITY ? 0.f : mn_a, off_b = mn_b == -INFINITY ? 0.f : mn_b;
-    const float corr_a = tile_exp2<EXT>(m_a - off_a), corr_b = tile_exp2<EXT>(m_b - off_b);   // m = -inf -> 0
+    const float corr_a = tile_exp2<EXT>(m_a - off_a);                                         // m = -inf -> 0
+    const float corr_b = REST == 1 ? corr_a : tile_exp2<EXT>(m_b - off_b);
     m_a = mn_a;
     m_b = mn_b;
     l_a *= corr_a;
@@ -174,21 +181,35 @@ __device__ __forceinline__ void attend_tile(const unsigned (&qf)[HD / 16][4], co
     for (int i = 0; i < VD / 8; ++i) {
         o[i][0] *= corr_a; o[i][1] *= corr_a;
         o[i][2] *= corr_b; o[i][3] *= corr_b;
+        if (REST == 2) {
+            rest[i][0] *= corr_a; rest[i][1] *= corr_a;
+            rest[i][2] *= corr_b; rest[i][3] *= corr_b;
+        }
     }
-    // P = exp2(S - m), rounded to bfloat16 for the second product; the row sum adds the
-    // rounded values, so numerator and denominator see the same numbers
-    unsigned pa[RV_BN / 16][4];
+    // P = exp2(S - m), rounded to bfloat16 for the second product; the row sum adds what is
+    // multiplied (but for some 2^-17 of it), so numerator and denominator see the same numbers
+    unsigned pa[RV_BN / 16][4], pr[REST == 2 ? RV_BN / 16 : 1][4];
 #pragma unroll
     for (int i = 0; i < RV_BN / 8; ++i) {
         const float e0 = tile_exp2<EXT>(s[i][0] - off_a), e1 = tile_exp2<EXT>(s[i][1] - off_a);
-        const float e2 = tile_exp2<EXT>(s[i][2] - off_b), e3 = tile_exp2<EXT>(s[i][3] - off_b);
         const __nv_bfloat162 ra = __floats2bfloat162_rn(e0, e1);
-        const __nv_bfloat162 rb = __floats2bfloat162_rn(e2, e3);
-        const float2 fa = __bfloat1622float2(ra), fb = __bfloat1622float2(rb);
-        l_a += fa.x + fa.y;
-        l_b += fb.x + fb.y;
+        const float2 fa = __bfloat1622float2(ra);
         pa[i >> 1][(i & 1) * 2] = *(const unsigned*)&ra;
+        if (REST == 1) {
+            l_a += e0 + e1;
+            pa[i >> 1][(i & 1) * 2 + 1] = pack_bf16(e0 - fa.x, e1 - fa.y);
+            continue;
+        }
+        const float e2 = tile_exp2<EXT>(s[i][2] - off_b), e3 = tile_exp2<EXT>(s[i][3] - off_b);
+        const __nv_bfloat162 rb = __floats2bfloat162_rn(e2, e3);
+        const float2 fb = __bfloat1622float2(rb);
+        l_a += REST ? e0 + e1 : fa.x + fa.y;
+        l_b += REST ? e2 + e3 : fb.x + fb.y;
         pa[i >> 1][(i & 1) * 2 + 1] = *(const unsigned*)&rb;
+        if (REST == 2) {
+            pr[i >> 1][(i & 1) * 2] = pack_bf16(e0 - fa.x, e1 - fa.y);
+            pr[i >> 1][(i & 1) * 2 + 1] = pack_bf16(e2 - fb.x, e3 - fb.y);
+        }
     }
     // O += P V
 #pragma unroll
@@ -200,6 +221,11 @@ __device__ __forceinline__ void attend_tile(const unsigned (&qf)[HD / 16][4], co
                                                           nd * 2 + (lane >> 4)));
             mma_bf16(o[2 * nd], pa[kk], b[0], b[1]);
             mma_bf16(o[2 * nd + 1], pa[kk], b[2], b[3]);
+            if (REST == 2) {
+                float (&r0)[4] = *(float (*)[4])rest[2 * nd], (&r1)[4] = *(float (*)[4])rest[2 * nd + 1];
+                mma_bf16(r0, pr[kk], b[0], b[1]);
+                mma_bf16(r1, pr[kk], b[2], b[3]);
+            }
         }
     }
 }
@@ -610,6 +636,8 @@ __global__ void __launch_bounds__(NW * 32) paged_attention_decode_mma_kernel(
 // completion counted on an mbarrier of the stage) and walks them with the online softmax; where
 // the run leaves a request, the rows so far go to memory as one of the request's segments, which
 // paged_attention_merge_segments_kernel (attention_simt.cu) puts together in order.
+// A long run's P is rounded against a maximum that few of its keys have made, so what bfloat16 leaves of
+// P is multiplied as well, where up to eight heads share keys by rows of the product that are free.
 // Splits of 128 or 256 keys, dealt out in turns, left some warps twice the others' work, and a replay's also
 // splits without keys.  Us with the merge, 32 / 8 heads, splits / runs: 8 requests of some 2,300 keys 14.2 / 11.6,
 // 31 of 950 20.7 / 16.2, 64 of 3,100 80.3 / 68.7 (5.9 TB/s), 8 of 240 7.3 / 4.4.
@@ -885,6 +913,9 @@ paged_attention_decode_stream_kernel(
         float o[HD / 8][4];
 #pragma unroll
         for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+        float rest[HD / 8][4];
+#pragma unroll
+        for (int i = 0; i < HD / 8; ++i) rest[i][0] = rest[i][1] = rest[i][2] = rest[i][3] = 0.f;
         for (int t = m.t_first; t <= m.t_last; ++t) {
             const int s = n_consumed % S;
             if (!st_mbar_wait(&full_bar[w][s], (unsigned)(n_consumed / S) & 1u)) {
@@ -892,13 +923,25 @@ paged_attention_decode_stream_kernel(
                 break;
             }
             const bf16* kt = my_ring + (size_t)s * 2 * TILE;
-            attend_tile<HD, true>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
-                                  scale_log2, m_a, m_b, l_a, l_b, o);
+            if (rows <= 8)
+                attend_tile<HD, true, false, 1>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
+                                                scale_log2, m_a, m_b, l_a, l_b, o);
+            else
+                attend_tile<HD, true, false, 2>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
+                                                scale_log2, m_a, m_b, l_a, l_b, o, 0.f, 0.f, rest);
             __syncwarp();
             ++n_consumed;
             fill();                                 // the freed stage takes the next tile
         }
         if (failed) break;
+        // what was left of P: with up to eight rows in rows 8 .. 15.  (An infinite value's share is no number there.)
+        auto add = [](float a, float b) { return fabsf(b) < INFINITY ? a + b : a; };
+#pragma unroll
+        for (int i = 0; i < HD / 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (rows > 8) o[i][e] = add(o[i][e], rest[i][e]);
+                else if (e < 2) o[i][e] = add(o[i][e], o[i][2 + e]);
         l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
         l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
         l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);

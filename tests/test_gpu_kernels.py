@@ -327,6 +327,36 @@ def test_decode_stream_runs(ops, reqs, nh, nkv, ps, window):
     assert torch.allclose(out.cpu().float(), ref.float(), atol=2e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("nh,nkv", [(1, 1), (32, 8), (8, 1), (12, 1), (20, 1)])
+def test_decode_stream_multiplies_all_of_p(ops, nh, nkv):
+    """The weights of long runs of keys are multiplied in two bfloat16 parts (2^-17 of each is left out), one query
+    head and eight of them with the rest in rows that are free, twelve and sixteen with a product of its own, and
+    four heads beyond sixteen: rows of 32 bits against float64.  Powers of two, sums and the products of up to 2,900 keys
+    add some 2^-20.  In one part it is 2^-10.  An infinite value stays one."""
+    lens, hd = [2900, 2037, 64, 1, 517], 64
+    g = torch.Generator().manual_seed(nh)
+    q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, [1] * len(lens), lens, nh, nkv, hd, 16)
+    page, slot = int(group.block_table[1, 31]), 5
+    vc[page, slot, 0, 3] = float("inf")
+    out = torch.full((len(lens), nh * hd), float("nan"), device="cuda")
+    d_ctx, d_group = to_cuda(ctx), to_cuda(group)
+    ops.paged_attention_decode_mma(q.cuda(), nh, nkv, hd, kc.cuda(), vc.cuda(), d_group.block_table, d_ctx.q_start,
+                                   d_ctx.ctx_lens, len(lens), max(lens), 16, 0.125, None, out)
+    ops.check_status()
+    vc[page, slot, 0, 3] = 0
+    for r, c in enumerate(lens):
+        at = torch.arange(c)
+        rows = lambda t: t[group.block_table[r].long()[at // 16], at % 16].double()          # noqa: E731
+        k, v = rows(kc), rows(vc)
+        for h in range(nh):
+            p = torch.softmax(k[:, h * nkv // nh] @ q[r, h * hd:(h + 1) * hd].double() * 0.125, 0)
+            got, want = out[r, h * hd:(h + 1) * hd].cpu().double(), p @ v[:, h * nkv // nh]
+            if r == 1 and h * nkv // nh == 0:
+                assert float(got[3]) == float("inf")
+                got[3] = want[3]
+            assert float((got - want).norm() / want.norm()) < 2.0 ** -16, (r, h)
+
+
 EDGE_CASES = [
     # q_len, context, window, page: where the window's first key `lo` of the last (and, for a
     # portion, of the first) query falls
