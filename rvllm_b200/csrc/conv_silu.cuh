@@ -19,12 +19,6 @@ __device__ __forceinline__ void cs_load(const float* p, float (&x)[V]) {
     }
 }
 
-// A quotient that is rounded to bfloat16 need not be correct to the last bit of a float32.
-template <typename T>
-__device__ __forceinline__ float cs_silu(float x) {
-    return sizeof(T) == 4 ? x / (1.f + expf(-x)) : __fdividef(x, 1.f + __expf(-x));
-}
-
 // TAPS 0: any number, `taps`.
 template <typename T, int TAPS, int TT, int V>
 __global__ void __launch_bounds__(128) conv_silu_kernel(
@@ -98,7 +92,7 @@ __global__ void __launch_bounds__(128) conv_silu_kernel(
 #pragma unroll
         for (int e = 0; e < V; ++e) {
             acc[e] += b[e];
-            acc[e] = cs_silu<T>(acc[e]);
+            acc[e] = acc[e] / (1.f + expf(-acc[e]));
         }
         la_store<T, V>(out + (size_t)t * C + c, acc);
     }

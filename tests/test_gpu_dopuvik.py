@@ -516,6 +516,28 @@ def test_state_space_kernels(ops, dtype, sizes):
     assert float((state[4] - 3.0).abs().max()) == 0 and float(state[1].abs().max()) == 0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n", [1, 17])
+def test_state_space_inputs_far_below_zero(ops, dtype, n):
+    """The convolution's silu where its exponential nears float32's end, seen through one token's share of the state:
+    B and x are rounded to bfloat16 (2^-9 of each; they may round the other way: twice that)."""
+    gen = torch.Generator().manual_seed(7)
+    H, dvv, N = 2, 16, 32
+    m, C, t = _ssm(gen, H, dvv, N, 1, 2, 1)
+    inner, at = H * dvv, n // 2
+    t["conv"][:], t["conv.b"][:], t["A_log"][:] = np.array([0.0, 1.0]), 0.0, -40.0
+    rows = rnd(gen, torch.float32, n, inner + C + H).numpy()
+    rows[:, inner:2 * inner] = 0.0
+    rows[at, inner:2 * inner] = np.float32(1e36)
+    rows[at, 2 * inner:2 * inner + N] = np.linspace(-88.0, -60.0, N).astype(np.float32)
+    state, conv = torch.zeros(1, H * N * dvv, device="cuda"), torch.zeros(1, 1, C, device="cuda")
+    ctx, _ = step_context([(n, 0)])
+    _ssm_run(ops, m, C, t, state, conv, dtype)(rows, ctx)
+    _, S = _ssm_plain(m, C, t, rows, dtype == torch.bfloat16)
+    want = torch.as_tensor(S.reshape(-1))
+    assert float(((state[0].cpu().double() - want) / want).abs().max()) < (2.0 ** -16 if dtype == torch.float32 else 2.0 ** -7)
+
+
 @pytest.mark.parametrize("dtype,sizes", [(torch.float32, (3, 16, 24, 1, 4, 1)), (torch.bfloat16, (3, 32, 48, 1, 4, 1)),
                                          (torch.bfloat16, (3, 12, 20, 3, 2, 1))])
 def test_state_space_decays_from_nothing_to_one(ops, dtype, sizes):
