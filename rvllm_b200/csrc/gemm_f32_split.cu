@@ -1,35 +1,36 @@
 // y = x . w^T in float32 on the 5th-generation tensor cores: x [M, K], w [N, K], y [M, N].
 //
-// A float32 value is the sum of two TF32 values and at most one bit: x = h + l, h the nearest value
-// with 11 bits of mantissa, l = x - h exactly, of which the product reads 11 bits.  A product of two such
-// sums is l h' + h l' + h h' (l l' is below 2^-24 of it): three tcgen05.mma of kind::tf32, whose
-// products are exact and whose sums are float32.  The tensor core cuts off what lies below the
+// A float32 value is the sum of three bfloat16 values, its bits 1 - 8, 9 - 16 and 17 - 24: x = h + m + l exactly.
+// A product of two such sums is formed as eight of the nine products of their parts (l l' is below 2^-30 of it):
+// tcgen05.mma of kind::f16, whose products are exact and whose sums are float32.  Where one
+// operand's value is a power of two the result is the other's.  The tensor core cuts off what lies below the
 // accumulator's last bit, so a sum is not left there for long: a chunk is 32 of K, its small
 // products first, and then goes to float32 registers, which add the chunks with round-to-nearest.
+// (Two TF32 parts and three products hold 22 bits and leave out 2^-22 of a product.)
 //
-//   split    x -> parts [row tile][chunk][h, l][rows][32], each [rows][32] as the swizzled image that a
+//   split    x -> parts [row tile][chunk][h, m, l][rows][32], each [rows][32] as the swizzled image that a
 //            product's operand has in shared memory, so that a chunk is one contiguous copy
 //   product  block per (128 columns, up to 160 rows, share of K).  128 rows of w are the M side, so an
 //            output column is a TMEM lane; the rows of x are the N side.
 //     warps 0 - 3    w: 32 rows each by cp.async into a ring of its own, split in registers, to TMEM
-//                    (the A operand; two chunks): shared memory, which the B operand's reads keep
+//                    (the A operand; three chunks): shared memory, which the B operand's reads keep
 //                    busy, sees w once in and once out
 //     warps 4 - 11   the accumulators (two chunks) to registers, and at the end the outputs
-//     warp 12        issues the twelve products of a chunk
+//     warp 12        issues the sixteen products of a chunk
 //     warp 13        copies the chunks of x
 //   K is shared by a cluster of up to eight blocks, which leave their tiles in shared memory and add
 //   them in rank order.
 //
-// Bound by the tensor cores' reads of shared memory and by the pipeline's meetings with many rows (128 x 13824 x
-// 1536: 0.8 us a chunk, of which the twelve products' own time is 0.45), by the matrix's bytes with few.  us at N x K, against
-// the library's kernels on the FP32 cores or gemm_f32.cu's, whichever was the faster: 131 rows 4608 x 1536 72 -> 34,
-// 1536 x 1536 32 -> 14, 13824 x 1536 196 -> 46, 1536 x 6912 128 -> 32; 1 row 18 -> 14, 15 -> 9, 31 -> 27, 53 -> 19; 2,048
-// rows 495 -> 166, 210 -> 84, 1,381 -> 402, 904 -> 258.  Relative error against 64 bits there: 1.5 - 2.7e-7 (the library's
-// 3e-7 - 1.5e-6, gemm_f32.cu's 1.9 - 5e-7).
+// Bound by the tensor cores' reads of shared memory and by the pipeline's meetings with many rows (131 x 13824 x
+// 1536: 0.9 us a chunk, of which the sixteen products' own time is some 0.55), by the matrix's bytes with few.  us at N x K,
+// a call with its launches, L2 flushed, against the library's kernels on the FP32 cores or gemm_f32.cu's, whichever
+// was the faster: 131 rows 4608 x 1536 78 -> 42, 1536 x 1536 37 -> 20, 13824 x 1536 166 -> 56, 1536 x 6912 131 -> 40; 16 rows
+// 25 -> 24, 18 -> 15, 45 -> 32, 55 -> 26; 2,048 rows 498 -> 202, 215 -> 103, 1,387 -> 501, 906 -> 327.  Relative error against
+// 64 bits there: 0.9 - 2.5e-7 (the library's 1.4e-7 - 1.5e-6, gemm_f32.cu's 1.9e-7 - 1.1e-6).
 //
-// A sum that is not finite is formed again from x and w by float32 multiply-adds: parts of an infinite
-// value are not numbers, and a part may round up to infinity where the value does not.  Operands below
-// 2^-102 lose the bits of l that fall below float32's normal range.
+// A sum that is not finite is formed again from x and w by float32 multiply-adds (parts of an infinite value are
+// not numbers), and one below 2^-100, whose small products leave float32's range.  Operands below 2^-110
+// lose the bits of l that bfloat16 does not have there; that is seen beside operands above 2^10 only.
 //
 // Every wait is bounded; one that runs out records 41 - 45 in `status` and the block ends.
 // Plain reference: tests/plain_ops.py linear.
@@ -40,29 +41,39 @@
 #define FS_BN 128           // rows of w in a block
 #define FS_WS 5             // chunks of w in a ring
 #define FS_XS 3             // chunks of x in a ring, and of w in TMEM
+#define FS_PARTS 3
 #define FS_MAX_ROWS 160     // of x in a block: with three chunks of w and two accumulators 512 columns of TMEM
 #define FS_THREADS 448
 
-__device__ __forceinline__ float fs_high(float x) {
-    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+// Two neighbours' parts, the first in the lower half.
+__device__ __forceinline__ void fs_parts(float a, float b, unsigned (&p)[FS_PARTS]) {
+#pragma unroll
+    for (int i = 0; i < FS_PARTS; ++i) {
+        const unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
+        p[i] = __byte_perm(ua, ub, 0x7632);
+        a -= __uint_as_float(ua & 0xffff0000u);
+        b -= __uint_as_float(ub & 0xffff0000u);
+    }
 }
 __device__ __forceinline__ void fs_mma(unsigned tmem_d, unsigned tmem_a, unsigned long long b_desc, unsigned idesc,
                                        unsigned accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void fs_tmem_store_32(unsigned taddr, const float (&v)[32]) {
+// Descriptor of a K-major tile with 64-byte swizzle: rows of 64 bytes, eight rows 512 bytes on, layout type 4.
+__device__ __forceinline__ unsigned long long fs_desc(const void* tile) {
+    const unsigned long long addr = (smem_u32(tile) & 0x3FFFFu) >> 4;
+    return addr | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
+__device__ __forceinline__ void fs_tmem_store_16(unsigned taddr, const unsigned (&v)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-        "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]),
-          "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]),
-          "f"(v[16]), "f"(v[17]), "f"(v[18]), "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]),
-          "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]), "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31])
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
 __device__ __forceinline__ void fs_tmem_load_8(unsigned taddr, unsigned* r) {
@@ -84,14 +95,15 @@ __device__ __forceinline__ float fs_cluster_load(const float* local, unsigned ra
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
     return v;
 }
-// The sum as it is, where its parts gave none.
+// The sum as it is, where its parts did not give it.
 __device__ __noinline__ float fs_plain(const float* x, const float* w, int K) {
     float s = 0.f;
     for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
     return s;
 }
 __device__ __forceinline__ float fs_checked(float v, const float* x, const float* w, int m, int n, int K) {
-    return fabsf(v) < INFINITY ? v : fs_plain(x + (size_t)m * K, w + (size_t)n * K, K);
+    const float a = fabsf(v);
+    return v == 0.f || (a >= 7.8886091e-31f && a < INFINITY) ? v : fs_plain(x + (size_t)m * K, w + (size_t)n * K, K);
 }
 
 // Block (chunk, row tile).  The next kernel, the product, may begin when all blocks here are past their
@@ -101,15 +113,20 @@ __global__ void __launch_bounds__(256) fs_split_kernel(const float* __restrict__
     rv_pdl_wait();
     rv_pdl_launch_dependents();
     const int kb = blockIdx.x, m0 = blockIdx.y * rows;
-    float* to = parts + ((size_t)blockIdx.y * gridDim.x + kb) * 2 * rows * FS_BK;
-    for (int i = threadIdx.x; i < rows * (FS_BK / 4); i += 256) {
-        const int r = i >> 3, c = i & 7, k = kb * FS_BK + c * 4;
-        const bool there = m0 + r < M && k < K;
-        const float4 v = there ? *(const float4*)(x + (size_t)(m0 + r) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 h = make_float4(fs_high(v.x), fs_high(v.y), fs_high(v.z), fs_high(v.w));
-        const int at = r * FS_BK + ((c ^ (r & 7)) << 2);
-        *(float4*)(to + at) = h;
-        *(float4*)(to + rows * FS_BK + at) = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+    unsigned char* to = (unsigned char*)parts + ((size_t)blockIdx.y * gridDim.x + kb) * FS_PARTS * rows * FS_BK * 2;
+    for (int i = threadIdx.x; i < rows * (FS_BK / 8); i += 256) {
+        const int r = i >> 2, c = i & 3, k = kb * FS_BK + c * 8;
+        const float* from = x + (size_t)(m0 + r) * K + k;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a = m0 + r < M && k < K ? *(const float4*)from : zero, b = m0 + r < M && k + 4 < K ? *(const float4*)(from + 4) : zero;
+        unsigned p[4][FS_PARTS];
+        fs_parts(a.x, a.y, p[0]);
+        fs_parts(a.z, a.w, p[1]);
+        fs_parts(b.x, b.y, p[2]);
+        fs_parts(b.z, b.w, p[3]);
+        unsigned char* at = to + r * FS_BK * 2 + ((c ^ ((r >> 1) & 3)) << 4);
+#pragma unroll
+        for (int s = 0; s < FS_PARTS; ++s) *(uint4*)(at + (size_t)s * rows * FS_BK * 2) = make_uint4(p[0][s], p[1][s], p[2][s], p[3][s]);
     }
 }
 
@@ -120,8 +137,8 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
     int* __restrict__ status, int M, int N, int K) {
     constexpr int XS = FS_XS;
     constexpr int CT = NT / 2;                            // columns of an accumulator that a thread holds
-    constexpr unsigned X_PART = NT * FS_BK * 4, X_STAGE = 2 * X_PART, W_STAGE = FS_BN * FS_BK * 4;
-    constexpr unsigned A_COLS = 2 * FS_BK, COLS = XS * A_COLS + 2 * NT <= 256 ? 256 : 512;
+    constexpr unsigned X_PART = NT * FS_BK * 2, X_STAGE = FS_PARTS * X_PART, W_STAGE = FS_BN * FS_BK * 4;
+    constexpr unsigned A_PART = FS_BK / 2, A_COLS = FS_PARTS * A_PART, COLS = XS * A_COLS + 2 * NT <= 256 ? 256 : 512;
     static_assert(XS * A_COLS + 2 * NT <= 512, "TMEM holds the chunks and the accumulators");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -170,7 +187,7 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
     for (int j = 0; j < CT; ++j) acc[j] = 0.f;
 
     if (warp < 4) {
-        // ---- w to TMEM in two parts -----------------------------------------------------------
+        // ---- w to TMEM in three parts ---------------------------------------------------------
         unsigned char* ring = ws + warp * (W_STAGE / 4);
         const int first = n0 + warp * 32;
         auto get = [&](int i) {
@@ -193,16 +210,18 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
             __syncwarp();                                 // chunk i is here, chunk i - 1 has been read
             if (i + FS_WS - 1 < n) get(i + FS_WS - 1);
             cp_async_commit();
-            float h[FS_BK], l[FS_BK];
+            unsigned p[FS_PARTS][A_PART];
             const unsigned char* row = ring + (i % FS_WS) * W_STAGE + lane * 128;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const float4 v = *(const float4*)(row + ((c ^ (lane & 7)) << 4));
-                const float in[4] = {v.x, v.y, v.z, v.w};
+                unsigned a[FS_PARTS], e[FS_PARTS];
+                fs_parts(v.x, v.y, a);
+                fs_parts(v.z, v.w, e);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    h[4 * c + e] = fs_high(in[e]);
-                    l[4 * c + e] = in[e] - h[4 * c + e];
+                for (int s = 0; s < FS_PARTS; ++s) {
+                    p[s][2 * c] = a[s];
+                    p[s][2 * c + 1] = e[s];
                 }
             }
             const int b = i % XS;
@@ -214,8 +233,8 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const unsigned to = tmem + ((unsigned)(warp * 32) << 16) + b * A_COLS;
-            fs_tmem_store_32(to, h);
-            fs_tmem_store_32(to + FS_BK, l);
+#pragma unroll
+            for (int s = 0; s < FS_PARTS; ++s) fs_tmem_store_16(to + s * A_PART, p[s]);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -254,7 +273,7 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
     } else if (warp == 12) {
         // ---- the products: the warp walks the chunks together, one lane issues -----------------------
         rv_pdl_wait();                                    // the bounded waits start when the kernel before is done
-        const unsigned idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(NT >> 3) << 17) |
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NT >> 3) << 17) |
                                ((unsigned)(FS_BN >> 4) << 24);
         int issued = 0;
         for (int i = 0; i < n; ++i) {
@@ -269,13 +288,18 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (rv_elect()) {
                 const unsigned d = tmem_d + b * NT, a = tmem + s * A_COLS;
-                const unsigned long long bh = smem_desc_sw128(xs + s * X_STAGE), bl = smem_desc_sw128(xs + s * X_STAGE + X_PART);
+                const unsigned long long x0 = fs_desc(xs + s * X_STAGE);
+                // parts of w and of x whose numbers add up to 3, 2, 1 and 0: the smallest products first
 #pragma unroll
-                for (int k = 0; k < FS_BK / 8; ++k) fs_mma(d, a + FS_BK + 8 * k, bh + 2 * k, idesc, k != 0);
+                for (int sum = 3; sum >= 0; --sum)
 #pragma unroll
-                for (int k = 0; k < FS_BK / 8; ++k) fs_mma(d, a + 8 * k, bl + 2 * k, idesc, 1);
+                    for (int p = 0; p < FS_PARTS; ++p)
+                        if (sum - p >= 0 && sum - p < FS_PARTS) {
 #pragma unroll
-                for (int k = 0; k < FS_BK / 8; ++k) fs_mma(d, a + 8 * k, bh + 2 * k, idesc, 1);
+                            for (int k = 0; k < FS_BK / 16; ++k)
+                                fs_mma(d, a + p * A_PART + 8 * k, x0 + (sum - p) * (X_PART >> 4) + 2 * k, idesc,
+                                       sum != 3 || p != 1 || k != 0);
+                        }
                 tcgen05_commit(&empty[s]);
                 tcgen05_commit(&d_full[b]);
             }
@@ -293,7 +317,7 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
     } else if (lane == 0) {
         // ---- the chunks of x ---------------------------------------------------------------------------
         rv_pdl_wait();
-        const float* from = parts + ((size_t)blockIdx.x * chunks + c0) * (X_STAGE / 4);
+        const unsigned char* from = (const unsigned char*)parts + ((size_t)blockIdx.x * chunks + c0) * X_STAGE;
         int issued = 0;
         for (int i = 0; i < n; ++i) {
             const int s = i % XS;
@@ -302,7 +326,7 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
                 break;
             }
             mbar_expect_tx(&full[s], X_STAGE);
-            bulk_load_1d(xs + s * X_STAGE, from + (size_t)i * (X_STAGE / 4), X_STAGE, &full[s]);
+            bulk_load_1d(xs + s * X_STAGE, from + (size_t)i * X_STAGE, X_STAGE, &full[s]);
             issued = i + 1;
         }
         for (int i = max(0, issued - XS); i < issued; ++i) {
@@ -353,7 +377,7 @@ __global__ void __launch_bounds__(FS_THREADS, NT <= 32 ? 2 : 1) fs_gemm_kernel(
 
 template <int NT>
 static constexpr size_t fs_smem() {
-    return (size_t)FS_XS * NT * FS_BK * 8 + FS_WS * FS_BN * FS_BK * 4 + 1024;
+    return (size_t)FS_XS * NT * FS_BK * 2 * FS_PARTS + FS_WS * FS_BN * FS_BK * 4 + 1024;
 }
 static_assert(fs_smem<FS_MAX_ROWS>() <= 227 * 1024, "the rings fit shared memory");
 
@@ -405,7 +429,7 @@ static cudaError_t fs_launch(const float* parts, const float* x, const float* w,
 // Rows of x that are split at a time: as few tiles as there can be, and 64 MB of parts at the most.
 struct FsRows { int tiles, rows; };
 static FsRows fs_rows(int M, int K) {
-    const long long tile = (long long)FS_MAX_ROWS * ((K + FS_BK - 1) / FS_BK * FS_BK) * 8;
+    const long long tile = (long long)FS_MAX_ROWS * ((K + FS_BK - 1) / FS_BK * FS_BK) * 2 * FS_PARTS;
     const int most = (int)((64ll << 20) / tile);
     int tiles = (M + FS_MAX_ROWS - 1) / FS_MAX_ROWS;
     const int rows = (((M + tiles - 1) / tiles + 15) & ~15);
@@ -414,7 +438,7 @@ static FsRows fs_rows(int M, int K) {
 extern "C" long long rv_gemm_f32_split_scratch(int M, int K) {
     if (M <= 0 || K <= 0) return 0;
     const FsRows r = fs_rows(M, K);
-    return (long long)r.tiles * r.rows * ((K + FS_BK - 1) / FS_BK) * FS_BK * 2;
+    return (long long)r.tiles * r.rows * ((K + FS_BK - 1) / FS_BK) * FS_BK * FS_PARTS / 2;
 }
 
 // K a multiple of 4, x, w and scratch (rv_gemm_f32_split_scratch floats) on 16-byte boundaries.

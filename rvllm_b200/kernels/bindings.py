@@ -379,7 +379,7 @@ class CudaOps:
         return k % 4 == 0 and k >= 768 and n >= (256 if m <= 32 else 1024)
 
     def _linear_split(self, x, w):
-        """y = x . w^T, float32, as sums of TF32 products (gemm_f32_split.cu)."""
+        """y = x . w^T, float32, as sums of products of bfloat16 parts (gemm_f32_split.cu)."""
         (m, k), n = x.shape, w.shape[0]
         y = torch.empty((m, n), dtype=torch.float32, device=x.device)
         parts = torch.empty(self.lib.rv_gemm_f32_split_scratch(c_int(m), c_int(k)), dtype=torch.float32,

@@ -835,6 +835,35 @@ def test_gemm_f32_split_of_what_is_not_finite(ops, M, N, K):
     assert bool(((y.double() - ref.double()).abs() <= bound)[fin].all())
 
 
+@pytest.mark.parametrize("M,N,K", [(20, 300, 1028), (161, 1024, 800)])
+def test_gemm_f32_split_holds_all_bits(ops, M, N, K):
+    """What float32 multiply-adds give without any rounding is that here too: values beside a power of two, in either
+    operand, and whole numbers whose sums stay below 2^24.  Operands near the ends of float32's range lose no more than
+    others (the bound is `test_gemm_f32_split`'s)."""
+    g = torch.Generator().manual_seed(K)
+    full = lambda *s: (torch.randint(1 << 23, 1 << 24, s, generator=g) * 2.0 ** -23 *           # noqa: E731
+                       (1 - 2 * torch.randint(0, 2, s, generator=g))).float().cuda()
+    x, w = torch.zeros(M, K, device="cuda"), torch.zeros(N, K, device="cuda")
+    at, power = torch.randint(0, K, (M,), generator=g), torch.randint(-20, 20, (M,), generator=g)
+    x[torch.arange(M), at] = (2.0 ** power.double()).float().cuda()
+    wide = full(N, K)
+    assert torch.equal(ops._linear_split(x, wide), wide[:, at].t() * x[torch.arange(M), at][:, None])
+    at = torch.randint(0, K, (N,), generator=g)
+    w[torch.arange(N), at] = 1.0
+    wide = full(M, K)
+    assert torch.equal(ops._linear_split(wide, w), wide[:, at])
+    x = torch.randint(-4095, 4096, (M, K), generator=g).cuda().float()
+    w = torch.randint(-3, 4, (N, K), generator=g).cuda().float()
+    assert torch.equal(ops._linear_split(x, w).double(), x.double() @ w.double().t())
+    for ex, ew in ((-108, 40), (-112, 0), (-60, -60), (-125, 9), (90, 25)):          # (4 K 2^115 is no overflow)
+        x, w = full(M, K) * 2.0 ** ex, full(N, K) * 2.0 ** ew
+        ref = x.double() @ w.double().t()
+        bound = (K / 32 + 64) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+        # (an output below 2^-126 has float32's last place, 2^-149, and so has every multiply-add there)
+        assert bool(((ops._linear_split(x, w).double() - ref).abs() <= bound + K * 2.0 ** -149).all()), (ex, ew)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("M,N,K", [(5, 4608, 1536), (64, 1536, 6912)])
 def test_gemm_f32_of_a_matrix_made_just_before(ops, M, N, K):
     """The matrix may be what the launch before writes: a bfloat16 one is cast for float32 rows, and
