@@ -21,7 +21,7 @@
 //   moe_combine   out[t] = sum_k weights[t, k] * ys[pair_pos[t * top + k]], in the order of k.
 //
 // A pair whose id is E or more (an identity expert) takes no row: its pair_pos is -1, and the sum
-// reads x[t] itself.
+// reads x[t] itself.  Nor does one whose id is negative (-2): it adds nothing.
 //
 // A row's sums depend on its own expert and values only, never on which other rows share its
 // tile, so a token's result does not depend on the batch.  Every wait on an mbarrier is
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(
         int at = 0;
         if (valid && lane == leader) at = atomicAdd(&cnt[e], __popc(same));
         at = __shfl_sync(0xffffffffu, at, leader) + __popc(same & ((1u << lane) - 1u));
-        if (p < P) pair_pos[p] = valid ? at : e >= E ? -1 : 0;
+        if (p < P) pair_pos[p] = valid ? at : e >= E ? -1 : -2;
     }
     __syncthreads();
     if (warp == 0) {
@@ -134,6 +134,7 @@ __global__ void moe_combine_kernel(const bf16* __restrict__ ys, const int* __res
         for (int k = 0; k < top; ++k) {
             const float wgt = weights[(size_t)t * top + k];
             const int pos = pair_pos[(size_t)t * top + k];
+            if (pos == -2) continue;
             const uint4 raw = *((const uint4*)(pos < 0 ? x + (size_t)t * W : ys + (size_t)pos * W) + i);
             const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
 #pragma unroll

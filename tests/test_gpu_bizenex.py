@@ -386,6 +386,36 @@ def test_moe_experts(ops, dtype, shape, n):
     close(out, want, dtype)
 
 
+@pytest.mark.parametrize("n", [9, 300])
+def test_moe_experts_of_negative_ids(ops, n):
+    """A negative id adds nothing and touches no other pair's row: the grouped products give the others what they give
+    without it, and the rest as the token by token form has it."""
+    E, top, W, F = 5, 3, 128, 64
+    g = torch.Generator().manual_seed(n)
+    x, gate_up, down = (dev(torch.randn(*s, generator=g), torch.bfloat16) for s in ((n, W), (E, 2 * F, W), (E, W, F)))
+    gate_up, down = gate_up * 0.1, down * 0.1
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).int()
+    some = ids.clone()
+    some[::4, 1], some[1::7, 0], some[2] = -1, -7, -1
+    wts = torch.rand(n, top, generator=g).cuda()
+    out = {}
+    saved = ops.moe_mode
+    try:
+        for mode, which in (("grouped", ids), ("grouped", some), ("simple", some)):
+            ops.moe_mode = mode
+            y = torch.empty(n, W, dtype=torch.bfloat16, device="cuda")
+            ops.moe_experts(x, dev(which), wts, gate_up, down, y)
+            out[mode, which is some] = y
+    finally:
+        ops.moe_mode = saved
+    ops.check_status()
+    whole = (some >= 0).all(1).cuda()
+    assert torch.equal(out["grouped", True][whole], out["grouped", False][whole])
+    assert not bool(out["grouped", True][2].any())
+    close(out["grouped", True], out["simple", True].double().cpu(), torch.bfloat16)
+
+
+
 def test_softcap(ops):
     x = torch.randn(5, 1001) * 40
     y = dev(x.clone())
