@@ -387,6 +387,9 @@ class CudaOps:
         self._check(self.lib.rv_gemm_f32_split(
             _ptr(x), _ptr(w), _ptr(y), _ptr(parts), _ptr(self._gemm_status(x.device)), c_int(m), c_int(n),
             c_int(k), self._stream()), "gemm_f32_split")
+        # two kernels for as many rows as there is room for (48 floats a row and 32 of K)
+        portion = max(1, parts.numel() // (48 * -(-k // 32)))
+        self.launches += 2 * -(-m // portion) - 1
         return y
 
     def linear(self, x, w, bias=None, out_dtype=None):
