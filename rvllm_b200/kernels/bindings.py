@@ -376,7 +376,8 @@ class CudaOps:
         # It was the faster one at all sizes that were measured (K 512 to 8,192, 256 to 65,536 columns, 1 to
         # 2,048 rows; 1.2 to 5 times the faster of the others) but for a few of up to 16 rows that were even.
         # Which of the small ones stay where they were is pinned by tests of the other kernel.
-        return k % 4 == 0 and k >= 768 and n >= (256 if m <= 32 else 1024)
+        # (More column tiles than a grid has rows are the library's.)
+        return k % 4 == 0 and k >= 768 and (256 if m <= 32 else 1024) <= n <= 65535 * 128
 
     def _linear_split(self, x, w):
         """y = x . w^T, float32, as sums of products of bfloat16 parts (gemm_f32_split.cu)."""

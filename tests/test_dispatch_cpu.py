@@ -80,6 +80,10 @@ def test_float32_product_of_parts_by_size(split_ops, m, n, k, taken):
     assert bool(split_ops.split) is taken and len(split_ops.split) + len(split_ops.calls) == 1
 
 
+def test_float32_product_of_parts_leaves_more_columns_than_a_grid_has():
+    assert CudaOps._split_better(8, 65535 * 128, 1024) and not CudaOps._split_better(8, 65535 * 128 + 1, 1024)
+
+
 def test_float32_product_of_parts_takes_what_fits(split_ops):
     """Operands with other strides, of other types, at other addresses, on other devices or that want
     gradients stay with the library; what it refuses stays refused."""
