@@ -373,11 +373,12 @@ class CudaOps:
 
     @staticmethod
     def _split_better(m: int, n: int, k: int) -> bool:
-        # It was the faster one at all sizes that were measured (K 512 to 8,192, 256 to 65,536 columns, 1 to
-        # 2,048 rows; 1.2 to 5 times the faster of the others) but for a few of up to 16 rows that were even.
-        # Which of the small ones stay where they were is pinned by tests of the other kernel.
-        # (More column tiles than a grid has rows are the library's.)
-        return k % 4 == 0 and k >= 768 and (256 if m <= 32 else 1024) <= n <= 65535 * 128
+        # Against the library's kernels, which are what else there is (gemm_f32.cu has the few sizes at which it is the
+        # fastest one; measured at 256 to 4,096 of K, 256 to 65,536 columns, 1 to 1,024 rows, replayed, us here / the
+        # library's): K 256 16 rows 8 / 8, 64 rows 10 / 7, 1,024 rows by 1,024 columns 16 / 15; K 512 7 / 12, 9 / 11
+        # (4,608 columns 17 / 16), 1,024 rows by 256 columns 13 / 12, by 512 15 / 16; from K 640 on 1.04 to 4.3 times as
+        # fast.  (More column tiles than a grid has rows are the library's.)
+        return k % 4 == 0 and k >= 512 and 256 <= n <= 65535 * 128
 
     def _linear_split(self, x, w):
         """y = x . w^T, float32, as sums of products of bfloat16 parts (gemm_f32_split.cu)."""
@@ -403,14 +404,14 @@ class CudaOps:
             return torch.empty((0, w.shape[0]), dtype=out_dtype, device=x.device)
         if self._small_product(x, w, out_dtype):
             y = self.linear_tcgen05(x, w, out_dtype)
-        elif self._float32_product(x, w, out_dtype) and self._split_better(x.shape[0], w.shape[0], x.shape[1]):
-            y = self._linear_split(x, w)
         elif (self._float32_product(x, w, out_dtype)
               and self.lib.rv_gemm_f32_better(x.shape[0], w.shape[0], x.shape[1])):
             y = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
             self._check(self.lib.rv_gemm_f32(_ptr(x), _ptr(w), _ptr(y), c_int(x.shape[0]),
                                              c_int(w.shape[0]), c_int(x.shape[1]), self._stream()),
                         "gemm_f32")
+        elif self._float32_product(x, w, out_dtype) and self._split_better(x.shape[0], w.shape[0], x.shape[1]):
+            y = self._linear_split(x, w)
         else:
             # The library chooses an algorithm per shape, and a shape it has not met costs it
             # some 70 us on the host: a prompt portion of 301 tokens, then 302, ... would pay

@@ -66,6 +66,7 @@ def test_float32_product_leaves_other_devices_and_gradients(ops):
 @pytest.fixture
 def split_ops(ops):
     ops.split = []
+    ops.lib.rv_gemm_f32_better = lambda M, N, K: 0
     ops.lib.rv_gemm_f32_split_scratch = lambda m, k: 8
     ops.lib.rv_gemm_f32_split = lambda *a: ops.split.append(a) or 0
     ops._gemm_status = lambda device: torch.zeros(1, dtype=torch.int32)
@@ -73,11 +74,14 @@ def split_ops(ops):
 
 
 @pytest.mark.parametrize("m,n,k,taken", [
-    (1, 256, 768, True), (32, 256, 768, True), (33, 256, 768, False), (33, 1024, 768, True), (2048, 1024, 768, True),
-    (8, 255, 768, False), (8, 2048, 764, False), (8, 2048, 770, False)])
+    (1, 256, 512, True), (32, 256, 768, True), (33, 256, 768, True), (33, 1024, 768, True), (2048, 1024, 768, True),
+    (8, 255, 768, False), (8, 2048, 508, False), (8, 2048, 764, True), (8, 2048, 770, False)])
 def test_float32_product_of_parts_by_size(split_ops, m, n, k, taken):
     split_ops.linear(on_device(m, k), on_device(n, k))
-    assert bool(split_ops.split) is taken and len(split_ops.split) + len(split_ops.calls) == 1
+    assert len(split_ops.split) == int(taken) and not split_ops.calls
+    split_ops.lib.rv_gemm_f32_better = lambda M, N, K: 1    # the other kernel is asked first
+    split_ops.linear(on_device(m, k), on_device(n, k))
+    assert len(split_ops.split) == int(taken) and len(split_ops.calls) == 1
 
 
 def test_float32_product_of_parts_leaves_more_columns_than_a_grid_has():

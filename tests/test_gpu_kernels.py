@@ -754,8 +754,8 @@ def test_gemm_tiled_weights(ops, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [
-    # every number of row groups, one and two row tiles, columns that fill no tile, K that fills no
-    # step (and no split of K), K split over one to eight blocks
+    # one to twenty row tiles, columns that fill no tile, K that fills no step (and no split of K), K split over one to
+    # eight blocks
     (1, 256, 256), (8, 300, 1028), (9, 2048, 260), (16, 70000, 512), (24, 4608, 1536), (32, 1001, 2052),
     (40, 520, 4096), (48, 640, 1024), (56, 257, 3000), (64, 6144, 256), (65, 1536, 6912), (131, 2048, 516),
     (160, 333, 1540)])
@@ -775,6 +775,23 @@ def test_gemm_f32(ops, M, N, K):
     bound = (K / 2 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
     assert bool(((y.double().cpu() - ref).abs() <= bound).all())
     assert float((y.double().cpu() - ref).norm() / ref.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("M,N,K,launches", [
+    # the split product, from K 512 and 256 columns on (two launches); the other kernel's few sizes (one), and beyond
+    # each of their ends; the library (none)
+    (40, 256, 512, 2), (8, 9216, 1024, 1), (9, 9216, 1024, 2), (8, 9216, 1020, 2), (8, 8188, 1024, 2), (8, 10244, 1024, 2),
+    (1, 8192, 2048, 1), (1, 8192, 2052, 2), (8, 256, 508, 0), (8, 252, 512, 0)])
+def test_float32_products_by_size(ops, M, N, K, launches):
+    """Which kernel a float32 product takes; the bound is `test_gemm_f32`'s, the widest of the three."""
+    g = torch.Generator().manual_seed(K)
+    x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    before = ops.launches
+    y = ops.linear(x, w)
+    assert ops.launches == before + launches
+    ref = x.double() @ w.double().t()
+    ops.check_status()
+    assert bool(((y.double() - ref).abs() <= (K / 2 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())).all())
 
 
 @pytest.mark.parametrize("M,N,K", [
