@@ -382,8 +382,14 @@ static int grouped_product(const void* xs, const void* w, void* out, int* status
     // 42.4 against 41.8, 2,048 60 against 47.)
     const long long tiles = max_tiles - E + (E + 1) / 2;
     const int w_tiles = (n_out + MG_BM - 1) / MG_BM, sms = rv_sm_count();
-    const int MT = TN >= 128 && n_out >= 4 * MG_BM && tiles * ((w_tiles + 1) / 2) > sms ? 2 : 1;
-    const int smem_limit = MT == 1 && tiles * w_tiles <= sms ? MG_SMEM_MAX : MG_SMEM_LIMIT;
+    // (RVLLM_MOE_MT=1 or 2 and RVLLM_MOE_SMEM_KB force the tiles and the ring's size.)
+    const char* mt_env = getenv("RVLLM_MOE_MT");
+    const char* smem_env = getenv("RVLLM_MOE_SMEM_KB");
+    const int forced_mt = mt_env ? atoi(mt_env) : 0;
+    const int MT = forced_mt == 1 || forced_mt == 2 ? forced_mt
+                   : TN >= 128 && n_out >= 4 * MG_BM && tiles * ((w_tiles + 1) / 2) > sms ? 2 : 1;
+    const int smem_limit = smem_env ? atoi(smem_env) * 1024
+                           : MT == 1 && tiles * w_tiles <= sms ? MG_SMEM_MAX : MG_SMEM_LIMIT;
     const int per_stage = MT * MG_BM * MG_BK * 2 + TN * MG_BK * 2;
     int stages = (smem_limit - 1024) / per_stage;
     if (stages > 6) stages = 6;

@@ -386,6 +386,33 @@ def test_moe_experts(ops, dtype, shape, n):
     close(out, want, dtype)
 
 
+def test_moe_experts_by_two_tiles(ops, monkeypatch):
+    """Many tokens an expert and many rows of its matrices: a block takes two tiles of 128 rows, the last pair of which
+    is there in part (1,168 rows) or without its second (1,096).  The same sums as a tile a block, and as float64 has them
+    (bfloat16 rows between and behind: 2^-7 of the largest)."""
+    n, E, top, W, F = 2100, 16, 4, 1096, 584
+    g = torch.Generator().manual_seed(3)
+    x, gate_up, down = (dev(torch.randn(*s, generator=g) * a, torch.bfloat16) for s, a in (
+        ((n, W), 1.0), ((E, 2 * F, W), W ** -0.5), ((E, W, F), F ** -0.5)))
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).int().cuda()
+    wts = torch.rand(n, top, generator=g).cuda()
+    out = []
+    for tiles in (None, "2", "1"):
+        if tiles:
+            monkeypatch.setenv("RVLLM_MOE_MT", tiles)
+        out.append(torch.full((n, W), float("nan"), dtype=torch.bfloat16, device="cuda"))
+        ops.moe_experts(x, ids, wts, gate_up, down, out[-1])
+    ops.check_status()
+    assert torch.equal(out[0], out[1]) and torch.equal(out[1], out[2])
+    want = torch.zeros(n, W, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t, k = (ids == e).nonzero(as_tuple=True)
+        h = x[t].double() @ gate_up[e].double().T
+        y = (torch.nn.functional.silu(h[:, 0::2]) * h[:, 1::2]) @ down[e].double().T
+        want.index_add_(0, t, wts[t, k, None].double() * y)
+    assert float((out[0].double() - want).abs().max() / want.abs().max()) < 2.0 ** -7
+
+
 @pytest.mark.parametrize("n", [9, 300])
 def test_moe_experts_of_negative_ids(ops, n):
     """A negative id adds nothing and touches no other pair's row: the grouped products give the others what they give
