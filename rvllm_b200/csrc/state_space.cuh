@@ -63,8 +63,11 @@ __global__ void __launch_bounds__(256) ss_decay_kernel(
 // of the row).  A thread keeps NV times V values of the row, all requested together (0: any number,
 // kept in shared memory).  2,048 tokens of 32 heads of 64: 24.4 us with a block per request that moved the inputs on
 // one place after the other and 256 threads a token, 15.4 so (50 MB, some 8 us of HBM's time).
+// Registers for four times V values leave one block a multiprocessor (8,192 values, 300 tokens: the whole layer 79.6 us
+// with three blocks and values spilled, 72.9 so); twice V are better with three and 16 bytes spilled (4,096 values, 2,048 tokens:
+// 171 us, 178 with two).
 template <typename T, int V, int NV>
-__global__ void __launch_bounds__(512, 3) ss_finish_kernel(
+__global__ void __launch_bounds__(512, NV == 4 ? 1 : 3) ss_finish_kernel(
     const float* __restrict__ num, const T* __restrict__ rows, const float* __restrict__ proj, int P,
     const float* __restrict__ D, const float* __restrict__ norm_w, float eps, float* __restrict__ conv_state,
     const int* __restrict__ token_req, const int* __restrict__ q_start, const int* __restrict__ state_slot,

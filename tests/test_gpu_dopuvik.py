@@ -516,6 +516,33 @@ def test_state_space_kernels(ops, dtype, sizes):
     assert float((state[4] - 3.0).abs().max()) == 0 and float(state[1].abs().max()) == 0
 
 
+@pytest.mark.parametrize("dtype,sizes,lens,heads", [
+    # a block takes two and four heads one after another, columns that leave warps without any in the second of two
+    # tiles; norms over 2,560 and 4,096 values (two pieces a thread), 8,192 (four) and 8,320 (shared memory)
+    (torch.bfloat16, (32, 64, 64, 1, 4, 1), [1500, 613], 2), (torch.bfloat16, (64, 64, 32, 1, 2, 1), [1800, 77], 4),
+    (torch.bfloat16, (32, 80, 32, 2, 2, 1), [1100, 13], 2), (torch.bfloat16, (128, 64, 16, 1, 2, 1), [70, 1], 1),
+    (torch.float32, (128, 64, 16, 1, 2, 1), [70, 1], 1), (torch.bfloat16, (130, 64, 16, 1, 2, 1), [40], 1),
+    (torch.float32, (64, 64, 16, 1, 2, 1), [40], 1)])
+def test_state_space_of_many_heads(ops, dtype, sizes, lens, heads):
+    H, dvv, N, G, taps, ng = sizes
+    if heads > 1:           # as many heads a block as leave three blocks a multiprocessor (lm_heads)
+        blocks = sum(-(-n // 64) for n in lens) * H * -(-dvv // 64)
+        full = 3 * torch.cuda.get_device_properties(0).multi_processor_count
+        assert blocks // heads >= full and (heads == 4 or blocks // (2 * heads) < full)
+    gen = torch.Generator().manual_seed(H)
+    m, C, t = _ssm(gen, H, dvv, N, G, taps, ng)
+    rows = [rnd(gen, torch.float32, n, H * dvv + C + H).numpy() for n in lens]
+    state, conv = torch.zeros(len(lens), H * N * dvv, device="cuda"), torch.zeros(len(lens), taps - 1, C, device="cuda")
+    ctx, q_start = step_context([(n, r) for r, n in enumerate(lens)])
+    got = _ssm_run(ops, m, C, t, state, conv, dtype)(np.concatenate(rows), ctx)
+    for r, x in enumerate(rows):
+        want, S = _ssm_plain(m, C, t, x, dtype == torch.bfloat16)
+        close(got[q_start[r]:q_start[r + 1]], want, dtype, bound=4e-5 if dtype == torch.float32 else None)
+        # (a value on the way between two bfloat16 numbers may round the other way)
+        close(state[r], S.reshape(-1), torch.float32, bound=4e-5 if dtype == torch.float32 else 2e-3)
+        close(conv[r], np.concatenate([np.zeros((taps - 1, C)), x[:, H * dvv:H * dvv + C]])[-(taps - 1):], torch.float32)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n", [1, 17])
 def test_state_space_inputs_far_below_zero(ops, dtype, n):
