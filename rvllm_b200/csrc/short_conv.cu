@@ -248,7 +248,7 @@ __global__ void short_conv_vec4_kernel(const T* __restrict__ proj, const float* 
 // Portions: a thread owns eight adjacent channels (one 16-byte access per bfloat16
 // row) of R consecutive tokens and requests all that it reads (B, C and x of its tokens, the window before them and,
 // for the new state, the portion's last rows) before it uses any of it: a launch is one latency for the index
-// arrays and one for the rows (LOOP: several rounds of R tokens).  The blocks are those that have tokens, found from
+// arrays and one for the rows (LOOP: several rounds of R tokens, and the portion's last rows behind them).  The blocks are those that have tokens, found from
 // `q_start`: blocks for every request as if it were the longest, 16 tokens each in two rounds, took 6.2 us in a replay
 // for a portion of 512 beside 31 single tokens of 1,024 channels, 3.3 now; four portions of some 33 float32 tokens of
 // 1,536 channels, token after token, 11.9 and 2.9.
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
             old[k][0] = a.x; old[k][1] = a.y; old[k][2] = a.z; old[k][3] = a.w;
             old[k][4] = b.x; old[k][5] = b.y; old[k][6] = b.z; old[k][7] = b.w;
         }
-        if (moves && !ends_here) {
+        if (!LOOP && moves && !ends_here) {
             const T* p = proj + (size_t)(q0 + qlen + k - HIST) * stride + c;
             nb[k] = rv_conv_raw8(p);
             nx[k] = rv_conv_raw8(p + 2 * hidden);
@@ -445,7 +445,10 @@ __global__ void __launch_bounds__(128) short_conv_rows_kernel(
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = win[k][i];
             } else {                                   // more tokens than a piece: as many as the window's at least
-                bx_of(nb[k], nx[k], v);
+                if (LOOP) {                            // (registers for these rows spill what the rounds need)
+                    const T* p = proj + (size_t)(q0 + qlen + k - HIST) * stride + c;
+                    bx_of(rv_conv_raw8(p), rv_conv_raw8(p + 2 * hidden), v);
+                } else bx_of(nb[k], nx[k], v);
             }
             float* sp = st + (size_t)k * hidden;
             *(float4*)sp = make_float4(v[0], v[1], v[2], v[3]);
@@ -492,7 +495,10 @@ extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, c
     // Us, 3 taps: 543 bfloat16 tokens of 1,024 channels with 2 / 4 / 8 tokens a thread 3.29 / 3.26 / 3.40, 108 2.45 /
     // 2.80 / 3.16, 600 of 2,048 channels 5.78 / 4.94 / 5.32, 2,000 of 1,536 10.8 / 8.5 / 9.0 and 8.9 in two rounds of 8
     // (no fewer than the window has: two only up to 3 taps.)  131 float32 tokens of 1,536 2.90 / 3.26, 2,048 of 2,048 17.1 / 13.7, 12.4 in four rounds of 4 (a thread reads the
-    // window before its tokens once more, so long rows are better read in longer pieces).
+    // window before its tokens once more, so long rows are better read in longer pieces).  With 4 taps' registers two blocks of 4
+    // tokens a thread fit a multiprocessor instead of three, so rounds are better from half as many pieces on: bfloat16, at once /
+    // in rounds: 2,048 tokens of 2,048 14.0 / 9.8, 1,200 9.2 / 8.3, 1,500 of 1,024 channels (below that) 6.5; float32 131 of 1,536 3.6,
+    // 500 of 2,048 6.3, with 388 bytes spilled (token after token 5.8, 9.4).
     static const int rows_from = [] {
         const char* e = getenv("RVLLM_CONV_WIDE_FROM");
         return e && *e ? atoi(e) : 2;
@@ -501,7 +507,7 @@ extern "C" int rv_short_conv(const void* proj, int dtype, const float* filter, c
         (uintptr_t)filter % 16 == 0) {
         const int wide = (hidden / 8 + 127) / 128, sms = rv_sm_count();
         auto pieces = [&](int r) { return (long long)n_tokens / r + n_reqs; };    // as many as there may be
-        const bool half = dtype == RV_DTYPE_BF16, in_rounds = pieces(16) * wide >= (half ? 2 : 1) * sms;
+        const bool half = dtype == RV_DTYPE_BF16, in_rounds = pieces(16) * wide >= (half && taps < 4 ? 2 : 1) * sms;
         const int r = in_rounds ? (half ? 8 : 4) : pieces(4) * wide >= sms || taps > 3 ? 4 : 2;
         const int rounds = in_rounds ? 16 / r : 1;
         if (pieces(r * rounds) <= 65535) {

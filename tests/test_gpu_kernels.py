@@ -476,9 +476,9 @@ def test_short_conv(ops, dtype, taps, bias):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("taps,rest", [(3, 2600), (4, 2600), (2, 700), (4, 700)])
+@pytest.mark.parametrize("taps,rest", [(3, 2600), (4, 2600), (2, 700), (4, 700), (4, 300)])
 def test_short_conv_pieces(ops, dtype, taps, rest):
-    """Pieces of 16 tokens in rounds (2,600 tokens of 1,032 channels) and of 4 at once (700), for more requests than
+    """Pieces of 16 tokens in rounds (2,600 tokens of 1,032 channels) and of 4 at once (700, with 4 taps 300), for more requests than
     are looked up at a time and portions around a piece's and a window's length."""
     g = torch.Generator().manual_seed(19)
     hidden = 1032
