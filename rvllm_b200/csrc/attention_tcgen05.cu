@@ -788,12 +788,17 @@ extern "C" long long AT_SYM(rv_paged_attention_prefill_tcgen05_scratch_bytes)(in
     return (long long)(6 * (size_t)(n_sms > 0 ? n_sms : 1) * AT_PART_BYTES);
 }
 
-static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window, int n_sms,
-                    long long scratch_bytes) {
+// RVLLM_PREFILL_SPLIT: so many parts through memory, 1: nothing is shared out, in clusters neither.
+static int at_forced_parts() {
     static const int forced = [] {
         const char* e = getenv("RVLLM_PREFILL_SPLIT");
         return e && *e ? atoi(e) : 0;
     }();
+    return forced;
+}
+static int at_parts(long long blocks, int max_ctx_len, int max_q_len, int window, int n_sms,
+                    long long scratch_bytes) {
+    const int forced = at_forced_parts();
     const long long places = 2ll * n_sms;
     int parts = forced > 0 ? forced : (int)((places + blocks / 2) / blocks);
     // the tiles every block of query tokens has before its own: a whole prompt (none before it)
@@ -839,6 +844,26 @@ static int at_cluster(long long blocks, int parts, int tiles, int n_sms) {
     if (tiles >= 8 && 5 * blocks <= places) return 4;
     if (tiles >= 11 && 8 * blocks <= places * (tiles >= 20 ? 5 : 4)) return 2;
     return 1;
+}
+
+struct AtShares { int parts, cluster; };          // through memory, in a cluster
+static AtShares at_shares(int n_tokens, int n_reqs, int max_q_len, int max_ctx_len, int num_heads, int num_kv_heads, int window,
+                          bool scratch, long long scratch_bytes, int n_sms) {
+    const int q_block = AT_ROWS / (num_heads / num_kv_heads), nqb = (max_q_len + q_block - 1) / q_block;
+    const long long blocks = (long long)num_kv_heads * nqb * n_reqs;
+    const int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;
+    if (n_sms <= 0 || at_forced_parts() > 0) return {parts, 1};
+    const long long real = (long long)num_kv_heads * (n_tokens / q_block + n_reqs);
+    int depth = (max_ctx_len + AT_KEYS - 1) / AT_KEYS;
+    if (window > 0 && window / AT_KEYS + 2 < depth) depth = window / AT_KEYS + 2;
+    const int cluster = at_cluster(blocks < real ? blocks : real, parts, depth, n_sms);
+    return {cluster > 1 ? 1 : parts, cluster};
+}
+// Blocks of a cluster that a launch of these sizes takes, with all the scratch that it may ask for.
+extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05_cluster)(int n_tokens, int n_reqs, int max_q_len, int max_ctx_len,
+                                                                  int num_heads, int num_kv_heads, int window, int n_sms) {
+    return at_shares(n_tokens, n_reqs, max_q_len, max_ctx_len, num_heads, num_kv_heads, window, true,
+                     AT_SYM(rv_paged_attention_prefill_tcgen05_scratch_bytes)(n_sms), n_sms).cluster;
 }
 
 static int at_configure(size_t smem) {
@@ -894,16 +919,13 @@ extern "C" int AT_SYM(rv_paged_attention_prefill_tcgen05)(
     if (at_configure(smem)) return 1;
     const int nqb = (max_q_len + q_block - 1) / q_block;
     const long long blocks = (long long)num_kv_heads * nqb * n_reqs;
-    int parts = scratch && n_sms > 0 ? at_parts(blocks, max_ctx_len, max_q_len, window, n_sms, scratch_bytes) : 1;
+    const AtShares shares = at_shares(n_tokens, n_reqs, max_q_len, max_ctx_len, num_heads, num_kv_heads, window,
+                                      scratch != nullptr, scratch_bytes, n_sms);
+    const int parts = shares.parts, cluster = shares.cluster;
     if ((long long)n_reqs * (parts > AT_ROWS / 16 ? parts : AT_ROWS / 16) > 65535)
         return at_fail("paged_attention_prefill_tcgen05: too many requests");
     float* part_o = (float*)scratch;
     float2* part_ml = (float2*)((char*)scratch + (size_t)blocks * parts * AT_ROWS * RV_HD * 4);
-    const long long real = (long long)num_kv_heads * (n_tokens / q_block + n_reqs);
-    int depth = (max_ctx_len + AT_KEYS - 1) / AT_KEYS;
-    if (window > 0 && window / AT_KEYS + 2 < depth) depth = window / AT_KEYS + 2;
-    const int cluster = n_sms > 0 ? at_cluster(blocks < real ? blocks : real, parts, depth, n_sms) : 1;
-    if (cluster > 1) parts = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_kv_heads, nqb, n_reqs * parts * cluster);
     cfg.blockDim = dim3(AT_THREADS);

@@ -2,7 +2,10 @@
 other than the engine's: widths that are no power of two, head sizes 48 and 80, groups
 of 3, pages of 8, filters of 2 to 5 taps."""
 import math
+import os
 import random
+import subprocess
+import sys
 from ctypes import c_int
 from types import SimpleNamespace
 
@@ -1038,19 +1041,40 @@ def test_prefill_attention_blocks_a_multiprocessor(ops, head_dim, same, blocks):
         torch.cuda.get_device_properties(0).shared_memory_per_multiprocessor
 
 
-@pytest.mark.parametrize("hd,heads,kv,lens,ctxs,window", [
+CLUSTERS = [
     # whole prompts in clusters of four and of two, just over one part's tiles; parts that become clusters
-    # of two, three and four; a second request of which most blocks have no tokens; blocks of the
-    # cluster without tiles (fewer tiles than blocks); a window; latent rows
-    (64, 16, 8, [449], [449], None), (64, 16, 8, [700], [700], None), (64, 16, 8, [1000], [1000], None),
-    (64, 32, 8, [512], [1212], None), (64, 32, 8, [128], [1128], None), (64, 32, 8, [256], [2256], None),
-    (64, 16, 8, [300, 700], [300, 700], None), (64, 16, 8, [700, 3], [700, 700], None), (64, 16, 8, [1000], [1500], 700),
-    (128, 16, 1, [1000], [1000], None), (128, 16, 1, [512], [2012], None), (128, 32, 8, [256], [2256], None),
-    (128, 16, 1, [1000], [1500], 640)])
-def test_prefill_attention_in_clusters(ops, hd, heads, kv, lens, ctxs, window):
+    # of four, three and two; a second request of which most blocks have no tokens; blocks of the
+    # cluster without tiles (fewer tiles than blocks); a window; latent rows; and one of many blocks, which takes none
+    (64, 16, 8, [449], [449], None, 4), (64, 16, 8, [700], [700], None, 4), (64, 16, 8, [1000], [1000], None, 2),
+    (64, 32, 8, [512], [1212], None, 2), (64, 32, 8, [128], [1128], None, 3), (64, 32, 8, [256], [2256], None, 4),
+    (64, 16, 8, [300, 700], [300, 700], None, 2), (64, 16, 8, [700, 3], [700, 700], None, 2), (64, 16, 8, [1000], [1500], 700, 2),
+    (128, 16, 1, [1000], [1000], None, 2), (128, 16, 1, [512], [2012], None, 4), (128, 32, 8, [256], [2256], None, 4),
+    (128, 16, 1, [1000], [1500], 640, 2), (64, 32, 8, [1000, 1000], [1000, 1000], None, 1)]
+
+
+def _cluster_of(ops, hd, heads, kv, lens, ctxs, window):
+    fn = getattr(ops._attn5_lib(hd, kv == 1), f"rv_paged_attention_prefill_tcgen05_cluster_hd{hd}")
+    return fn(*(c_int(v) for v in (sum(lens), len(lens), max(lens), max(ctxs), heads, kv, window or 0, ops._sm_count)))
+
+
+def test_prefill_attention_forced_parts_take_no_cluster():
+    """RVLLM_PREFILL_SPLIT=1 shares nothing out, other numbers through memory."""
+    code = ("import sys; sys.path.insert(0, 'tests'); import test_gpu_kernels as t; from rvllm_b200.kernels import cuda_ops; "
+            "print(*[t._cluster_of(cuda_ops(), *c[:-1]) for c in t.CLUSTERS])")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for parts in ("1", "3"):
+        out = subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, RVLLM_PREFILL_SPLIT=parts),
+                             capture_output=True, text=True, timeout=300)
+        assert out.returncode == 0, out.stderr[-2000:]
+        assert out.stdout.split() == ["1"] * len(CLUSTERS)
+
+
+@pytest.mark.parametrize("hd,heads,kv,lens,ctxs,window,cluster", CLUSTERS)
+def test_prefill_attention_in_clusters(ops, hd, heads, kv, lens, ctxs, window, cluster):
     """Blocks that share a block's key tiles and meet in distributed shared memory, against float64.  P and
     the outputs are rounded to bfloat16 (2^-9 of each at the most, of both signs): 2^-8 of the outputs' norm."""
     g = torch.Generator().manual_seed(sum(lens) + hd)
+    assert _cluster_of(ops, hd, heads, kv, lens, ctxs, window) == cluster
     q, kc, vc, ctx, group = attention_case(torch.bfloat16, g, lens, ctxs, heads, kv, hd, 16)
     same = kv == 1
     if same:
