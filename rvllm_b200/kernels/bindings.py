@@ -304,13 +304,17 @@ class CudaOps:
         and pass what it read to `raise_for_status`, which costs no synchronisation."""
         return self._gemm_status(device)
 
+    @staticmethod
+    def _gave_up(code: int, where: str = "") -> KernelError:
+        return KernelError(f"a kernel gave up waiting on an mbarrier (code {code}: 1-4 gemm_tcgen05, 12 decode "
+                           f"attention, 21 prefill attention, 31-34 grouped experts, 41-45 float32 products)"
+                           f"{where}; its output is not valid")
+
     def raise_for_status(self, code: int, device=None) -> None:
         if code != 0:
             if device is not None:
                 self._gemm_status(device).zero_()
-            raise KernelError(f"a kernel gave up waiting on an mbarrier (code {code}: 1-4 "
-                              f"gemm_tcgen05, 12 decode attention, 21 prefill attention, 31-34 "
-                              f"grouped experts, 41-45 float32 products); its output is not valid")
+            raise self._gave_up(code)
 
     def check_status(self) -> None:
         """Raise if a kernel recorded that one of its bounded waits ran out (this
@@ -319,9 +323,7 @@ class CudaOps:
             code = int(st.item())
             if code != 0:
                 st.zero_()
-                raise KernelError(f"a kernel gave up waiting on an mbarrier (code {code}: 1-4 "
-                                  f"gemm_tcgen05, 12 decode attention, 21 prefill attention) on {device}; its "
-                                  f"output is not valid")
+                raise self._gave_up(code, f" on {device}")
 
     def _small_product(self, x, w, out_dtype) -> bool:
         """Whether x . w^T goes to the tcgen05 weight-streaming kernel."""

@@ -5,6 +5,7 @@ from types import SimpleNamespace
 import pytest
 import torch
 
+from rvllm_b200.errors import KernelError
 from rvllm_b200.kernels.bindings import CudaOps
 
 
@@ -105,6 +106,19 @@ def test_float32_product_of_parts_takes_what_fits(split_ops):
     split_ops.linear(x, w)
     split_ops.linear(x, w.bfloat16())                       # cast, then multiplied
     assert len(split_ops.split) == 2
+
+
+@pytest.mark.parametrize("code", [12, 33, 45])
+def test_a_wait_that_ran_out_is_named_wherever_it_is_asked_for(ops, code):
+    word = torch.tensor([code], dtype=torch.int32)
+    ops._gemm_state = {"cuda:0": word}
+    with pytest.raises(KernelError, match=f"code {code}:.*31-34 grouped experts, 41-45 float32 products.* on cuda:0"):
+        ops.check_status()
+    assert int(word) == 0
+    with pytest.raises(KernelError, match=f"code {code}:.*31-34 grouped experts, 41-45 float32 products"):
+        ops.raise_for_status(code)
+    ops.check_status()
+    ops.raise_for_status(0)
 
 
 class Cuda(OnDevice):
