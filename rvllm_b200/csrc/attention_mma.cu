@@ -697,7 +697,8 @@ struct StreamMeta {
     int r, g, m0, place, key_lo, key_hi, t_first, t_last;
 };
 
-template <int HD>
+// REST: how the rest of P is multiplied (attend_tile); 1 for up to eight heads a key/value head.
+template <int HD, int REST>
 __global__ void __launch_bounds__(RV_STREAM_WARPS * 32, 1)
 paged_attention_decode_stream_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -923,24 +924,20 @@ paged_attention_decode_stream_kernel(
                 break;
             }
             const bf16* kt = my_ring + (size_t)s * 2 * TILE;
-            if (rows <= 8)
-                attend_tile<HD, true, false, 1>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
-                                                scale_log2, m_a, m_b, l_a, l_b, o);
-            else
-                attend_tile<HD, true, false, 2>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
-                                                scale_log2, m_a, m_b, l_a, l_b, o, 0.f, 0.f, rest);
+            attend_tile<HD, true, false, REST>(qf, kt, kt + TILE, t * RV_BN, lane, m.key_lo, hi_a, m.key_lo, hi_b,
+                                               scale_log2, m_a, m_b, l_a, l_b, o, 0.f, 0.f, rest);
             __syncwarp();
             ++n_consumed;
             fill();                                 // the freed stage takes the next tile
         }
         if (failed) break;
-        // what was left of P: with up to eight rows in rows 8 .. 15.  (An infinite value's share is no number there.)
+        // what was left of P.  (An infinite value's share is no number there.)
         auto add = [](float a, float b) { return fabsf(b) < INFINITY ? a + b : a; };
 #pragma unroll
         for (int i = 0; i < HD / 8; ++i)
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (rows > 8) o[i][e] = add(o[i][e], rest[i][e]);
+                if (REST == 2) o[i][e] = add(o[i][e], rest[i][e]);
                 else if (e < 2) o[i][e] = add(o[i][e], o[i][2 + e]);
         l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
         l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
@@ -1262,12 +1259,13 @@ extern "C" int RV_SYM(rv_paged_attention_decode_stream)(
     const size_t ring_bytes = (size_t)RV_STREAM_WARPS * RV_STREAM_STAGES * 2 * RV_BN * RV_HD * sizeof(bf16);
     const size_t q_bytes = (size_t)RV_STREAM_WARPS * 2 * 16 * (RV_HD + 8) * sizeof(bf16);
     const size_t smem = ring_bytes + q_bytes + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(paged_attention_decode_stream_kernel<RV_HD>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const bool few = num_heads / num_kv_heads <= 8;
+    auto kernel = few ? paged_attention_decode_stream_kernel<RV_HD, 1> : paged_attention_decode_stream_kernel<RV_HD, 2>;
+    static bool configured[2];
+    if (!configured[few]) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(cudaGetErrorString(e));
-        configured = true;
+        configured[few] = true;
     }
     CUtensorMap map_k, map_v;
     if (kv_map(&map_k, k_cache, total_slots, num_kv_heads, page_size)) return 1;
@@ -1276,7 +1274,7 @@ extern "C" int RV_SYM(rv_paged_attention_decode_stream)(
     if (blocks > n_sms) blocks = n_sms;
     float* part_o = (float*)scratch;
     float2* part_ml = (float2*)(part_o + (size_t)num_heads * (teams + n_reqs) * RV_VD);
-    rv_launch(paged_attention_decode_stream_kernel<RV_HD>, dim3((unsigned)blocks),
+    rv_launch(kernel, dim3((unsigned)blocks),
               dim3(RV_STREAM_WARPS * 32), smem, (cudaStream_t)stream, map_k, map_v,
               (const bf16*)q, q_stride, block_table, max_blocks, ctx_lens, part_o, part_ml, keys, teams,
               num_heads, num_kv_heads, page_size, scale * 1.4426950408889634f, window, n_reqs, status);
