@@ -35,7 +35,8 @@
 // every output of the head is NaN, and so is its state; a bad query's own output is.
 //
 // Everything is float32: operands enter the bfloat16 products as three parts each (chunks.cuh), six of
-// the nine products.  What one kernel leaves for another's products lies in the order in which a
+// the nine products (the state's error against 64 bits, mean of 16 prompts of 640 tokens with weak / middling / strong
+// decays: 3.05e-7 / 1.94e-7 / 1.41e-7; with multiply-adds in the diagonal blocks 3.07e-7 / 1.93e-7 / 1.41e-7).  What one kernel leaves for another's products lies in the order in which a
 // warp's fragments hold it, 16 bytes a lane, so that it goes from memory to registers as it is.
 //
 // The scan by token is a chain of some 360 cycles a token; here it is two products and two barriers a

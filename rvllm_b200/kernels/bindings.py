@@ -3,10 +3,11 @@ parts call (`embed`, `add_rmsnorm`, `linear`, `qk_norm_rope_write`, `paged_atten
 `short_conv`, `swiglu`, `add_bias`, `argmax`, `sample`).
 
 Every kernel launches on torch's current stream, so captured graphs and ordinary
-stream order both work.  Matrix products go to cuBLAS through `torch.mm`, as the
-reference sends them to cuBLAS (src/cuda/cublas_ops.rs:44-92); with float32 operands
-TF32 is switched off, so the float32 path is float32 throughout.  There is no CPU
-path here: constructing `CudaOps` without a CUDA device or without the library raises.
+stream order both work.  Matrix products of few bfloat16 rows and most float32 ones run in this
+library's kernels, the others in cuBLAS through `torch.mm`, as the reference sends them to
+cuBLAS (src/cuda/cublas_ops.rs:44-92).  Float32 operands are multiplied in three bfloat16
+parts that hold all their bits, with float32 sums, or on the FP32 cores: TF32 is switched off
+in the library, so the float32 path is float32 throughout.  There is no CPU path here: constructing `CudaOps` without a CUDA device or without the library raises.
 """
 from __future__ import annotations
 
@@ -116,7 +117,7 @@ class CudaOps:
         # memory and of the delta rule with a decay per channel (the reasons are where they are asked)
         self.mlstm_above = 384
         self.gated_delta_above = 288
-        # float32 products must be float32: no TF32, no reduced-precision accumulation
+        # the library's float32 products must be float32: no TF32, no reduced-precision accumulation
         torch.backends.cuda.matmul.allow_tf32 = False
         torch.backends.cudnn.allow_tf32 = False
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
